@@ -698,10 +698,12 @@ template <typename T> void tune_rhs_shapes(fi_handle* h)
     // row of 1024 points at 256 threads left most warp slots empty
     int best_rb = 0, best_cb = 0, best_rt = 0, best_ct = 0;
     float tr = 1e30f, tc = 1e30f;
-    for (int rb : {1, 2, 4, 8}) {
-        if (2 * (size_t)rb * p.h * sizeof(C2) > (size_t)optin) continue;
+    // (register lines fix the threads of a line: only the lines per block are tried)
+    const int lr = rhs_line_threads(p.h, sizeof(T) == 4), lc = rhs_line_threads(p.ny, sizeof(T) == 4);
+    for (int rb : {1, 2, 4, 8, 16, 32}) {
+        if (lr ? rb * lr > 512 || rb * lr < 32 : rb > 8 || 2 * (size_t)rb * p.h * sizeof(C2) > (size_t)optin) continue;
         for (int rt : {128, 256, 512, 1024}) {
-            if (rt > 128 && rt > rb * p.h / 2) continue;   // at most one element pair per thread
+            if (rt > 128 && (lr || rt > rb * p.h / 2)) continue;   // at most one element pair per thread
             p.rb = rb;
             p.rt = rt;
             const float t = time_it([&] {
@@ -712,10 +714,11 @@ template <typename T> void tune_rhs_shapes(fi_handle* h)
             if (t < tr) { tr = t; best_rb = rb; best_rt = rt; }
         }
     }
-    for (int cb : {1, 2, 4, 8}) {
-        if (2 * (size_t)cb * (p.ny + 1) * sizeof(C2) > (size_t)optin) continue;
+    for (int cb : {1, 2, 4, 8, 16}) {
+        if (lc ? (cb * lc > 1024 || cb * lc < 32) && cb > 1
+               : cb > 8 || 2 * (size_t)cb * (p.ny + 1) * sizeof(C2) > (size_t)optin) continue;
         for (int ct : {128, 256, 512, 1024}) {
-            if (ct > 128 && ct > cb * p.ny / 2) continue;
+            if (ct > 128 && (lc || ct > cb * p.ny / 2)) continue;
             p.cb = cb;
             p.ct = ct;
             const float t = time_it([&] {
@@ -820,10 +823,11 @@ template <typename T> void tune_conv_shapes(fi_handle* h)
     const double scale = 1.0 / ((double)h->Px * (double)h->Py);
     int best_rb = 0, best_cb = 0, best_rt = 0, best_ct = 0;
     float tr = 1e30f, tc = 1e30f;
-    for (int rb : {1, 2, 4}) {
-        if (2 * (size_t)rb * p.h * sizeof(C2) > (size_t)optin) continue;
+    const int lr = rhs_line_threads(p.h, sizeof(T) == 4), lc = rhs_line_threads(p.ny, sizeof(T) == 4);
+    for (int rb : {1, 2, 4, 8, 16, 32}) {
+        if (lr ? rb * lr > 512 || rb * lr < 32 : rb > 4 || 2 * (size_t)rb * p.h * sizeof(C2) > (size_t)optin) continue;
         for (int rt : {128, 256, 512, 1024}) {
-            if (rt > 128 && rt > rb * p.h / 2) continue;   // at most one element pair per thread
+            if (rt > 128 && (lr || rt > rb * p.h / 2)) continue;   // at most one element pair per thread
             p.rb = rb;
             p.rt = rt;
             const float t = time_it([&] {
@@ -837,10 +841,11 @@ template <typename T> void tune_conv_shapes(fi_handle* h)
     }
     p.rb = best_rb;
     p.rt = best_rt;
-    for (int cb : {1, 2, 4}) {
-        if (2 * (size_t)cb * (p.ny + 1) * sizeof(C2) > (size_t)optin) continue;
+    for (int cb : {1, 2, 4, 8, 16}) {
+        if (lc ? (cb * lc > 1024 || cb * lc < 32) && cb > 1
+               : cb > 4 || 2 * (size_t)cb * (p.ny + 1) * sizeof(C2) > (size_t)optin) continue;
         for (int ct : {128, 256, 512, 1024}) {
-            if (ct > 128 && ct > cb * p.ny / 2) continue;
+            if (ct > 128 && (lc || ct > cb * p.ny / 2)) continue;
             p.cb = cb;
             p.ct = ct;
             const float t = time_it([&] {
@@ -2421,10 +2426,31 @@ int batch_shape(fi_batch* b, int RB, int CB, int fseg, int waves)
     const size_t c2 = b->mixed ? sizeof(float2) : sizeof(double2);
     b->rows_threads = b->cols_threads = 0;
     b->rows_smem = b->cols_smem = 0;
-    for (int i = 0; i < n; ++i) {
-        BMember& m = b->hM[i];
+    // threads of a transform block: the most any member's shape asks for; a
+    // member on register lines then takes as many lines as they make
+    auto shape_of = [&](BMember& m, int& rt, int& ct) {
         m.RB = RB > 0 ? RB : rhs_rows_per_block(m.p.h);
         m.CB = CB > 0 ? CB : (b->mixed ? rhs_cols_per_block<float>(m.p.ny) : rhs_cols_per_block<double>(m.p.ny));
+        const int lr = rhs_line_threads(m.p.h, b->mixed), lc = rhs_line_threads(m.p.ny, b->mixed);
+        m.lines = (lr > 0 ? 1 : 0) | (lc > 0 ? 2 : 0);
+        auto line_block = [](int lines, int th) {
+            int t = lines * th;
+            while (t > 512) t /= 2;
+            return t < th ? th : t < 32 ? 32 : t;
+        };
+        rt = lr > 0 ? line_block(m.RB, lr) : rhs_threads_for(m.RB * m.p.h / 4);
+        ct = lc > 0 ? line_block(m.CB, lc) : rhs_threads_for(m.CB * m.p.ny / 4);
+    };
+    for (int i = 0; i < n; ++i) {
+        int rt, ct;
+        shape_of(b->hM[i], rt, ct);
+        if (rt > b->rows_threads) b->rows_threads = rt;
+        if (ct > b->cols_threads) b->cols_threads = ct;
+    }
+    for (int i = 0; i < n; ++i) {
+        BMember& m = b->hM[i];
+        if (m.lines & 1) m.RB = b->rows_threads / rhs_line_threads(m.p.h, b->mixed);
+        if (m.lines & 2) m.CB = b->cols_threads / rhs_line_threads(m.p.ny, b->mixed);
         m.fseg = fseg;
         const int fblk = (b->mixed && (!b->true_stages || m.yhi)) ? batch_flexure_blocks(m.p.nx, m.p.ny, m.fseg)
                                                                   : m.fgx * ((m.p.ny + 7) / 8);
@@ -2434,10 +2460,10 @@ int batch_shape(fi_batch* b, int RB, int CB, int fseg, int waves)
         off[(n + 1) + i + 1] = off[(n + 1) + i] + rblk;
         off[2 * (n + 1) + i + 1] = off[2 * (n + 1) + i] + cblk;
         off[3 * (n + 1) + i + 1] = off[3 * (n + 1) + i] + m.red_nblk;
-        const int rt = rhs_threads_for(m.RB * m.p.h / 4), ct = rhs_threads_for(m.CB * m.p.ny / 4);
-        if (rt > b->rows_threads) b->rows_threads = rt;
-        if (ct > b->cols_threads) b->cols_threads = ct;
-        const size_t rs = 2 * (size_t)m.RB * m.p.h * c2, cs = 2 * (size_t)m.CB * (m.p.ny + 1) * c2;   // padded columns
+        const size_t rs = (m.lines & 1) ? (size_t)m.RB * rhs_line_bytes(m.p.h, b->mixed)
+                                        : 2 * (size_t)m.RB * m.p.h * c2;
+        const size_t cs = (m.lines & 2) ? (size_t)m.CB * rhs_line_bytes(m.p.ny, b->mixed)
+                                        : 2 * (size_t)m.CB * (m.p.ny + 1) * c2;   // padded columns
         if (rs > b->rows_smem) b->rows_smem = rs;
         if (cs > b->cols_smem) b->cols_smem = cs;
     }

@@ -41,6 +41,7 @@ struct BMember {
     const float *wrhi, *wrlo;
     int even;
     int RB, CB;               // rows per row block, columns per column block
+    int lines;                // transforms on register lines: bit 0 rows, bit 1 columns
     int fgx;                  // flexure blocks along x (FP64 tiles)
     int fseg;                 // output rows per flexure warp task (mixed column strips)
     int red_nblk;             // blocks of the reduction kernels
@@ -85,6 +86,8 @@ int batch_flexure_blocks(int nx, int ny, int seg);
 // Block shapes of the single-domain launches (shared with the batched ones).
 int rhs_rows_per_block(int h);
 int rhs_threads_for(int work);
+int rhs_line_threads(int n, bool f32);      // threads of a register line of n points, 0: none
+size_t rhs_line_bytes(int n, bool f32);     // its shared memory
 template <typename T> int rhs_cols_per_block(int ny);
 int reduce_grid(size_t n);
 int ts_grid(size_t n);           // blocks of the Tsit5 attempt reductions

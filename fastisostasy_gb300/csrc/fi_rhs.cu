@@ -24,6 +24,7 @@
 
 #include "fi_batch.h"
 #include "fi_kernels.h"
+#include "fi_lines.cuh"
 
 namespace fi {
 
@@ -729,6 +730,7 @@ void launch_rows_fwd(const T* in, int in_pitch, int in_width, int nrows_in, type
                      const Plan2D& p, cudaStream_t s, const int* gate)
 {
     typedef typename vec2<T>::type C2;
+    if (lines_rows_fwd<T>(in, in_pitch, in_width, nrows_in, S, p, s, gate)) return;
     const int RB = p.rb > 0 ? p.rb : rows_per_block(p.h);
     const size_t sm = 2 * (size_t)RB * p.h * sizeof(C2);
     set_smem(k_rows_fwd<T>, sm);
@@ -791,6 +793,7 @@ void launch_rows_inv(const typename vec2<T>::type* S, T* out, const Plan2D& p, d
                      const int* gate)
 {
     typedef typename vec2<T>::type C2;
+    if (lines_rows_inv<T>(S, out, p, scale, s, gate)) return;
     const int RB = p.rb > 0 ? p.rb : rows_per_block(p.h);
     const size_t sm = 2 * (size_t)RB * p.h * sizeof(C2);
     set_smem(k_rows_inv<T>, sm);
@@ -901,6 +904,7 @@ void launch_cols_hartley(typename vec2<T>::type* S, const T* mA, const T* mB, in
                          cudaStream_t s, const int* gate)
 {
     typedef typename vec2<T>::type C2;
+    if (lines_cols_hartley<T>(S, mA, mB, even, p, s, gate)) return;
     const int CB = p.cb > 0 ? p.cb : cols_per_block<T>(p.ny);
     const size_t sm = 2 * (size_t)CB * col_stride(p.ny) * sizeof(C2);
     set_smem(k_cols_hartley<T>, sm);
@@ -951,6 +955,7 @@ void launch_cols_conv(typename vec2<T>::type* S, const typename vec2<T>::type* K
                       int n_out, const Plan2D& p, cudaStream_t s)
 {
     typedef typename vec2<T>::type C2;
+    if (lines_cols_conv<T>(S, K, nrows_in, n_out, p, s)) return;
     const int CB = p.cb > 0 ? p.cb : cols_per_block<T>(p.ny);
     const size_t sm = 2 * (size_t)CB * col_stride(p.ny) * sizeof(C2);
     set_smem(k_cols_conv<T>, sm);
@@ -1030,6 +1035,7 @@ void launch_conv_rows_inv(const typename vec2<T>::type* S, int n_out, double* ou
                           const Plan2D& p, double scale, cudaStream_t s)
 {
     typedef typename vec2<T>::type C2;
+    if (lines_conv_rows_inv<T>(S, n_out, out, nx, ny, i_off, corners, corner_col1, p, scale, s)) return;
     const int RB = p.rb > 0 ? p.rb : rows_per_block(p.h);
     const size_t sm = 2 * (size_t)RB * p.h * sizeof(C2);
     set_smem(k_conv_rows_inv<T>, sm);
@@ -1045,6 +1051,14 @@ void launch_conv_rows_inv(const typename vec2<T>::type* S, int n_out, double* ou
 int rhs_rows_per_block(int h) { return rows_per_block(h); }
 int rhs_threads_for(int work) { return threads_for(work); }
 template <typename T> int rhs_cols_per_block(int ny) { return cols_per_block<T>(ny); }
+int rhs_line_threads(int n, bool f32)
+{
+    // the batched kernels carry every line length they take; one that a
+    // single domain would transform on lines has to be among them, or the
+    // member would not get the bits it gets alone
+    return f32 ? line_threads<float>(n) : line_threads<double>(n);
+}
+size_t rhs_line_bytes(int n, bool f32) { return f32 ? line_bytes<float>(n) : line_bytes<double>(n); }
 template int rhs_cols_per_block<float>(int);
 template int rhs_cols_per_block<double>(int);
 
@@ -1070,29 +1084,41 @@ __global__ void __launch_bounds__(256) k_b_flexure(const BMember* __restrict__ M
 }
 
 template <typename T>
-__global__ void k_b_rows_fwd(const BMember* __restrict__ M, BList L)
+__global__ void __launch_bounds__(512) k_b_rows_fwd(const BMember* __restrict__ M, BList L)
 {
     typedef typename vec2<T>::type C2;
     batch_walk(L, [&](int m) { return true; }, [&](int m, int local) {   // the list holds the members with work
         const BMember& b = M[m];
-        rows_fwd_body<T>((const T*)b.f, b.p.nx, b.p.nx, b.p.ny, (C2*)b.S, b.p, b.RB, local, 0);
+        if (b.lines & 1) {
+#define FI_GO(N) rows_fwd_lines<T, N>((const T*)b.f, b.p.nx, b.p.nx, b.p.ny, (C2*)b.S, b.p, local)
+            FI_LINE_SWITCH(b.p.h, FI_GO)
+#undef FI_GO
+        } else {
+            rows_fwd_body<T>((const T*)b.f, b.p.nx, b.p.nx, b.p.ny, (C2*)b.S, b.p, b.RB, local, 0);
+        }
         __syncthreads();
     });
 }
 
 template <typename T>
-__global__ void k_b_cols_hartley(const BMember* __restrict__ M, BList L)
+__global__ void __launch_bounds__(512) k_b_cols_hartley(const BMember* __restrict__ M, BList L)
 {
     typedef typename vec2<T>::type C2;
     batch_walk(L, [&](int m) { return true; }, [&](int m, int local) {   // the list holds the members with work
         const BMember& b = M[m];
-        cols_hartley_body<T>((C2*)b.S, (const T*)b.mA, (const T*)b.mB, b.even, b.p, b.CB, local, 0);
+        if (b.lines & 2) {
+#define FI_GO(N) cols_hartley_lines<T, N>((C2*)b.S, (const T*)b.mA, (const T*)b.mB, b.even, b.p, local)
+            FI_LINE_SWITCH(b.p.ny, FI_GO)
+#undef FI_GO
+        } else {
+            cols_hartley_body<T>((C2*)b.S, (const T*)b.mA, (const T*)b.mB, b.even, b.p, b.CB, local, 0);
+        }
         __syncthreads();
     });
 }
 
 template <typename T>
-__global__ void k_b_rows_inv(const BMember* __restrict__ M, BList L, int stage)
+__global__ void __launch_bounds__(512) k_b_rows_inv(const BMember* __restrict__ M, BList L, int stage)
 {
     typedef typename vec2<T>::type C2;
     batch_walk(L, [&](int m) { return true; }, [&](int m, int local) {
@@ -1100,7 +1126,13 @@ __global__ void k_b_rows_inv(const BMember* __restrict__ M, BList L, int stage)
         T scale;   // 1/(nx*ny*1.), converted on the host
         if constexpr (sizeof(T) == 4) scale = b.norm_scale_f;
         else scale = b.norm_scale;
-        rows_inv_body<T>((const C2*)b.S, b.p.ny, (T*)b.raw7[stage], b.p.nx, b.p, b.RB, scale, local, 0);
+        if (b.lines & 1) {
+#define FI_GO(N) rows_inv_lines<T, N>((const C2*)b.S, b.p.ny, (T*)b.raw7[stage], b.p.nx, b.p, scale, local)
+            FI_LINE_SWITCH(b.p.h, FI_GO)
+#undef FI_GO
+        } else {
+            rows_inv_body<T>((const C2*)b.S, b.p.ny, (T*)b.raw7[stage], b.p.nx, b.p, b.RB, scale, local, 0);
+        }
         __syncthreads();
     });
 }
