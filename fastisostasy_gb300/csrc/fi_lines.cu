@@ -1,9 +1,13 @@
 // fi_lines.cu — transforms of one domain on register lines (fi_rfft.cuh):
-// row and column passes of the RHS and of the convolutions for power-of-two
-// lengths.
+// row and column passes of the RHS and of the convolutions for the lengths
+// that have one.
 #include <mutex>
 
 #include "fi_lines.cuh"
+
+#ifndef FI_LINES_T   // one translation unit per precision (fi_lines64.cu)
+#define FI_LINES_T float
+#endif
 
 namespace fi {
 
@@ -90,7 +94,7 @@ k_lines_conv_rows_inv(const typename vec2<T>::type* __restrict__ S, int n_out, d
     const bool live = j < n_out;
     const size_t jj = live ? j : 0;
     C2 v[E];
-    line_rows_inv<T, H, WARP>(S + jj * p.sp, v, sm, LineTab<T>::tw(p.row), LineTab<T>::rtw(p), t, live);
+    line_rows_inv<T, H, WARP>([&](int k) { return S[jj * p.sp + k]; }, v, sm, LineTab<T>::tw(p.row), LineTab<T>::rtw(p), t, live);
     if (!live) return;
 #pragma unroll
     for (int m = 0; m < E; ++m) {
@@ -201,6 +205,7 @@ bool lines_cols_conv(typename vec2<T>::type* S, const typename vec2<T>::type* K,
     FI_LAUNCH(k_lines_cols_conv, N, (p.cb > 0 ? p.cb : line_default<T, N, true>()), p.h + 1, S, K, nrows_in, p)
     FI_LINE_SWITCH(p.ny, FI_GO)
     if (p.ny == 4096) FI_GO(4096);
+    if (p.ny == 3072) FI_GO(3072);
 #undef FI_GO
     return true;
 }
@@ -227,7 +232,6 @@ bool lines_conv_rows_inv(const typename vec2<T>::type* S, int n_out, double* out
     template bool lines_cols_conv<T>(vec2<T>::type*, const vec2<T>::type*, int, int, const Plan2D&, cudaStream_t); \
     template bool lines_conv_rows_inv<T>(const vec2<T>::type*, int, double*, int, int, int, double*, int,         \
                                          const Plan2D&, double, cudaStream_t);
-FI_LINES_INST(float)
-FI_LINES_INST(double)
+FI_LINES_INST(FI_LINES_T)
 
 }  // namespace fi

@@ -1,4 +1,4 @@
-// fi_lines.cuh — row and column passes over power-of-two lines, shared by the
+// fi_lines.cuh — row and column passes over register lines, shared by the
 // single-domain kernels (fi_lines.cu) and the batched ones (fi_rhs.cu).
 //
 // A block holds blockDim.x / T lines of T threads each (LineShape).  Rows lie
@@ -24,42 +24,32 @@ template <> struct LineTab<double> {
 
 // Threads of a line of n points, 0 where there is no such line kernel (the
 // shared-memory transforms of fi_fft.cuh take every other length).
+inline bool has_line(int n)
+{
+    const int m = n % 3 == 0 ? n / 3 : n;
+    return (m & (m - 1)) == 0 && n >= (n % 3 == 0 ? 24 : 16) && n <= 4096;
+}
 template <typename T> inline int line_threads(int n)
 {
-    switch (n) {
-    case 16: return LineShape<T, 16>::threads;
-    case 32: return LineShape<T, 32>::threads;
-    case 64: return LineShape<T, 64>::threads;
-    case 128: return LineShape<T, 128>::threads;
-    case 256: return LineShape<T, 256>::threads;
-    case 512: return LineShape<T, 512>::threads;
-    case 1024: return LineShape<T, 1024>::threads;
-    case 2048: return LineShape<T, 2048>::threads;
-    case 4096: return LineShape<T, 4096>::threads;
-    }
-    return 0;
+    return has_line(n) ? n / line_points(n, sizeof(T) == 4) : 0;
 }
-// Shared memory of one line.
+// points of shared memory of one line (line_smem)
+__host__ __device__ constexpr int line_room(int n, bool f32)
+{
+    const int e = line_points(n, f32), pad = (e & (e - 1)) == 0 ? e : 16;
+    return ((n + n / pad + 15) / 16) * 16 + 2;
+}
+static_assert(line_room(192, true) == line_smem<float, 192>() && line_room(2048, true) == line_smem<float, 2048>() &&
+                  line_room(96, false) == line_smem<double, 96>(), "one layout");
 template <typename T> inline size_t line_bytes(int n)
 {
-    switch (n) {
-    case 16: return line_smem<T, 16>() * 2 * sizeof(T);
-    case 32: return line_smem<T, 32>() * 2 * sizeof(T);
-    case 64: return line_smem<T, 64>() * 2 * sizeof(T);
-    case 128: return line_smem<T, 128>() * 2 * sizeof(T);
-    case 256: return line_smem<T, 256>() * 2 * sizeof(T);
-    case 512: return line_smem<T, 512>() * 2 * sizeof(T);
-    case 1024: return line_smem<T, 1024>() * 2 * sizeof(T);
-    case 2048: return line_smem<T, 2048>() * 2 * sizeof(T);
-    case 4096: return line_smem<T, 4096>() * 2 * sizeof(T);
-    }
-    return 0;
+    return has_line(n) ? line_room(n, sizeof(T) == 4) * 2 * sizeof(T) : 0;
 }
 // largest block of the line kernels: 16 points a thread or double points
 // need up to 128 registers
 template <typename T, int N> constexpr int line_block_max()
 {
-    return sizeof(T) == 8 || LineShape<T, N>::E == 16 ? 512 : 1024;
+    return sizeof(T) == 8 || LineShape<T, N>::E > 8 ? 512 : 1024;
 }
 
 template <typename T, int H>
@@ -75,8 +65,15 @@ __device__ __forceinline__ void rows_fwd_lines(const T* __restrict__ in, int pit
     C2* sm = reinterpret_cast<C2*>(smem_raw) + (size_t)line * line_smem<T, H>();
     const bool live = j < nrows;
     const size_t jj = live ? j : 0;
-    line_rows_fwd<T, H, WARP>(in + jj * pitch, (pitch & 1) == 0, width, S + jj * p.sp, sm, LineTab<T>::tw(p.row),
-                              LineTab<T>::rtw(p), t, live);
+    const T* row = in + jj * pitch;
+    C2* out = S + jj * p.sp;
+    const bool pairs = (pitch & 1) == 0;
+    line_rows_fwd<T, H, WARP>(
+        [&](int i) {
+            if (i + 1 < width) return pairs ? *reinterpret_cast<const C2*>(row + i) : mk2<T>(row[i], row[i + 1]);
+            return mk2<T>(i < width ? row[i] : (T)0, (T)0);
+        },
+        [&](int k, C2 v) { out[k] = v; }, sm, LineTab<T>::tw(p.row), LineTab<T>::rtw(p), t, live);
 }
 
 template <typename T, int H>
@@ -93,7 +90,7 @@ __device__ __forceinline__ void rows_inv_lines(const typename vec2<T>::type* __r
     const bool live = j < nrows;
     const size_t jj = live ? j : 0;
     C2 v[E];
-    line_rows_inv<T, H, WARP>(S + jj * p.sp, v, sm, LineTab<T>::tw(p.row), LineTab<T>::rtw(p), t, live);
+    line_rows_inv<T, H, WARP>([&](int k) { return S[jj * p.sp + k]; }, v, sm, LineTab<T>::tw(p.row), LineTab<T>::rtw(p), t, live);
     if (!live) return;
 #pragma unroll
     for (int m = 0; m < E; ++m)
@@ -114,17 +111,21 @@ __device__ __forceinline__ void cols_hartley_lines(typename vec2<T>::type* __res
     C2* sm = reinterpret_cast<C2*>(smem_raw) + (size_t)c * line_smem<T, N>();
     const C2* tw = LineTab<T>::tw(p.col);
     C2 v[E];
-    T fa[E];   // even factors, requested with the column
+    constexpr bool AHEAD = E <= 16;   // request the even factors with the column, registers allowing
+    T fa[E];
 #pragma unroll
     for (int m = 0; m < E; ++m) {
         const size_t e = (size_t)(t + TH * m) * p.sp + k;
         v[m] = live ? S[e] : mk2<T>((T)0, (T)0);
-        fa[m] = (live && even) ? __ldg(mA + e) : (T)0;
+        if (AHEAD) fa[m] = (live && even) ? __ldg(mA + e) : (T)0;
     }
     line_fft<T, N, -1, false>(v, sm, tw, t);
     if (even) {
 #pragma unroll
-        for (int m = 0; m < E; ++m) v[m] = cscale(v[m], fa[m]);
+        for (int m = 0; m < E; ++m) {
+            if (!AHEAD) fa[m] = live ? __ldg(mA + (size_t)(t + TH * m) * p.sp + k) : (T)0;
+            v[m] = cscale(v[m], fa[m]);
+        }
     } else {
         // Hartley values at (k,l), (-k,-l), (-k,l), (k,-l)
         __syncthreads();
@@ -133,7 +134,7 @@ __device__ __forceinline__ void cols_hartley_lines(typename vec2<T>::type* __res
         __syncthreads();
 #pragma unroll
         for (int m = 0; m < E; ++m) {
-            const int l = t + TH * m, lm = (N - l) & (N - 1);
+            const int l = t + TH * m, lm = l == 0 ? 0 : N - l;
             const size_t ia = (size_t)l * p.sp + k, ib = (size_t)lm * p.sp + k;
             const C2 Fa = v[m], Fb = sm[line_pad<E>(lm)];
             const T H_kl = Fb.x - Fa.y, H_mkml = Fb.x + Fa.y;
@@ -154,6 +155,13 @@ __device__ __forceinline__ void cols_hartley_lines(typename vec2<T>::type* __res
 #define FI_LINE_SWITCH(n, FN) \
     switch (n) {              \
     case 16: FN(16); break;   \
+    case 24: FN(24); break;   \
+    case 48: FN(48); break;   \
+    case 96: FN(96); break;   \
+    case 192: FN(192); break; \
+    case 384: FN(384); break; \
+    case 768: FN(768); break; \
+    case 1536: FN(1536); break; \
     case 32: FN(32); break;   \
     case 64: FN(64); break;   \
     case 128: FN(128); break; \

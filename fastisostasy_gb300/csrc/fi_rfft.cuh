@@ -1,4 +1,4 @@
-// fi_rfft.cuh — power-of-two FFT lines with the points in registers.
+// fi_rfft.cuh — FFT lines of 2^k and 3 2^k points, the points in registers.
 //
 // T = N/E threads share one line of N complex points; thread t holds the E
 // points x[t + T m], m < E, before every stage, and after the last one again
@@ -20,8 +20,8 @@
 // 10.3, 8.8 -> 7.9 us.  FP64, bound by the FP64 pipe (2 instructions a clock
 // and SM), gains the smaller operation count: 1024^2 52 -> 43, 94 -> 80,
 // 50 -> 43 us, 512^2 20.9 -> 16.1, 30.9 -> 24.2, 19.1 -> 15.3 us.
-// Every power of two from 16 on takes this form (faster at each one
-// measured); the other lengths keep the shared-memory stages.
+// Lengths 2^k from 16 and 3 2^k from 24 on take this form (faster at each one
+// measured); the others keep the shared-memory stages.
 #pragma once
 
 #include "fi_fft.cuh"
@@ -30,15 +30,27 @@ namespace fi {
 
 // points per thread: 8 keeps a double-precision line at 32 data registers;
 // 16 saves an exchange where a float line is long (1024 = 16 16 4 against
-// 8 8 8 2)
+// 8 8 8 2).  Lengths 3 2^k: 12 (radices 4, 2 and a last 3), or 24 (8, 4, 2, 3)
+// where a float line is long.
+__host__ __device__ constexpr int line_points(int n, bool f32)
+{
+    return n % 3 == 0 ? (f32 && n >= 768 ? 24 : 12) : f32 && n >= 1024 ? 16 : 8;
+}
 template <typename T, int N> struct LineShape {
-    static constexpr int E = (sizeof(T) == 4 && N >= 1024) ? 16 : (N >= 8 ? 8 : N);
+    static constexpr int E = line_points(N, sizeof(T) == 4);
     static constexpr int threads = N / E;
 };
+// radix of the stage that has `rem` = N / Ns left: the powers of two first
+constexpr int line_radix(int E, int rem)
+{
+    const int most = E == 24 ? 8 : E == 12 ? 4 : E;
+    const int p2 = rem % 3 == 0 ? rem / 3 : rem;
+    return p2 > 1 ? (p2 < most ? p2 : most) : rem;
+}
 
-// index of point i in shared memory: one point of padding per E points, so
-// the strided stores of a stage fall in different banks
-template <int E> __host__ __device__ constexpr int line_pad(int i) { return i + i / E; }
+// index of point i in shared memory: one point of padding per E (or 16)
+// points, so the strided stores of a stage fall in different banks
+template <int E> __host__ __device__ constexpr int line_pad(int i) { return i + i / ((E & (E - 1)) == 0 ? E : 16); }
 template <typename T, int N> __host__ __device__ constexpr int line_smem()
 {
     // an odd multiple of two points: lines side by side start two banks apart
@@ -138,6 +150,16 @@ template <typename T, typename C2, int SIGN> __device__ __forceinline__ void rdf
         }
 }
 
+template <typename T, typename C2, int SIGN> __device__ __forceinline__ void rdft3(C2& a, C2& b, C2& c)
+{
+    const T s1 = (T)(SIGN < 0 ? -0.86602540378443864676372317075293618 : 0.86602540378443864676372317075293618);
+    const C2 s = cadd(b, c), d = csub(b, c);
+    const C2 m = mk2<T>(a.x - (T)0.5 * s.x, a.y - (T)0.5 * s.y);
+    a = cadd(a, s);
+    b = mk2<T>(m.x - s1 * d.y, m.y + s1 * d.x);
+    c = mk2<T>(m.x + s1 * d.y, m.y - s1 * d.x);
+}
+
 // Barrier among the threads of a line: a warp barrier where a line never
 // leaves a warp (WARP), else the block's.
 template <bool WARP> __device__ __forceinline__ void line_sync()
@@ -150,13 +172,13 @@ template <bool WARP> __device__ __forceinline__ void line_sync()
 // sm: the line's shared memory; tw: exp(-2 pi i k / N).  Every thread of the
 // block calls it (threads without a line pass live = false: they only keep
 // the barriers).
-template <typename T, int N, int SIGN, bool WARP, int Ns>
+template <typename T, int N, int SIGN, bool WARP, bool TWSH, int Ns>
 __device__ __forceinline__ void line_stages(typename vec2<T>::type* v, typename vec2<T>::type* sm,
                                             const typename vec2<T>::type* __restrict__ tw, int t)
 {
     typedef typename vec2<T>::type C2;
     constexpr int E = LineShape<T, N>::E, TH = LineShape<T, N>::threads;
-    constexpr int R = N / Ns < E ? N / Ns : E;
+    constexpr int R = line_radix(E, N / Ns);
     constexpr int NB = E / R;                      // butterflies per thread
     C2 u[NB][R];
 #pragma unroll
@@ -166,9 +188,7 @@ __device__ __forceinline__ void line_stages(typename vec2<T>::type* v, typename 
         for (int r = 0; r < R; ++r) {
             C2 a = v[b + NB * r];
             if (Ns > 1 && r > 0) {
-                C2 w = __ldg(tw + jm * r * (N / (Ns * R)));
-                if (SIGN > 0) w.y = -w.y;
-                a = cmul(a, w);
+                a = cmul(a, tw_load<T, C2, TWSH>(tw, jm * r * (N / (Ns * R)), SIGN));
             }
             u[b][r] = a;
         }
@@ -176,6 +196,8 @@ __device__ __forceinline__ void line_stages(typename vec2<T>::type* v, typename 
             const C2 a = u[b][0], c = u[b][1 % R];
             u[b][0] = cadd(a, c);
             u[b][1 % R] = csub(a, c);
+        } else if (R == 3) {
+            rdft3<T, C2, SIGN>(u[b][0], u[b][1 % R], u[b][2 % R]);
         } else if (R == 4) {
             rdft4<T, C2, SIGN>(u[b][0], u[b][1 % R], u[b][2 % R], u[b][3 % R]);
         } else if (R == 8) {
@@ -195,7 +217,7 @@ __device__ __forceinline__ void line_stages(typename vec2<T>::type* v, typename 
         line_sync<WARP>();
 #pragma unroll
         for (int m = 0; m < E; ++m) v[m] = sm[line_pad<E>(t + TH * m)];
-        line_stages<T, N, SIGN, WARP, Ns * R>(v, sm, tw, t);
+        line_stages<T, N, SIGN, WARP, TWSH, Ns * R>(v, sm, tw, t);
     } else {
 #pragma unroll
         for (int b = 0; b < NB; ++b)
@@ -204,11 +226,12 @@ __device__ __forceinline__ void line_stages(typename vec2<T>::type* v, typename 
     }
 }
 
-template <typename T, int N, int SIGN, bool WARP>
+// TWSH: the twiddles are in shared memory
+template <typename T, int N, int SIGN, bool WARP, bool TWSH = false>
 __device__ __forceinline__ void line_fft(typename vec2<T>::type* v, typename vec2<T>::type* sm,
                                          const typename vec2<T>::type* __restrict__ tw, int t)
 {
-    line_stages<T, N, SIGN, WARP, 1>(v, sm, tw, t);
+    line_stages<T, N, SIGN, WARP, TWSH, 1>(v, sm, tw, t);
 }
 
 // ---------------------------------------------------------------------------
@@ -219,10 +242,9 @@ __device__ __forceinline__ void line_fft(typename vec2<T>::type* v, typename vec
 // H-point transform, then X[k] and X[H-k] from Z[k] and Z[H-k] together:
 // with E = (Z[k] + conj Z[H-k])/2 and W = w^k (Z[k] - conj Z[H-k])/(2i),
 // X[k] = E + W and X[H-k] = conj(E - W).
-template <typename T, int H, bool WARP>
-__device__ __forceinline__ void line_rows_fwd(const T* __restrict__ row, bool pairs, int width,
-                                              typename vec2<T>::type* __restrict__ out,
-                                              typename vec2<T>::type* sm,
+// load(i): samples i and i + 1 of the row (i even); store(k, X[k]).
+template <typename T, int H, bool WARP, bool TWSH = false, typename Load, typename Store>
+__device__ __forceinline__ void line_rows_fwd(Load load, Store store, typename vec2<T>::type* sm,
                                               const typename vec2<T>::type* __restrict__ tw,
                                               const typename vec2<T>::type* __restrict__ rtw, int t, bool live)
 {
@@ -230,20 +252,8 @@ __device__ __forceinline__ void line_rows_fwd(const T* __restrict__ row, bool pa
     constexpr int E = LineShape<T, H>::E, TH = LineShape<T, H>::threads;
     C2 v[E];
 #pragma unroll
-    for (int m = 0; m < E; ++m) {
-        const int i = 2 * (t + TH * m);
-        C2 a = mk2<T>((T)0, (T)0);
-        if (live) {
-            if (i + 1 < width) {
-                if (pairs) a = *reinterpret_cast<const C2*>(row + i);
-                else a = mk2<T>(row[i], row[i + 1]);
-            } else if (i < width) {
-                a = mk2<T>(row[i], (T)0);
-            }
-        }
-        v[m] = a;
-    }
-    line_fft<T, H, -1, WARP>(v, sm, tw, t);
+    for (int m = 0; m < E; ++m) v[m] = live ? load(2 * (t + TH * m)) : mk2<T>((T)0, (T)0);
+    line_fft<T, H, -1, WARP, TWSH>(v, sm, tw, t);
     line_sync<WARP>();
 #pragma unroll
     for (int m = 0; m < E; ++m) sm[line_pad<E>(t + TH * m)] = v[m];
@@ -255,10 +265,10 @@ __device__ __forceinline__ void line_rows_fwd(const T* __restrict__ row, bool pa
         const int k = t + TH * q;
         const C2 Zk = v[q];                        // point t + TH q
         if (k == 0) {
-            out[0] = mk2<T>(Zk.x + Zk.y, (T)0);
-            out[H] = mk2<T>(Zk.x - Zk.y, (T)0);
+            store(0, mk2<T>(Zk.x + Zk.y, (T)0));
+            store(H, mk2<T>(Zk.x - Zk.y, (T)0));
             const C2 Zm = sm[line_pad<E>(H / 2)];
-            out[H / 2] = mk2<T>(Zm.x, -Zm.y);
+            store(H / 2, mk2<T>(Zm.x, -Zm.y));
         } else {
             const C2 Zc = sm[line_pad<E>(H - k)];
             C2 Ev, O;
@@ -266,9 +276,9 @@ __device__ __forceinline__ void line_rows_fwd(const T* __restrict__ row, bool pa
             Ev.y = half * (Zk.y - Zc.y);
             O.x = half * (Zk.y + Zc.y);
             O.y = half * (Zc.x - Zk.x);
-            const C2 W = cmul(__ldg(rtw + k), O);
-            out[k] = cadd(Ev, W);
-            out[H - k] = mk2<T>(Ev.x - W.x, W.y - Ev.y);
+            const C2 W = cmul(tw_load<T, C2, TWSH>(rtw, k, -1), O);
+            store(k, cadd(Ev, W));
+            store(H - k, mk2<T>(Ev.x - W.x, W.y - Ev.y));
         }
     }
 }
@@ -276,8 +286,9 @@ __device__ __forceinline__ void line_rows_fwd(const T* __restrict__ row, bool pa
 // Half spectrum of a row -> the H-point line whose inverse transform is the
 // packed real row: with s = X[k] + conj X[H-k] and u = conj(w^k) (X[k] -
 // conj X[H-k]), z[k] = s + i u and z[H-k] = conj(s) + i conj(u).
-template <typename T, int H, bool WARP>
-__device__ __forceinline__ void line_rows_inv(const typename vec2<T>::type* __restrict__ X,
+// X(k): the spectrum value k.
+template <typename T, int H, bool WARP, bool TWSH = false, typename Load>
+__device__ __forceinline__ void line_rows_inv(Load X,
                                               typename vec2<T>::type* v, typename vec2<T>::type* sm,
                                               const typename vec2<T>::type* __restrict__ tw,
                                               const typename vec2<T>::type* __restrict__ rtw, int t, bool live)
@@ -288,15 +299,15 @@ __device__ __forceinline__ void line_rows_inv(const typename vec2<T>::type* __re
 #pragma unroll
         for (int q = 0; q < E / 2; ++q) {
             const int k = t + TH * q;
-            const C2 A = X[k], B = X[H - k];
+            const C2 A = X(k), B = X(H - k);
             if (k == 0) {
                 // the imaginary parts of X[0] and X[H] do not enter a real row's transform
-                const C2 M = X[H / 2];
+                const C2 M = X(H / 2);
                 sm[0] = mk2<T>(A.x + B.x, A.x - B.x);
                 sm[line_pad<E>(H / 2)] = mk2<T>((T)2 * M.x, (T)-2 * M.y);
             } else {
                 const C2 s = mk2<T>(A.x + B.x, A.y - B.y), d = mk2<T>(A.x - B.x, A.y + B.y);
-                const C2 u = cmulc(d, __ldg(rtw + k));
+                const C2 u = cmulc(d, tw_load<T, C2, TWSH>(rtw, k, -1));
                 sm[line_pad<E>(k)] = mk2<T>(s.x - u.y, s.y + u.x);
                 sm[line_pad<E>(H - k)] = mk2<T>(s.x + u.y, u.x - s.y);
             }
@@ -305,7 +316,7 @@ __device__ __forceinline__ void line_rows_inv(const typename vec2<T>::type* __re
     line_sync<WARP>();
 #pragma unroll
     for (int m = 0; m < E; ++m) v[m] = sm[line_pad<E>(t + TH * m)];
-    line_fft<T, H, +1, WARP>(v, sm, tw, t);
+    line_fft<T, H, +1, WARP, TWSH>(v, sm, tw, t);
 }
 
 }  // namespace fi

@@ -1,4 +1,4 @@
-"""Transforms on register lines: every power-of-two length they take, both
+"""Transforms on register lines: every length they take, both
 Hartley forms, against the oracle and a direct linear convolution.
 
 Tolerances are the ones the right-hand side and the convolutions are held to
@@ -31,7 +31,8 @@ def _domain(name, nx, ny, precision):
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("nx,ny,even", [(32, 2048, False), (32, 2048, True), (64, 1024, False), (128, 512, True),
                                         (512, 32, False), (1024, 16, True), (2048, 64, False), (256, 48, False),
-                                        (2048, 34, True)])
+                                        (2048, 34, True), (48, 1536, False), (1536, 96, True), (384, 192, False),
+                                        (768, 24, True), (96, 768, False)])
 def test_rate_on_lines(nx, ny, even, precision):
     dom, p = _domain("test1d", nx, ny, precision)
     rng = np.random.default_rng(nx + ny)
@@ -57,7 +58,7 @@ def linear_convolution(G, x):
 
 
 @pytest.mark.parametrize("precision", [0, 1])
-@pytest.mark.parametrize("nx,ny", [(2048, 32), (32, 2048), (16, 16), (512, 64), (64, 1024)])
+@pytest.mark.parametrize("nx,ny", [(2048, 32), (32, 2048), (16, 16), (512, 64), (64, 1024), (1536, 48), (48, 1536), (192, 96)])
 def test_convolution_on_lines(nx, ny, precision):
     dom, _ = _domain("test2c", nx, ny, precision)
     x = np.random.default_rng(nx).standard_normal((ny, nx)) * 1e7
