@@ -24,6 +24,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include "../../include/fi_gpu.h"
+#include "fi_cluster.h"
 #include "fi_engine.h"
 #include "fi_init.h"
 #include "fi_kernels.h"
@@ -243,6 +244,10 @@ struct fi_handle {
     bool require_tsit_graph = false;   // FI_REQUIRE_TSIT_GRAPH=1: no host-loop fallback (tests)
     // persistent cooperative RK4 engine (true stages, uniform spacing)
     bool engine_ok = false;
+    // small mixed domains: all steps of an update in one thread-block cluster
+    bool clu_ok = false;
+    int clu_mode = 0, clu_nc = 0, clu_threads = 0;
+    size_t clu_smem = 0;
     int eng_grid = 0, eng_CB = 1, eng_RA = 2, eng_P2 = 0;
     size_t eng_smem = 0;
     float *xhi = nullptr, *xlo = nullptr, *wrefhi = nullptr, *wreflo = nullptr;
@@ -1064,6 +1069,47 @@ template <typename T> T* enqueue_engine(fi_handle* h, int nsteps)
     return (T*)h->raw[3];
 }
 
+ClusterArgs cluster_args(const fi_handle* h)
+{
+    ClusterArgs a;
+    memset(&a, 0, sizeof(a));
+    a.p = h->prhs;
+    a.fcf = flex_coef_f32(h->fc);
+    a.x = h->d.x;
+    a.w = h->d.w;
+    a.wrhi = h->wrefhi;
+    a.wrlo = h->wreflo;
+    a.q0 = (const float*)h->q0;
+    a.D = (const float*)h->Dt;
+    a.inv2eta = (const float*)h->inv2eta;
+    a.mAT = (const float*)h->mAT;
+    a.mBT = (const float*)h->mBT;
+    a.even = h->even;
+    a.mask = h->d.mactive;
+    for (int i = 0; i < 7; ++i) a.raw[i] = (float*)h->raw[i];
+    a.ctl = h->ctl;
+    a.spy = h->spy;
+    a.atol = h->p.atol;
+    a.rtol = h->p.rtol;
+    a.q = h->p.q;
+    a.dt_max = h->p.dt_max;
+    a.norm_scale_f = (float)(1.0 / (double)(float)((long long)h->nx * h->ny));
+    cluster_split(a, h->clu_nc);
+    return a;
+}
+
+// All RK4 steps of one update in one cluster (fi_cluster.cu).
+float* enqueue_cluster(fi_handle* h, int nsteps)
+{
+    ClusterArgs a = cluster_args(h);
+    a.nsteps = nsteps;
+    cudaError_t le = cudaSuccess;
+    PROF(h, K_ENGINE, le = cluster_launch(a, nullptr, 1, h->clu_mode, h->clu_nc, h->clu_threads, 0, h->clu_smem, h->s));
+    if (le != cudaSuccess && h->launch_err == cudaSuccess) h->launch_err = le;
+    h->launches += 1;
+    return (float*)h->raw[3];
+}
+
 const int kMaxAttempts = 10000000;
 const long long kDefaultMaxReject = 1000000;   // rejections per update (fi_set_max_rejections)
 
@@ -1289,7 +1335,9 @@ template <typename T> int update_T(fi_handle* h, const double* dH, double time, 
             enqueue_post<T>(h, raw_last, have_rhs);
             return FI_OK;
         }
-        T* raw_last = (h->engine_ok && nsteps > 0) ? enqueue_engine<T>(h, nsteps) : enqueue_steps<T>(h, nsteps);
+        T* raw_last = (h->clu_ok && nsteps > 0)      ? (T*)enqueue_cluster(h, nsteps)
+                      : (h->engine_ok && nsteps > 0) ? enqueue_engine<T>(h, nsteps)
+                                                     : enqueue_steps<T>(h, nsteps);
         enqueue_post<T>(h, raw_last, nsteps > 0 ? 1 : 0);
         return FI_OK;
     };
@@ -1702,7 +1750,19 @@ int fi_create(const fi_params* pin, int nx_ice, int ny_ice, double dx, double dy
         const bool tsit_true = p.method == 3 && p.stage_mode == 1 && p.dt_method == 2 && h->uniform;
         const bool want = rk4_true && !(ev && ev[0] == '1');
 #define AL2(ptr, bytes) if ((rc = dalloc(h, &(ptr), (bytes)))) return rc
-        if (want) {
+        const size_t nk = (size_t)(h->prhs.h + 1) * h->ny;
+        auto is_set = [](const char* name) {
+            const char* e = getenv(name);
+            return e && e[0] && e[0] != '0';
+        };
+        if (want && mixed(h) && !is_set("FI_NO_CLUSTER") && !is_set("FI_ENGINE_RA") &&
+            !is_set("FI_ENGINE_BARRIER_PHANTOM")) {
+            h->clu_mode = CLU_RK4;
+            h->clu_ok = cluster_config(h->prhs, h->clu_mode, &h->clu_nc, &h->clu_threads, &h->clu_smem) != 0;
+            cudaGetLastError();
+            if (h->clu_ok) { AL2(h->mAT, nk * tsz(h)); AL2(h->mBT, nk * tsz(h)); }
+        }
+        if (want && !h->clu_ok) {
             int ok = mixed(h) ? engine_config<float>(h->prhs, &h->eng_grid, &h->eng_CB, &h->eng_smem, &h->eng_RA,
                                                   &h->eng_P2)
                               : engine_config<double>(h->prhs, &h->eng_grid, &h->eng_CB, &h->eng_smem, &h->eng_RA,
@@ -1710,7 +1770,6 @@ int fi_create(const fi_params* pin, int nx_ice, int ny_ice, double dx, double dy
             h->engine_ok = ok != 0;
             cudaGetLastError();
             if (h->engine_ok) {
-                const size_t nk = (size_t)(h->prhs.h + 1) * h->ny;
                 AL2(h->ST, nk * c2); AL2(h->mAT, nk * tsz(h)); AL2(h->mBT, nk * tsz(h));
                 AL2(h->eng_bar, sizeof(unsigned));
             }
@@ -1718,7 +1777,7 @@ int fi_create(const fi_params* pin, int nx_ice, int ny_ice, double dx, double dy
         if ((rk4_true || tsit_true) && mixed(h)) {
             // the float pairs of x and w_ref (the stage states of every path)
             AL2(h->xhi, n * 4); AL2(h->xlo, n * 4); AL2(h->wrefhi, n * 4); AL2(h->wreflo, n * 4);
-            if (!h->engine_ok) AL2(h->dxw, n * 4);
+            if (!h->engine_ok && !h->clu_ok) AL2(h->dxw, n * 4);
         }
         if (tsit_true && mixed(h)) { AL2(h->yhi, n * 4); AL2(h->ylo, n * 4); AL2(h->ydw, n * 4); }
 #undef AL2
@@ -1729,7 +1788,7 @@ int fi_create(const fi_params* pin, int nx_ice, int ny_ice, double dx, double dy
         if (mixed(h)) tune_conv_shapes<float>(h);
         else tune_conv_shapes<double>(h);
     }
-    if (p.method == 3 && !h->engine_ok && !(getenv("FI_NO_TUNE") && getenv("FI_NO_TUNE")[0] == '1')) {
+    if (p.method == 3 && !h->engine_ok && !h->clu_ok && !(getenv("FI_NO_TUNE") && getenv("FI_NO_TUNE")[0] == '1')) {
         if (mixed(h)) tune_rhs_shapes<float>(h);
         else tune_rhs_shapes<double>(h);
         CK(cudaGetLastError());
@@ -2022,7 +2081,7 @@ int fi_metrics_json(fi_handle* h, char* buf, size_t len)
                            "\"n_attempt\": %lld, \"kernels_enqueued\": %lld, \"graphs_captured\": %d, "
                            "\"host_update_ms\": %.6f, \"status\": %d}",
                            h->nx, h->ny, h->nx_ice, h->ny_ice, mixed(h) ? "mixed" : "fp64", p.method, p.dt_method,
-                           p.stage_mode, h->engine_ok ? "true" : "false", h->updates, hc.t, hc.dt, hc.n_accept,
+                           p.stage_mode, h->engine_ok || h->clu_ok ? "true" : "false", h->updates, hc.t, hc.dt, hc.n_accept,
                            hc.n_reject, hc.n_attempt, h->launches, (int)h->graphs.size(), 1e3 * h->host_update_s,
                            hc.status);
     return (n < 0 || (size_t)n >= len) ? FI_E_SIZE : FI_OK;

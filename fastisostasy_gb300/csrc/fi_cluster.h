@@ -1,0 +1,47 @@
+// fi_cluster.h — small mixed domains advanced by one thread-block cluster each
+// (fi_cluster.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "fi_common.cuh"
+#include "fi_kernels.h"
+
+namespace fi {
+
+enum { CLU_RK4 = 0, CLU_TSIT = 1, CLU_TSIT_TRUE = 2 };
+
+struct ClusterArgs {
+    Plan2D p;
+    FlexCoefF fcf;
+    double* x;                       // integrator state
+    double* w;                       // now%w
+    const float* wrhi;               // w_ref as a float pair (true stages)
+    const float* wrlo;
+    const float* q0;                 // load term
+    const float* D;
+    const float* inv2eta;
+    const float* mAT;                // 1/(kappa R) factors, column-major (k*ny + l)
+    const float* mBT;
+    int even;
+    const uint8_t* mask;
+    float* raw[7];                   // stage outputs; the last one evaluated is left in raw[0] (raw[3] in RK4)
+    Ctl* ctl;
+    int nsteps;                      // RK4: steps of this update
+    int rpc, cpc;                    // rows and spectrum columns per block
+    double spy, atol, rtol, q, dt_max;
+    int max_iter;
+    float norm_scale_f;
+};
+
+// Blocks per cluster, threads and shared memory for a domain of this plan;
+// 0 where it does not fit (then the other paths take it).
+int cluster_config(const Plan2D& p, int mode, int* nc, int* threads, size_t* smem);
+void cluster_split(ClusterArgs& a, int nc);
+// one domain, or (many != null, in device memory) n domains in one launch, none
+// of which has a thread own more than run_most rows
+cudaError_t cluster_launch(const ClusterArgs& a, const ClusterArgs* many, int n, int mode, int nc, int threads,
+                           int run_most, size_t smem, cudaStream_t s);
+
+}  // namespace fi
