@@ -27,7 +27,10 @@ def _nvcc():
 
 
 def sources():
-    return sorted(glob.glob(os.path.join(CSRC, "*.cu")))
+    """Translation units, the longest to compile first."""
+    slow = ("fi_cluster_", "fi_rhs", "fi_lines")
+    return sorted(glob.glob(os.path.join(CSRC, "*.cu")),
+                  key=lambda p: (not os.path.basename(p).startswith(slow), p))
 
 
 def deps():
@@ -59,7 +62,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             print(r.stderr)
         return obj
 
-    with cf.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 2)) as ex:
+    with cf.ThreadPoolExecutor(max_workers=min(16, os.cpu_count() or 2)) as ex:
         objs = list(ex.map(one, sources()))
     tmp = LIB + ".tmp%d" % os.getpid()
     cmd = [nvcc] + ARCH + ["-shared", "-o", tmp] + objs + ["-lcudart"]

@@ -246,7 +246,7 @@ struct fi_handle {
     bool engine_ok = false;
     // small mixed domains: all steps of an update in one thread-block cluster
     bool clu_ok = false;
-    int clu_mode = 0, clu_nc = 0, clu_threads = 0;
+    int clu_mode = 0, clu_nc = 0, clu_threads = 0, clu_stages = 0;
     size_t clu_smem = 0;
     int eng_grid = 0, eng_CB = 1, eng_RA = 2, eng_P2 = 0;
     size_t eng_smem = 0;
@@ -1069,6 +1069,8 @@ template <typename T> T* enqueue_engine(fi_handle* h, int nsteps)
     return (T*)h->raw[3];
 }
 
+const int kMaxAttempts = 10000000;
+
 ClusterArgs cluster_args(const fi_handle* h)
 {
     ClusterArgs a;
@@ -1094,23 +1096,25 @@ ClusterArgs cluster_args(const fi_handle* h)
     a.q = h->p.q;
     a.dt_max = h->p.dt_max;
     a.norm_scale_f = (float)(1.0 / (double)(float)((long long)h->nx * h->ny));
+    a.stages = h->clu_stages;
+    a.max_iter = kMaxAttempts;
     cluster_split(a, h->clu_nc);
     return a;
 }
 
-// All RK4 steps of one update in one cluster (fi_cluster.cu).
+// All steps (RK4) or attempts (tsit54) of one update in one cluster
+// (fi_cluster.cu); returns the buffer of the last RHS.
 float* enqueue_cluster(fi_handle* h, int nsteps)
 {
     ClusterArgs a = cluster_args(h);
     a.nsteps = nsteps;
     cudaError_t le = cudaSuccess;
-    PROF(h, K_ENGINE, le = cluster_launch(a, nullptr, 1, h->clu_mode, h->clu_nc, h->clu_threads, 0, h->clu_smem, h->s));
+    PROF(h, K_ENGINE, le = cluster_launch(a, h->clu_mode, h->clu_nc, h->clu_threads, h->clu_smem, h->s));
     if (le != cudaSuccess && h->launch_err == cudaSuccess) h->launch_err = le;
     h->launches += 1;
-    return (float*)h->raw[3];
+    return (float*)h->raw[h->clu_mode == CLU_RK4 ? 3 : 0];
 }
 
-const int kMaxAttempts = 10000000;
 const long long kDefaultMaxReject = 1000000;   // rejections per update (fi_set_max_rejections)
 
 // One attempt of Tsitouras 5(4) with true stages (the Dormand-Prince 5(4)
@@ -1327,6 +1331,10 @@ template <typename T> int update_T(fi_handle* h, const double* dH, double time, 
     // eager: Tsit5 attempts are decided on the host (one wait per attempt)
     auto enqueue = [&]() -> int {
         enqueue_pre<T>(h, dH, diag, run_integrator);
+        if (tsit && h->clu_ok) {
+            enqueue_post<T>(h, (T*)enqueue_cluster(h, 0), -1);
+            return FI_OK;
+        }
         if (tsit) {
             int have_rhs = 0;
             T* raw_last = nullptr;
@@ -1343,7 +1351,7 @@ template <typename T> int update_T(fi_handle* h, const double* dH, double time, 
     };
     // captured: Tsit5 attempts loop on the device (graph WHILE node)
     auto enqueue_captured = [&]() -> int {
-        if (!tsit) return enqueue();
+        if (!tsit || h->clu_ok) return enqueue();
         enqueue_pre<T>(h, dH, diag, true);
         const int rc = enqueue_tsit_loop<T>(h);
         if (rc) return rc;
@@ -1755,10 +1763,12 @@ int fi_create(const fi_params* pin, int nx_ice, int ny_ice, double dx, double dy
             const char* e = getenv(name);
             return e && e[0] && e[0] != '0';
         };
-        if (want && mixed(h) && !is_set("FI_NO_CLUSTER") && !is_set("FI_ENGINE_RA") &&
+        const bool tsit_any = p.method == 3 && p.dt_method == 2 && h->uniform && !is_set("FI_NO_ENGINE");
+        if ((want || tsit_any) && mixed(h) && !is_set("FI_NO_CLUSTER") && !is_set("FI_ENGINE_RA") &&
             !is_set("FI_ENGINE_BARRIER_PHANTOM")) {
-            h->clu_mode = CLU_RK4;
-            h->clu_ok = cluster_config(h->prhs, h->clu_mode, &h->clu_nc, &h->clu_threads, &h->clu_smem) != 0;
+            h->clu_mode = p.dt_method == 1 ? CLU_RK4 : p.stage_mode == 1 ? CLU_TSIT_TRUE : CLU_TSIT;
+            h->clu_ok = cluster_config(h->prhs, h->clu_mode, &h->clu_nc, &h->clu_threads, &h->clu_stages,
+                                       &h->clu_smem) != 0;
             cudaGetLastError();
             if (h->clu_ok) { AL2(h->mAT, nk * tsz(h)); AL2(h->mBT, nk * tsz(h)); }
         }
@@ -2449,6 +2459,10 @@ struct fi_batch {
     std::vector<fi_handle*> hs;
     bool mixed = false;
     int nm = 0;
+    // members advanced in the batched attempt loop; the others (small mixed
+    // domains) make their whole update in a cluster of their own beside it
+    std::vector<int> loop;
+    int nl() const { return (int)loop.size(); }
     cudaStream_t s = nullptr, s_body = nullptr;
     cudaEvent_t ev_fork = nullptr;
     std::vector<cudaEvent_t> ev;
@@ -2480,7 +2494,8 @@ struct fi_batch {
 // RB / CB <= 0: the single-domain shapes.
 int batch_shape(fi_batch* b, int RB, int CB, int fseg, int waves)
 {
-    const int n = b->nm;
+    const int n = b->nl();
+    if (n == 0) return 0;
     std::vector<int> off(4 * (n + 1), 0);
     const size_t c2 = b->mixed ? sizeof(float2) : sizeof(double2);
     b->rows_threads = b->cols_threads = 0;
@@ -2563,7 +2578,7 @@ namespace {
 // One Tsit5 attempt of every member that still has one, as batched launches.
 template <typename T> void batch_attempt(fi_batch* b, cudaStream_t s, cudaGraphConditionalHandle loop, int* more_out)
 {
-    const int nm = b->nm;
+    const int nm = b->nl();
     const int* off = b->doff;
     batch_attempt_begin(b->dM, nm, kMaxAttempts, off, b->dcl, s);
     const BList LF = blist(b->dcl, nm, 0), LR = blist(b->dcl, nm, 1), LC = blist(b->dcl, nm, 2),
@@ -2610,38 +2625,69 @@ template <typename T> void batch_attempt(fi_batch* b, cudaStream_t s, cudaGraphC
     batch_attempt_end(b->dM, nm, loop, s, more_out);
 }
 
+// The members' branches up to the attempt loop: the update head of a loop
+// member (the batch stream waits for it), the whole update of a member with a
+// cluster of its own (the batch stream waits in batch_join).
+template <typename T> int batch_fork(fi_batch* b, bool diag)
+{
+    if (cudaEventRecord(b->ev_fork, b->s) != cudaSuccess) return FI_E_CUDA;
+    for (int i = 0; i < b->nm; ++i) {
+        fi_handle* h = b->hs[i];
+        if (cudaStreamWaitEvent(h->s, b->ev_fork, 0) != cudaSuccess) return FI_E_CUDA;
+        enqueue_pre<T>(h, h->dH, diag, true);
+        if (h->clu_ok) {
+            enqueue_post<T>(h, (T*)enqueue_cluster(h, 0), -1);
+            if (h->launch_err != cudaSuccess) {
+                h->launch_err = cudaSuccess;
+                return FI_E_CUDA;
+            }
+        } else {
+            if (h->d.whi) split_hilo(h->d.w, h->d.whi, h->d.wlo, h->n, h->s);
+            if (h->yhi) split_hilo_dxw(h->d.x, h->xhi, h->xlo, h->wrefhi, h->wreflo, h->dxw, h->n, h->s);
+        }
+        if (cudaEventRecord(b->ev[i], h->s) != cudaSuccess) return FI_E_CUDA;
+    }
+    for (int i : b->loop)
+        if (cudaStreamWaitEvent(b->s, b->ev[i], 0) != cudaSuccess) return FI_E_CUDA;
+    return FI_OK;
+}
+
+// The update tails of the loop members, then all members joined.
+template <typename T> int batch_join(fi_batch* b)
+{
+    for (int i = 0; i < b->nm; ++i)
+        if (b->hs[i]->clu_ok && cudaStreamWaitEvent(b->s, b->ev[i], 0) != cudaSuccess) return FI_E_CUDA;
+    if (b->nl() == 0) return FI_OK;
+    if (cudaEventRecord(b->ev_fork, b->s) != cudaSuccess) return FI_E_CUDA;
+    for (int i : b->loop) {
+        fi_handle* h = b->hs[i];
+        if (cudaStreamWaitEvent(h->s, b->ev_fork, 0) != cudaSuccess) return FI_E_CUDA;
+        enqueue_post<T>(h, (T*)h->raw[0], -1);
+        if (cudaEventRecord(b->ev[i], h->s) != cudaSuccess || cudaStreamWaitEvent(b->s, b->ev[i], 0) != cudaSuccess)
+            return FI_E_CUDA;
+    }
+    return FI_OK;
+}
+
 // The same update without a graph: the host reads the loop condition after
 // every attempt (profiling; FI_BATCH_EAGER=1).
 template <typename T> int batch_eager(fi_batch* b, bool diag)
 {
-    auto fork_join = [&](auto&& body) -> int {
-        if (cudaEventRecord(b->ev_fork, b->s) != cudaSuccess) return FI_E_CUDA;
-        for (int i = 0; i < b->nm; ++i) {
-            fi_handle* h = b->hs[i];
-            if (cudaStreamWaitEvent(h->s, b->ev_fork, 0) != cudaSuccess) return FI_E_CUDA;
-            body(h);
-            if (cudaEventRecord(b->ev[i], h->s) != cudaSuccess) return FI_E_CUDA;
-            if (cudaStreamWaitEvent(b->s, b->ev[i], 0) != cudaSuccess) return FI_E_CUDA;
-        }
-        return FI_OK;
-    };
-    int rc = fork_join([&](fi_handle* h) {
-        enqueue_pre<T>(h, h->dH, diag, true);
-        if (h->d.whi) split_hilo(h->d.w, h->d.whi, h->d.wlo, h->n, h->s);
-        if (h->yhi) split_hilo_dxw(h->d.x, h->xhi, h->xlo, h->wrefhi, h->wreflo, h->dxw, h->n, h->s);
-    });
+    int rc = batch_fork<T>(b, diag);
     if (rc) return rc;
-    batch_loop_begin(b->dM, b->nm, b->s);
-    for (long long it = 0;; ++it) {
-        batch_attempt<T>(b, b->s, 0, b->dmore);
-        int more = 0;
-        if (cudaMemcpyAsync(&more, b->dmore, sizeof(int), cudaMemcpyDeviceToHost, b->s) != cudaSuccess ||
-            cudaStreamSynchronize(b->s) != cudaSuccess)
-            return FI_E_CUDA;
-        if (!more) break;
-        if (it > kMaxAttempts) return FI_E_STEP;
+    if (b->nl() > 0) {
+        batch_loop_begin(b->dM, b->nl(), b->s);
+        for (long long it = 0;; ++it) {
+            batch_attempt<T>(b, b->s, 0, b->dmore);
+            int more = 0;
+            if (cudaMemcpyAsync(&more, b->dmore, sizeof(int), cudaMemcpyDeviceToHost, b->s) != cudaSuccess ||
+                cudaStreamSynchronize(b->s) != cudaSuccess)
+                return FI_E_CUDA;
+            if (!more) break;
+            if (it > kMaxAttempts) return FI_E_STEP;
+        }
     }
-    return fork_join([&](fi_handle* h) { enqueue_post<T>(h, (T*)h->raw[0], -1); });
+    return batch_join<T>(b);
 }
 
 template <typename T> int batch_capture(fi_batch* b, bool diag, cudaGraph_t* out)
@@ -2651,24 +2697,9 @@ template <typename T> int batch_capture(fi_batch* b, bool diag, cudaGraph_t* out
     auto ck = [&](cudaError_t e) { return e == cudaSuccess ? FI_OK : FI_E_CUDA; };
     int rc;
     if ((rc = ck(cudaStreamBeginCapture(b->s, cudaStreamCaptureModeThreadLocal)))) return rc;
-    auto join_members = [&](auto&& body) -> int {
-        if (cudaEventRecord(b->ev_fork, b->s) != cudaSuccess) return FI_E_CUDA;
-        for (int i = 0; i < b->nm; ++i) {
-            fi_handle* h = b->hs[i];
-            if (cudaStreamWaitEvent(h->s, b->ev_fork, 0) != cudaSuccess) return FI_E_CUDA;
-            body(h);
-            if (cudaEventRecord(b->ev[i], h->s) != cudaSuccess) return FI_E_CUDA;
-            if (cudaStreamWaitEvent(b->s, b->ev[i], 0) != cudaSuccess) return FI_E_CUDA;
-        }
-        return FI_OK;
-    };
-    rc = join_members([&](fi_handle* h) {
-        enqueue_pre<T>(h, h->dH, diag, true);
-        if (h->d.whi) split_hilo(h->d.w, h->d.whi, h->d.wlo, h->n, h->s);
-        if (h->yhi) split_hilo_dxw(h->d.x, h->xhi, h->xlo, h->wrefhi, h->wreflo, h->dxw, h->n, h->s);
-    });
-    if (!rc) {
-        batch_loop_begin(b->dM, b->nm, b->s);
+    rc = batch_fork<T>(b, diag);
+    if (!rc && b->nl() > 0) {
+        batch_loop_begin(b->dM, b->nl(), b->s);
         cudaStreamCaptureStatus st;
         cudaGraph_t g = nullptr;
         const cudaGraphNode_t* deps = nullptr;
@@ -2696,7 +2727,7 @@ template <typename T> int batch_capture(fi_batch* b, bool diag, cudaGraph_t* out
             }
         }
     }
-    if (!rc) rc = join_members([&](fi_handle* h) { enqueue_post<T>(h, (T*)h->raw[0], -1); });
+    if (!rc) rc = batch_join<T>(b);
     cudaGraph_t graph = nullptr;
     const cudaError_t e = cudaStreamEndCapture(b->s, &graph);
     if (rc || e != cudaSuccess) {
@@ -2754,10 +2785,12 @@ int fi_batch_create(fi_handle* const* hs, int n, fi_batch** out)
     b->nm = n;
     b->mixed = mixed(hs[0]);
     b->true_stages = hs[0]->p.stage_mode == 1;
-    std::vector<BMember> M(n);
-    for (int i = 0; i < n; ++i) {
-        fi_handle* h = hs[i];
-        BMember& m = M[i];
+    for (int i = 0; i < n; ++i)
+        if (!hs[i]->clu_ok) b->loop.push_back(i);
+    std::vector<BMember> M(b->nl());
+    for (int k = 0; k < b->nl(); ++k) {
+        fi_handle* h = hs[b->loop[k]];
+        BMember& m = M[k];
         memset(&m, 0, sizeof(m));
         m.p = h->prhs;
         m.fc = h->fc;
@@ -2830,7 +2863,7 @@ namespace {
 // Lists of all members (every list kind) for timing the batched passes.
 int batch_all_lists(fi_batch* b)
 {
-    const int n = b->nm;
+    const int n = b->nl();
     std::vector<int> cl(blist_ints(n), 0);
     cl[0] = cl[1] = n;
     for (int i = 0; i < n; ++i) cl[2 + i] = cl[2 + n + i] = i;
@@ -2849,7 +2882,7 @@ int batch_all_lists(fi_batch* b)
 // `reps` after one warm-up.
 template <typename T> float batch_time_rhs(fi_batch* b, int part, int reps)
 {
-    const int nm = b->nm;
+    const int nm = b->nl();
     const BList LF = blist(b->dcl, nm, 0), LR = blist(b->dcl, nm, 1), LC = blist(b->dcl, nm, 2);
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
@@ -2883,6 +2916,11 @@ int fi_batch_autotune(fi_batch* b, int32_t* chosen4)
     if (b->seen[0] || b->seen[1]) return FI_E_STATE;
     for (fi_handle* h : b->hs)
         if (cudaStreamSynchronize(h->s) != cudaSuccess) return FI_E_CUDA;
+    if (b->nl() == 0) {   // nothing runs in the batched loop
+        if (chosen4)
+            for (int k = 0; k < 4; ++k) chosen4[k] = b->shape[k];
+        return FI_OK;
+    }
     // the stencil of the reference stages reads now%w's float pair
     for (fi_handle* h : b->hs) {
         if (h->d.whi) split_hilo(h->d.w, h->d.whi, h->d.wlo, h->n, b->s);

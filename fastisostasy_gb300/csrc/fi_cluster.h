@@ -31,17 +31,18 @@ struct ClusterArgs {
     int nsteps;                      // RK4: steps of this update
     int rpc, cpc;                    // rows and spectrum columns per block
     double spy, atol, rtol, q, dt_max;
-    int max_iter;
+    int max_iter;                    // adaptive: attempts per update
+    int stages;                      // stage outputs kept in shared memory
     float norm_scale_f;
 };
 
-// Blocks per cluster, threads and shared memory for a domain of this plan;
+// Blocks per cluster, threads, stage outputs kept in shared memory (true-stage
+// tsit54) and its size for a domain of this plan;
 // 0 where it does not fit (then the other paths take it).
-int cluster_config(const Plan2D& p, int mode, int* nc, int* threads, size_t* smem);
+int cluster_config(const Plan2D& p, int mode, int* nc, int* threads, int* stages, size_t* smem);
 void cluster_split(ClusterArgs& a, int nc);
-// one domain, or (many != null, in device memory) n domains in one launch, none
-// of which has a thread own more than run_most rows
-cudaError_t cluster_launch(const ClusterArgs& a, const ClusterArgs* many, int n, int mode, int nc, int threads,
-                           int run_most, size_t smem, cudaStream_t s);
+// probe: no launch, only whether such a cluster can be resident
+cudaError_t cluster_launch(const ClusterArgs& a, int mode, int nc, int threads, size_t smem, cudaStream_t s,
+                           bool probe = false);
 
 }  // namespace fi

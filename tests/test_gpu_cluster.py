@@ -59,3 +59,33 @@ def test_cluster_against_the_kernel_sequence(monkeypatch):
         assert pair.dom.scalars()["n_accept"] == 12
         pair.close()
     assert rel(res[1], res[0]) <= 1e-5
+
+
+@pytest.mark.parametrize("nx,ny", [(16, 16), (34, 34), (64, 64), (96, 96), (64, 20), (32, 256), (128, 192), (192, 192),
+                                   (256, 256)])
+@pytest.mark.parametrize("stage_mode", [0, 1])
+def test_tsit54_in_a_cluster(nx, ny, stage_mode):
+    """Same attempts as the oracle, rejections among them, within the bound."""
+    wl = workload(nx, ny, nx + 5 * ny, nx != 64, dt_method=2, stage_mode=stage_mode, dt_init=8.0, dt_max=8.0)
+    pair = Pair(wl, precision=1)
+    assert pair.dom.metrics()["step_engine"]
+    pair.init()
+    pair.step(3)
+    a, b = pair.dom.scalars(), pair.orc.scalars()
+    assert a["t"] == pair.t and a["n_accept"] == b["n_accept"] and a["n_reject"] == b["n_reject"]
+    for f in ("w", "z_bed"):
+        assert rel(pair.dom.field(f), pair.orc.field(f)) <= 1e-5
+    pair.close()
+
+
+def test_rejection_limit_in_a_cluster():
+    """The step floor ends the update in every block alike: FI_E_STEP, and the domain answers on."""
+    from fastisostasy_gb300 import _lib
+    wl = workload(64, 64, 9, True, dt_method=2, stage_mode=0, dt_init=8.0, dt_max=8.0, dt_min=4.0, atol=1e-9, rtol=0.0)
+    pair = Pair(wl, precision=1)
+    pair.init()
+    with pytest.raises(_lib.FiError) as e:
+        pair.dom.update(wl.H_at(10.0), 10.0, pair.bg)
+    assert e.value.code == _lib.FI_E_STEP
+    assert pair.dom.scalars()["n_reject"] >= 1
+    pair.close()
