@@ -915,6 +915,22 @@ void rhs_pair_stage(fi_handle* h, const float* rprev, double a, float* raw_out)
     h->launches += 4;
 }
 
+// One RK4 stage RHS of the plain form (rprev: the previous stage's raw RHS,
+// null at the first stage; a: its tableau weight).
+void rhs_stage64(fi_handle* h, const double* rprev, double a, double* raw_out)
+{
+    PROF(h, K_FLEX, launch_flexure_stage64(h->d.x, rprev, h->w_ref, (const double*)h->q0, h->d.mactive,
+                                           (const double*)h->Dt, (const double*)h->inv2eta, (double*)h->f, h->nx,
+                                           h->ny, h->fc, h->ctl, a, h->rate_scale, h->s));
+    PROF(h, K_ROWS_FWD,
+         launch_rows_fwd<double>((const double*)h->f, h->nx, h->nx, h->ny, (double2*)h->S, h->prhs, h->s));
+    PROF(h, K_COLS_HARTLEY, launch_cols_hartley<double>((double2*)h->S, (const double*)h->mA, (const double*)h->mB,
+                                                        h->even, h->prhs, h->s));
+    const double norm = (double)(float)((long long)h->nx * h->ny);   // nx*ny*1. (default real)
+    PROF(h, K_ROWS_INV, launch_rows_inv<double>((const double2*)h->S, raw_out, h->prhs, 1.0 / norm, h->s));
+    h->launches += 4;
+}
+
 // One RHS of the mixed true-stage Tsit5 at a stage state given as a float
 // pair with its dxw (rhs with the column-strip stencil in stage mode).
 void rhs_tpair(fi_handle* h, const float* hi, const float* lo, const float* dw, float* raw_out, const int* gate)
@@ -988,6 +1004,14 @@ template <typename T> T* enqueue_steps(fi_handle* h, int nsteps)
             PROF(h, K_RK_FINAL, rk4_final_pair(h->ctl, h->d.x, h->d.w, h->xhi, h->xlo, h->wrefhi, h->wreflo, h->dxw,
                                                (const float*)r0, (const float*)r1, (const float*)r2,
                                                (const float*)r3, h->nx, h->ny, spy, h->s));
+            h->launches += 1;
+            last = r3;
+        } else if (p.dt_method == 1 && truem && sizeof(T) == 8 && h->uniform && p.method == 3) {
+            // plain form: the stage state is formed inside the stencil
+            T* const r[4] = {r0, r1, r2, r3};
+            const double aw[4] = {0.0, 0.5, 0.5, 1.0};
+            for (int q = 0; q < 4; ++q) rhs_stage64(h, q ? (const double*)r[q - 1] : nullptr, aw[q], (double*)r[q]);
+            PROF(h, K_RK_FINAL, rk4_final<T>(h->ctl, h->d.x, h->d.w, r0, r1, r2, r3, h->nx, h->ny, spy, h->s));
             h->launches += 1;
             last = r3;
         } else if (p.dt_method == 1 && truem) {
@@ -2526,8 +2550,10 @@ int batch_shape(fi_batch* b, int RB, int CB, int fseg, int waves)
         if (m.lines & 1) m.RB = b->rows_threads / rhs_line_threads(m.p.h, b->mixed);
         if (m.lines & 2) m.CB = b->cols_threads / rhs_line_threads(m.p.ny, b->mixed);
         m.fseg = fseg;
-        const int fblk = (b->mixed && (!b->true_stages || m.yhi)) ? batch_flexure_blocks(m.p.nx, m.p.ny, m.fseg)
-                                                                  : m.fgx * ((m.p.ny + 7) / 8);
+        const int fblk = b->mixed ? (!b->true_stages || m.yhi ? batch_flexure_blocks(m.p.nx, m.p.ny, m.fseg)
+                                                              : m.fgx * ((m.p.ny + 7) / 8))
+                         : m.fc.dxm == nullptr ? batch_flexure_tiles64(m.p.nx, m.p.ny)
+                                               : m.fgx * ((m.p.ny + 7) / 8);
         const int rblk = (m.p.ny + m.RB - 1) / m.RB;
         const int cblk = (m.p.h + 1 + m.CB - 1) / m.CB;
         off[i + 1] = off[i] + fblk;
@@ -2795,6 +2821,7 @@ int fi_batch_create(fi_handle* const* hs, int n, fi_batch** out)
         m.p = h->prhs;
         m.fc = h->fc;
         m.fcf = flex_coef_f32(h->fc);
+        if (!h->fc.dxm) m.fc64 = flex_coef_f64(h->fc);
         m.norm_scale = 1.0 / (double)(float)((long long)h->prhs.nx * h->prhs.ny);   // nx*ny*1. (default real)
         m.norm_scale_f = (float)m.norm_scale;
         m.y = h->d.w;

@@ -21,6 +21,7 @@ struct BMember {
     Plan2D p;                 // RHS transform plan
     FlexCoef fc;              // flexure coefficients
     FlexCoefF fcf;            // the same in float (mixed form)
+    FlexCoef64 fc64;          // factors of the FP64 tiles on uniform spacing
     const double* y;          // the RHS is evaluated at now%w
     const void* q0;           // load term (T)
     const uint8_t* mask;
@@ -42,7 +43,7 @@ struct BMember {
     int even;
     int RB, CB;               // rows per row block, columns per column block
     int lines;                // transforms on register lines: bit 0 rows, bit 1 columns
-    int fgx;                  // flexure blocks along x (FP64 tiles)
+    int fgx;                  // flexure blocks along x (tiles)
     int fseg;                 // output rows per flexure warp task (mixed column strips)
     int red_nblk;             // blocks of the reduction kernels
     double norm_scale;        // 1 / (nx*ny*1.) as the reference normalises
@@ -82,6 +83,8 @@ inline BList blist(const int* base, int nm, int kind)
 
 // Virtual blocks of the mixed batched flexure (8 column-strip warp tasks each).
 int batch_flexure_blocks(int nx, int ny, int seg);
+// ... and of the FP64 one on uniform spacing (32 x 16 tiles).
+int batch_flexure_tiles64(int nx, int ny);
 
 // Block shapes of the single-domain launches (shared with the batched ones).
 int rhs_rows_per_block(int h);

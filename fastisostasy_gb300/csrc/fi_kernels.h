@@ -37,6 +37,27 @@ inline FlexCoefF flex_coef_f32(const FlexCoef& c)
     return f;
 }
 
+// The FP64 stencil on uniform spacing works on unscaled differences: the
+// spacings enter through these.
+struct FlexCoef64 {
+    double rxy, ryx;               // nu inv_dy2 / inv_dx2 and its counterpart
+    double cxx, cyy, cxy;          // factors of the unscaled second differences of the moments in f
+    double cm;                     // coef_mantle
+};
+
+inline FlexCoef64 flex_coef_f64(const FlexCoef& c)
+{
+    FlexCoef64 f;
+    f.rxy = c.nu * (c.inv_dy2 / c.inv_dx2);
+    f.ryx = c.nu * (c.inv_dx2 / c.inv_dy2);
+    f.cxx = -(c.inv_dx2 * c.inv_dx2);
+    f.cyy = -(c.inv_dy2 * c.inv_dy2);
+    const double d = c.inv_2dx * c.inv_2dy;
+    f.cxy = -2.0 * c.one_minus_nu * (d * d);
+    f.cm = c.coef_mantle;
+    return f;
+}
+
 // One FFT length: factorisation + twiddle tables in both precisions.
 struct FftLen {
     FftDesc d;
@@ -73,6 +94,12 @@ void launch_flexure_stage(const float* whi, const float* wlo, const float* rprev
                           const uint8_t* mask, const float* D, const float* inv2eta, float* f, int nx, int ny,
                           const FlexCoef& c, const Ctl* ctl, double a, double spy, cudaStream_t s,
                           const int* gate = nullptr);
+
+// Plain form, uniform spacing: the RHS at the RK4 stage state
+// x + (a h spy) (rprev - corner mean), formed on the fly (rprev null: at x).
+void launch_flexure_stage64(const double* x, const double* rprev, const double* wref, const double* q0,
+                            const uint8_t* mask, const double* D, const double* inv2eta, double* f, int nx, int ny,
+                            const FlexCoef& c, const Ctl* ctl, double a, double spy, cudaStream_t s);
 
 template <typename T>
 void launch_rows_fwd(const T* in, int in_pitch, int in_width, int nrows_in, typename vec2<T>::type* S,

@@ -589,6 +589,149 @@ static int strip_seg_single(int nx, int ny)
     return (int)seg;
 }
 
+// ---------------------------------------------------------------------------
+// FP64 flexure of the plain form on uniform spacing.  GB300 issues one FP64
+// warp instruction every 64 clocks per SM quarter, whatever the instruction-
+// level parallelism, so the stencil costs their number.  The tile form with
+// per-cell spacing (k_flexure) executes about 70 per cell: its 32 x 8 tiles
+// take every level on a halo of two, and every difference is scaled where it
+// is taken.  Here the tile is 32 x 16, moments are formed straight from the
+// stage state, all differences are left unscaled (the spacings sit in five
+// factors, FlexCoef64), and the RK4 stage state x + sc raw is one FMA on the
+// way into the tile instead of a kernel and a field of its own: 30 per cell.
+// A walk down column strips as in flexure_strip needs 25 a lane and row but
+// ran slower (512^2 50 us against 31 of the old tiles): at one or two warps a
+// quarter nothing covers its loads, shuffles and addressing (FP64 pipe 39 %).
+// STAGE: y = x + sc rprev; `off` = sc times the corner mean of rprev, which the
+// differences drop and the mantle term takes off.
+// ---------------------------------------------------------------------------
+constexpr int TY64 = 16;                              // 32 x 16 outputs, 32 x 8 threads
+constexpr int YR = TY64 + 4, YC = TX + 4, MR = TY64 + 2, MC = TX + 2;
+
+template <bool STAGE>
+__device__ __forceinline__ void flexure_tile64(const double* __restrict__ x, const double* __restrict__ rprev,
+                                               const double* __restrict__ wref, const double* __restrict__ q0,
+                                               const uint8_t* __restrict__ mask, const double* __restrict__ D,
+                                               const double* __restrict__ inv2eta, double* __restrict__ f, int nx,
+                                               int ny, const FlexCoef64& c, int bx, int by, double sc = 0.0,
+                                               double off = 0.0)
+{
+    __shared__ double ys[YR][YC];
+    __shared__ double Mxx[MR][MC], Myy[MR][MC], Mxy[MR][MC];
+    const int tid = (int)(threadIdx.x + threadIdx.y * blockDim.x);   // 1D or 32 x 8 blocks
+    const int i0 = bx * TX, j0 = by * TY64;
+    // tiles that touch no edge of the grid carry none of the one-sided forms
+    const bool inner = i0 >= 2 && i0 + TX + 2 <= nx && j0 >= 2 && j0 + TY64 + 2 <= ny;
+    for (int e = tid; e < YR * YC; e += TX * TY) {
+        const int ly = e / YC, lx = e - ly * YC;
+        const int gi = i0 - 2 + lx, gj = j0 - 2 + ly;
+        double v = 0.0;
+        if (inner || (gi >= 0 && gi < nx && gj >= 0 && gj < ny)) {
+            const size_t g = (size_t)gj * nx + gi;
+            v = __ldg(x + g);
+            if (STAGE) v += sc * __ldg(rprev + g);
+        }
+        ys[ly][lx] = v;
+    }
+    __syncthreads();
+    if (inner) {
+        for (int e = tid; e < MR * MC; e += TX * TY) {
+            const int my = e / MC, mx = e - my * MC;
+            const int ly = my + 1, lx = mx + 1;
+            const double Dl = __ldg(D + (size_t)(j0 - 1 + my) * nx + (i0 - 1 + mx));
+            const double y = ys[ly][lx];
+            const double wxx = (ys[ly][lx + 1] + ys[ly][lx - 1]) - 2.0 * y;
+            const double wyy = (ys[ly + 1][lx] + ys[ly - 1][lx]) - 2.0 * y;
+            const double wxy = (ys[ly + 1][lx + 1] - ys[ly + 1][lx - 1]) - (ys[ly - 1][lx + 1] - ys[ly - 1][lx - 1]);
+            Mxx[my][mx] = Dl * (wxx + c.rxy * wyy);
+            Myy[my][mx] = Dl * (wyy + c.ryx * wxx);
+            Mxy[my][mx] = Dl * wxy;
+        }
+    } else {
+        for (int e = tid; e < MR * MC; e += TX * TY) {
+            const int my = e / MC, mx = e - my * MC;
+            const int gi = i0 - 1 + mx, gj = j0 - 1 + my;
+            if (gi < 0 || gi >= nx || gj < 0 || gj >= ny) continue;
+            const int ly = my + 1, lx = mx + 1;
+            // the one-sided second differences are the central ones one cell
+            // inside, a one-sided first difference counts twice
+            const int cx = lx + (gi == 0) - (gi == nx - 1), cy = ly + (gj == 0) - (gj == ny - 1);
+            const int xl = lx - (gi > 0), xr = lx + (gi < nx - 1), yl = ly - (gj > 0), yr = ly + (gj < ny - 1);
+            const double tw = (xr - xl == 2 ? 1.0 : 2.0) * (yr - yl == 2 ? 1.0 : 2.0);
+            const double Dl = __ldg(D + (size_t)gj * nx + gi);
+            const double wxx = (ys[ly][cx + 1] + ys[ly][cx - 1]) - 2.0 * ys[ly][cx];
+            const double wyy = (ys[cy + 1][lx] + ys[cy - 1][lx]) - 2.0 * ys[cy][lx];
+            const double wxy = tw * ((ys[yr][xr] - ys[yr][xl]) - (ys[yl][xr] - ys[yl][xl]));
+            Mxx[my][mx] = Dl * (wxx + c.rxy * wyy);
+            Myy[my][mx] = Dl * (wyy + c.ryx * wxx);
+            Mxy[my][mx] = Dl * wxy;
+        }
+    }
+    __syncthreads();
+    for (int e = tid; e < TX * TY64; e += TX * TY) {
+        const int ly = e / TX, lx = e - ly * TX;
+        const int gi = i0 + lx, gj = j0 + ly;
+        if (!inner && (gi >= nx || gj >= ny)) continue;
+        const size_t g = (size_t)gj * nx + gi;
+        double p = __ldg(q0 + g);
+        const uint32_t on = __ldg(mask + g);
+        const double ie = __ldg(inv2eta + g);
+        const int my = ly + 1, mx = lx + 1;
+        double mxx, myy, mxy;
+        if (inner) {
+            mxx = (Mxx[my][mx + 1] + Mxx[my][mx - 1]) - 2.0 * Mxx[my][mx];
+            myy = (Myy[my + 1][mx] + Myy[my - 1][mx]) - 2.0 * Myy[my][mx];
+            mxy = (Mxy[my + 1][mx + 1] - Mxy[my + 1][mx - 1]) - (Mxy[my - 1][mx + 1] - Mxy[my - 1][mx - 1]);
+        } else {
+            const int cx = mx + (gi == 0) - (gi == nx - 1), cy = my + (gj == 0) - (gj == ny - 1);
+            const int xl = mx - (gi > 0), xr = mx + (gi < nx - 1), yl = my - (gj > 0), yr = my + (gj < ny - 1);
+            const double tw = (xr - xl == 2 ? 1.0 : 2.0) * (yr - yl == 2 ? 1.0 : 2.0);
+            mxx = (Mxx[my][cx + 1] + Mxx[my][cx - 1]) - 2.0 * Mxx[my][cx];
+            myy = (Myy[cy + 1][mx] + Myy[cy - 1][mx]) - 2.0 * Myy[cy][mx];
+            mxy = tw * ((Mxy[yr][xr] - Mxy[yr][xl]) - (Mxy[yl][xr] - Mxy[yl][xl]));
+        }
+        if (wref) p += c.cm * ((STAGE ? ys[ly + 2][lx + 2] - off : ys[ly + 2][lx + 2]) - __ldg(wref + g));
+        if (on == 0) p = 0.0;
+        f[g] = (((p + c.cxx * mxx) + c.cxy * mxy) + c.cyy * myy) * ie;
+    }
+}
+
+__global__ void __launch_bounds__(TX* TY)
+k_flexure64(const double* __restrict__ y, const double* __restrict__ wref, const double* __restrict__ q0,
+            const uint8_t* __restrict__ mask, const double* __restrict__ D, const double* __restrict__ inv2eta,
+            double* __restrict__ f, int nx, int ny, FlexCoef64 c, const int* __restrict__ gate)
+{
+    if (gate && *gate == 0) return;
+    flexure_tile64<false>(y, nullptr, wref, q0, mask, D, inv2eta, f, nx, ny, c, blockIdx.x, blockIdx.y);
+}
+
+__global__ void __launch_bounds__(TX* TY)
+k_flexure64_stage(const double* __restrict__ x, const double* __restrict__ rprev, const double* __restrict__ wref,
+                  const double* __restrict__ q0, const uint8_t* __restrict__ mask, const double* __restrict__ D,
+                  const double* __restrict__ inv2eta, double* __restrict__ f, int nx, int ny, FlexCoef64 c,
+                  const Ctl* __restrict__ ctl, double a, double spy)
+{
+    __shared__ double s_sc[2];
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        s_sc[0] = (a * ctl->h) * spy;
+        s_sc[1] = s_sc[0] * corner_mean_of(rprev, nx, ny);
+    }
+    __syncthreads();
+    flexure_tile64<true>(x, rprev, wref, q0, mask, D, inv2eta, f, nx, ny, c, blockIdx.x, blockIdx.y, s_sc[0], s_sc[1]);
+}
+
+void launch_flexure_stage64(const double* x, const double* rprev, const double* wref, const double* q0,
+                            const uint8_t* mask, const double* D, const double* inv2eta, double* f, int nx, int ny,
+                            const FlexCoef& c, const Ctl* ctl, double a, double spy, cudaStream_t s)
+{
+    const FlexCoef64 cf = flex_coef_f64(c);
+    const dim3 b(TX, TY), g((nx + TX - 1) / TX, (ny + TY64 - 1) / TY64);
+    if (rprev)
+        k_flexure64_stage<<<g, b, 0, s>>>(x, rprev, wref, q0, mask, D, inv2eta, f, nx, ny, cf, ctl, a, spy);
+    else
+        k_flexure64<<<g, b, 0, s>>>(x, wref, q0, mask, D, inv2eta, f, nx, ny, cf, nullptr);
+}
+
 __global__ void __launch_bounds__(TX* TY)
 k_flexure_f32(const double* __restrict__ y, const double* __restrict__ wref, const float* __restrict__ q0,
               const uint8_t* __restrict__ mask, const float* __restrict__ D, const float* __restrict__ inv2eta,
@@ -637,6 +780,12 @@ void launch_flexure(const double* y, const double* wref, const T* q0, const uint
         }
         k_flexure_f32<<<g, b, 0, s>>>(y, wref, (const float*)q0, mask, (const float*)D, (const float*)inv2eta,
                                       (float*)f, nx, ny, cf, gate);
+        return;
+    }
+    if (sizeof(T) == 8 && c.dxm == nullptr) {
+        k_flexure64<<<dim3((nx + TX - 1) / TX, (ny + TY64 - 1) / TY64), b, 0, s>>>(
+            y, wref, (const double*)q0, mask, (const double*)D, (const double*)inv2eta, (double*)f, nx, ny,
+            flex_coef_f64(c), gate);
         return;
     }
     k_flexure<T><<<g, b, 0, s>>>(y, wref, q0, mask, D, inv2eta, f, nx, ny, c, gate);
@@ -1075,6 +1224,9 @@ __global__ void __launch_bounds__(256) k_b_flexure(const BMember* __restrict__ M
             if (task < strip_tasks(b.p.nx, b.p.ny, b.fseg))
                 flexure_strip<true>(b.d.whi, b.d.wlo, (const float*)b.q0, b.mask, (const float*)b.D,
                               (const float*)b.inv2eta, (float*)b.f, b.p.nx, b.p.ny, b.fcf, b.fseg, task);
+        } else if (b.fc.dxm == nullptr) {
+            flexure_tile64<false>(b.y, nullptr, nullptr, (const double*)b.q0, b.mask, (const double*)b.D,
+                                  (const double*)b.inv2eta, (double*)b.f, b.p.nx, b.p.ny, b.fc64, bx, by);
         } else {
             flexure_body<T>(b.y, nullptr, (const T*)b.q0, b.mask, (const T*)b.D, (const T*)b.inv2eta, (T*)b.f,
                             b.p.nx, b.p.ny, b.fc, bx, by);
@@ -1161,6 +1313,7 @@ template <typename T> void batch_flexure(const BMember* M, BList L, int nblk, cu
     // 256 threads: the tile body reads them as TX x TY, the strip body as 8 warps
     k_b_flexure<T><<<nblk, dim3(TX, TY), 0, s>>>(M, L);
 }
+int batch_flexure_tiles64(int nx, int ny) { return ((nx + TX - 1) / TX) * ((ny + TY64 - 1) / TY64); }
 int batch_flexure_blocks(int nx, int ny, int seg) { return (((nx + SW - 1) / SW) * ((ny + seg - 1) / seg) + 7) / 8; }
 template <typename T>
 void batch_rows_fwd(const BMember* M, BList L, int nblk, int threads, size_t smem, cudaStream_t s)
@@ -1206,6 +1359,9 @@ __global__ void __launch_bounds__(256) k_b_flexure_y(const BMember* __restrict__
                 flexure_f32_body<false>(y, b.wref, (const float*)b.q0, b.mask, (const float*)b.D,
                                         (const float*)b.inv2eta, (float*)b.f, b.p.nx, b.p.ny, b.fcf, bx, by);
             }
+        } else if (b.fc.dxm == nullptr) {
+            flexure_tile64<false>(y, nullptr, b.wref, (const double*)b.q0, b.mask, (const double*)b.D,
+                                  (const double*)b.inv2eta, (double*)b.f, b.p.nx, b.p.ny, b.fc64, bx, by);
         } else {
             flexure_body<T>(y, b.wref, (const T*)b.q0, b.mask, (const T*)b.D, (const T*)b.inv2eta, (T*)b.f, b.p.nx,
                             b.p.ny, b.fc, bx, by);
