@@ -640,8 +640,11 @@ __device__ __forceinline__ void flexure_tile64(const double* __restrict__ x, con
             const int ly = my + 1, lx = mx + 1;
             const double Dl = __ldg(D + (size_t)(j0 - 1 + my) * nx + (i0 - 1 + mx));
             const double y = ys[ly][lx];
-            const double wxx = (ys[ly][lx + 1] + ys[ly][lx - 1]) - 2.0 * y;
-            const double wyy = (ys[ly + 1][lx] + ys[ly - 1][lx]) - 2.0 * y;
+            // differences of first differences, which are exact between
+            // neighbours of a smooth field (a sum of neighbours less 2 y saves
+            // two instructions and rounds at the size of y)
+            const double wxx = (ys[ly][lx + 1] - y) - (y - ys[ly][lx - 1]);
+            const double wyy = (ys[ly + 1][lx] - y) - (y - ys[ly - 1][lx]);
             const double wxy = (ys[ly + 1][lx + 1] - ys[ly + 1][lx - 1]) - (ys[ly - 1][lx + 1] - ys[ly - 1][lx - 1]);
             Mxx[my][mx] = Dl * (wxx + c.rxy * wyy);
             Myy[my][mx] = Dl * (wyy + c.ryx * wxx);
@@ -659,8 +662,8 @@ __device__ __forceinline__ void flexure_tile64(const double* __restrict__ x, con
             const int xl = lx - (gi > 0), xr = lx + (gi < nx - 1), yl = ly - (gj > 0), yr = ly + (gj < ny - 1);
             const double tw = (xr - xl == 2 ? 1.0 : 2.0) * (yr - yl == 2 ? 1.0 : 2.0);
             const double Dl = __ldg(D + (size_t)gj * nx + gi);
-            const double wxx = (ys[ly][cx + 1] + ys[ly][cx - 1]) - 2.0 * ys[ly][cx];
-            const double wyy = (ys[cy + 1][lx] + ys[cy - 1][lx]) - 2.0 * ys[cy][lx];
+            const double wxx = (ys[ly][cx + 1] - ys[ly][cx]) - (ys[ly][cx] - ys[ly][cx - 1]);
+            const double wyy = (ys[cy + 1][lx] - ys[cy][lx]) - (ys[cy][lx] - ys[cy - 1][lx]);
             const double wxy = tw * ((ys[yr][xr] - ys[yr][xl]) - (ys[yl][xr] - ys[yl][xl]));
             Mxx[my][mx] = Dl * (wxx + c.rxy * wyy);
             Myy[my][mx] = Dl * (wyy + c.ryx * wxx);
