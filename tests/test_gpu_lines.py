@@ -34,6 +34,18 @@ def _domain(name, nx, ny, precision):
                                         (2048, 34, True), (48, 1536, False), (1536, 96, True), (384, 192, False),
                                         (768, 24, True), (96, 768, False)])
 def test_rate_on_lines(nx, ny, even, precision):
+    _check_rate(nx, ny, even, precision)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("nx,ny,even", [(70, 44, True), (50, 98, False), (154, 26, False), (34, 250, True),
+                                        (122, 142, False)])
+def test_rate_with_odd_radices(nx, ny, even, precision):
+    """Radices 5 and 7 in registers, larger primes by the symmetry of their roots."""
+    _check_rate(nx, ny, even, precision)
+
+
+def _check_rate(nx, ny, even, precision):
     dom, p = _domain("test1d", nx, ny, precision)
     rng = np.random.default_rng(nx + ny)
     w, cf = rng.standard_normal((ny, nx)) * 100, rng.standard_normal((ny, nx)) * 1e5
