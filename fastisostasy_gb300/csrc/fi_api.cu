@@ -323,7 +323,7 @@ struct fi_handle {
     size_t hpin_elems = 0;
     const double** gsrc = nullptr;
     const uint8_t** gmsrc = nullptr;
-    double *dxm = nullptr, *dym = nullptr;
+    double *ixm = nullptr, *iym = nullptr;   // 1/(dx K), 1/(dy K) on a distorted grid
     // reference-state device pointers (non-const views)
     double *z_bed_ref, *Hice_ref, *Haf_ref, *z_ss_ref, *we_ref, *w_ref, *dz_ss_ref;
     uint8_t *mo_ref, *mg_ref, *mc_ref;
@@ -1765,11 +1765,15 @@ int fi_create(const fi_params* pin, int nx_ice, int ny_ice, double dx, double dy
         h->fc.inv_2dy = 1.0 / (2 * dy);
         h->fc.inv_dy2 = 1.0 / (dy * dy);
         if (!h->uniform) {
-            AL(h->dxm, n * 8);
-            AL(h->dym, n * 8);
-            if ((rc = upload(h, h->dxm, dxm.data(), n * 8)) || (rc = upload(h, h->dym, dym.data(), n * 8))) return rc;
-            h->fc.dxm = h->dxm;
-            h->fc.dym = h->dym;
+            AL(h->ixm, n * 8);
+            AL(h->iym, n * 8);
+            for (size_t e = 0; e < n; ++e) {
+                dxm[e] = 1.0 / dxm[e];
+                dym[e] = 1.0 / dym[e];
+            }
+            if ((rc = upload(h, h->ixm, dxm.data(), n * 8)) || (rc = upload(h, h->iym, dym.data(), n * 8))) return rc;
+            h->fc.ixm = h->ixm;
+            h->fc.iym = h->iym;
         }
     }
 #undef AL
@@ -2352,7 +2356,7 @@ int fi_lvelva(fi_handle* h, const double* w, const double* canom_full, double* d
     if ((rc = upload(h, h->y, w, n * 8)) || (rc = upload(h, tmp, canom_full, n * 8))) return rc;
     if (mixed(h)) {
         q0_from_cf<float>((float*)h->q0, tmp, h->d.mactive, h->p.g, n, h->s);
-        if (h->p.method == 3 && h->fc.dxm == nullptr) {
+        if (h->p.method == 3 && h->fc.ixm == nullptr) {
             // uniform spacing: w as a float pair through the column-strip
             // stencil, as the mixed reference-compatible Tsit5 evaluates it
             float* pair;
@@ -2552,8 +2556,7 @@ int batch_shape(fi_batch* b, int RB, int CB, int fseg, int waves)
         m.fseg = fseg;
         const int fblk = b->mixed ? (!b->true_stages || m.yhi ? batch_flexure_blocks(m.p.nx, m.p.ny, m.fseg)
                                                               : m.fgx * ((m.p.ny + 7) / 8))
-                         : m.fc.dxm == nullptr ? batch_flexure_tiles64(m.p.nx, m.p.ny)
-                                               : m.fgx * ((m.p.ny + 7) / 8);
+                                  : batch_flexure_tiles64(m.p.nx, m.p.ny);
         const int rblk = (m.p.ny + m.RB - 1) / m.RB;
         const int cblk = (m.p.h + 1 + m.CB - 1) / m.CB;
         off[i + 1] = off[i] + fblk;
@@ -2800,7 +2803,7 @@ int fi_batch_create(fi_handle* const* hs, int n, fi_batch** out)
         if (!h->state_ready) return fail(h, FI_E_STATE, "fi_batch_create before fi_init_state");
         const fi_handle* h0 = hs[0];
         if (h->p.method != 3 || h->p.dt_method != 2 || h->p.stage_mode != h0->p.stage_mode || mixed(h) != mixed(h0) ||
-            (mixed(h) && h->p.stage_mode == 0 && !h->d.whi) || (mixed(h) && h->fc.dxm != nullptr) ||
+            (mixed(h) && h->p.stage_mode == 0 && !h->d.whi) || (mixed(h) && h->fc.ixm != nullptr) ||
             h->p.dt_diagnostics != h0->p.dt_diagnostics || h->time_diag != h0->time_diag || !h->tsit_graph_ok)
             return fail(h, FI_E_CONFIG,
                         "batched members must run tsit54 with the same stage mode and precision, in lockstep "
@@ -2821,7 +2824,7 @@ int fi_batch_create(fi_handle* const* hs, int n, fi_batch** out)
         m.p = h->prhs;
         m.fc = h->fc;
         m.fcf = flex_coef_f32(h->fc);
-        if (!h->fc.dxm) m.fc64 = flex_coef_f64(h->fc);
+        if (!h->fc.ixm) m.fc64 = flex_coef_f64(h->fc);
         m.norm_scale = 1.0 / (double)(float)((long long)h->prhs.nx * h->prhs.ny);   // nx*ny*1. (default real)
         m.norm_scale_f = (float)m.norm_scale;
         m.y = h->d.w;

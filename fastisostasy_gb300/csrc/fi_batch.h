@@ -83,7 +83,7 @@ inline BList blist(const int* base, int nm, int kind)
 
 // Virtual blocks of the mixed batched flexure (8 column-strip warp tasks each).
 int batch_flexure_blocks(int nx, int ny, int seg);
-// ... and of the FP64 one on uniform spacing (32 x 16 tiles).
+// ... and of the FP64 one (32 x 16 tiles).
 int batch_flexure_tiles64(int nx, int ny);
 
 // Block shapes of the single-domain launches (shared with the batched ones).

@@ -13,8 +13,8 @@ struct FlexCoef {
     double nu, one_minus_nu;
     double coef_mantle;            // -g*rho_m in true-stage mode (mantle anomaly at the stage state), else 0
     double inv_dx, inv_2dx, inv_dx2, inv_dy, inv_2dy, inv_dy2;
-    const double* dxm;             // per-cell dx*K, or null for uniform spacing
-    const double* dym;
+    const double* ixm;             // per-cell 1/(dx*K), or null for uniform spacing
+    const double* iym;
 };
 
 // The same coefficients rounded to float (mixed form, uniform spacing).

@@ -139,12 +139,14 @@ int line_block(int lines, int th, int most)
 }  // namespace
 
 // Lines per block where nothing was tuned: 128 threads for rows, 32-byte
-// segments for columns.
+// segments for columns; half of that in double precision, where the time of a
+// small grid is the FP64 instructions of its busiest SM quarter.
 template <typename T, int N, bool COL> int line_default()
 {
     constexpr int th = LineShape<T, N>::threads;
-    if (COL) return sizeof(T) == 4 ? 4 : 2;
-    return th >= 128 ? 1 : 128 / th;
+    if (COL) return sizeof(T) == 4 ? 4 : 1;
+    constexpr int most = sizeof(T) == 4 ? 128 : 64;
+    return th >= most ? 1 : most / th;
 }
 
 #define FI_LAUNCH(kern, N, lines, count, ...)                                                          \

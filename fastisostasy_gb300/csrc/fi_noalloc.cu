@@ -61,33 +61,45 @@ static_assert(NA_BYTES == 3219472, "scratch size stated in the header comment");
 
 static __device__ __align__(256) unsigned char g_fi_static_scratch[NA_BYTES];
 
-// exp(-2 pi i t / n) for t < n, and exp(-2 pi i k / nx) for k <= nx/2
-__global__ void k_na_twiddles(double2* twr, int nr, double2* twc, int nc, double2* rtw, int nx)
+// Everything a call derives from its arguments before the stencil, in one
+// launch: the load term, 1/(2 eta) and the multipliers m(k, l), m(-k, l) in the
+// half-spectrum layout, 1/(dx K) and 1/(dy K) of a distorted grid, and, in the
+// blocks after those of the grid, the twiddles exp(-2 pi i t / n), one a
+// thread (an FP64 sine is a chain of hundreds of FP64 instructions, three in a
+// row took 9 us in a launch of their own).
+__global__ void k_na_prepare(const double* __restrict__ cf, const uint8_t* __restrict__ mask,
+                             const double* __restrict__ eta, const double* __restrict__ kappa,
+                             const double* __restrict__ R, const double* __restrict__ dxm,
+                             const double* __restrict__ dym, double g, int nx, int ny, int sp, double* q0, double* i2e,
+                             double* mA, double* mB, double* ixm, double* iym, double2* twr, double2* twc,
+                             double2* rtw)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    double s, c;
-    if (t < nr) { sincospi(-2.0 * t / nr, &s, &c); twr[t] = make_double2(c, s); }
-    if (t < nc) { sincospi(-2.0 * t / nc, &s, &c); twc[t] = make_double2(c, s); }
-    if (t <= nx / 2) { sincospi(-2.0 * t / nx, &s, &c); rtw[t] = make_double2(c, s); }
-}
-
-// load term, 1/(2 eta) and the multipliers m(k, l), m(-k, l) in the half-spectrum layout
-__global__ void k_na_fields(const double* __restrict__ cf, const uint8_t* __restrict__ mask,
-                            const double* __restrict__ eta, const double* __restrict__ kappa,
-                            const double* __restrict__ R, double g, int nx, int ny, int sp, double* q0,
-                            double* i2e, double* mA, double* mB)
-{
-    const size_t n = (size_t)nx * ny;
-    const int h = nx / 2;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-        q0[e] = mask[e] ? -g * cf[e] : 0.0;
-        i2e[e] = 1.0 / (2.0 * eta[e]);
-        const int i = (int)(e % nx), l = (int)(e / nx);
-        if (i <= h) {
-            const size_t a = (size_t)l * nx + i, b = (size_t)l * nx + (nx - i) % nx;
-            mA[(size_t)l * sp + i] = 1.0 / (kappa[a] * R[a]);
-            mB[(size_t)l * sp + i] = 1.0 / (kappa[b] * R[b]);
-        }
+    const int n = nx * ny, h = nx / 2;
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    const int cells = (n + (int)blockDim.x - 1) / (int)blockDim.x * (int)blockDim.x;
+    if (e >= cells) {
+        int t = e - cells, len = h;
+        double2* out = twr;
+        if (t >= h) { t -= h; len = ny; out = twc; }
+        if (out == twc && t >= ny) { t -= ny; len = nx; out = rtw; }
+        if (out == rtw && t > h) return;
+        double s, c;
+        sincospi(-2.0 * t / len, &s, &c);
+        out[t] = make_double2(c, s);
+        return;
+    }
+    if (e >= n) return;
+    q0[e] = mask[e] ? -g * cf[e] : 0.0;
+    i2e[e] = 1.0 / (2.0 * eta[e]);
+    if (dxm) {
+        ixm[e] = 1.0 / dxm[e];
+        iym[e] = 1.0 / dym[e];
+    }
+    const int i = e % nx, l = e / nx;
+    if (i <= h) {
+        const int a = l * nx + i, b = l * nx + (nx - i) % nx;
+        mA[l * sp + i] = 1.0 / (kappa[a] * R[a]);
+        mB[l * sp + i] = 1.0 / (kappa[b] * R[b]);
     }
 }
 
@@ -150,10 +162,13 @@ extern "C" int fi_lvelva_static(const double* d_w, const double* d_canom_full, c
     p.col.tw64 = twc;
     p.rtw64 = rtw;
 
-    const int nt = ny > nx / 2 + 1 ? ny : nx / 2 + 1;
-    k_na_twiddles<<<(nt + 255) / 256, 256, 0, s>>>(twr, p.h, twc, ny, rtw, nx);
-    k_na_fields<<<(int)(((size_t)nx * ny + 255) / 256), 256, 0, s>>>(d_canom_full, d_maskactive, d_eta_eff, d_kappa,
-                                                                     d_R, g, nx, ny, p.sp, q0, i2e, mA, mB);
+    // the inverse spacings live where the transforms write later: the raw
+    // output and the half spectrum
+    double* ixm = raw;
+    double* iym = reinterpret_cast<double*>(S);
+    const int nb = (nx * ny + 255) / 256, tb = (p.h + ny + p.h + 1 + 255) / 256;
+    k_na_prepare<<<nb + tb, 256, 0, s>>>(d_canom_full, d_maskactive, d_eta_eff, d_kappa, d_R, d_dx_matrix, d_dy_matrix, g,
+                                         nx, ny, p.sp, q0, i2e, mA, mB, ixm, iym, twr, twc, rtw);
     FlexCoef c;
     memset(&c, 0, sizeof(c));
     c.nu = nu;
@@ -164,8 +179,10 @@ extern "C" int fi_lvelva_static(const double* d_w, const double* d_canom_full, c
     c.inv_dy = 1.0 / dy;
     c.inv_2dy = 1.0 / (2 * dy);
     c.inv_dy2 = 1.0 / (dy * dy);
-    c.dxm = d_dx_matrix;   // null: uniform spacing from dx, dy
-    c.dym = d_dy_matrix;
+    if (d_dx_matrix) {   // else uniform spacing from dx, dy
+        c.ixm = ixm;
+        c.iym = iym;
+    }
     launch_flexure<double>(d_w, nullptr, q0, d_maskactive, d_D_lith, i2e, f, nx, ny, c, s);
     launch_rows_fwd<double>(f, nx, nx, ny, S, p, s);
     launch_cols_hartley<double>(S, mA, mB, 0, p, s);

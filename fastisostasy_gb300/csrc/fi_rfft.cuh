@@ -30,11 +30,14 @@ namespace fi {
 
 // points per thread: 8 keeps a double-precision line at 32 data registers;
 // 16 saves an exchange where a float line is long (1024 = 16 16 4 against
-// 8 8 8 2).  Lengths 3 2^k: 12 (radices 4, 2 and a last 3), or 24 (8, 4, 2, 3)
+// 8 8 8 2).  Double lines up to 256 points have 4: a small FP64 grid has fewer
+// warps than the GPU has SM quarters, and an FP64 instruction takes a quarter
+// 64 clocks however little it has to do (256^2: rows 12.1 -> 8.2 us, columns
+// 23 -> 14.7; 512^2 rows unchanged).  Lengths 3 2^k: 12 (radices 4, 2 and a last 3), or 24 (8, 4, 2, 3)
 // where a float line is long.
 __host__ __device__ constexpr int line_points(int n, bool f32)
 {
-    return n % 3 == 0 ? (f32 && n >= 768 ? 24 : 12) : f32 && n >= 1024 ? 16 : 8;
+    return n % 3 == 0 ? (f32 && n >= 768 ? 24 : 12) : f32 ? (n >= 1024 ? 16 : 8) : n <= 256 ? 4 : 8;
 }
 template <typename T, int N> struct LineShape {
     static constexpr int E = line_points(N, sizeof(T) == 4);

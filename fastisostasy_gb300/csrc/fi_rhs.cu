@@ -77,22 +77,24 @@ __device__ __forceinline__ void flexure_body(const double* __restrict__ y, const
     __shared__ T Mxyx[RY][RX];
     const int tid = threadIdx.x + TX * threadIdx.y;
     const int i0 = bx * TX, j0 = by * TY;
-    const bool uni = (c.dxm == nullptr);
+    const bool uni = (c.ixm == nullptr);
 
     // per-cell spacing accessors (uniform fast path)
-    auto idx1 = [&](int i, int j) -> double { return uni ? c.inv_dx : 1.0 / c.dxm[(size_t)j * nx + i]; };
-    auto idx2h = [&](int i, int j) -> double { return uni ? c.inv_2dx : 1.0 / (2 * c.dxm[(size_t)j * nx + i]); };
+    // (1/(2 d) and 1/d^2 from the stored 1/d: an FP64 division is a chain of a
+    // dozen FP64 instructions, and a cell took eight)
+    auto idx1 = [&](int i, int j) -> double { return uni ? c.inv_dx : c.ixm[(size_t)j * nx + i]; };
+    auto idx2h = [&](int i, int j) -> double { return uni ? c.inv_2dx : 0.5 * c.ixm[(size_t)j * nx + i]; };
     auto idxx = [&](int i, int j) -> double {
         if (uni) return c.inv_dx2;
-        const double d = c.dxm[(size_t)j * nx + i];
-        return 1.0 / (d * d);
+        const double d = c.ixm[(size_t)j * nx + i];
+        return d * d;
     };
-    auto idy1 = [&](int i, int j) -> double { return uni ? c.inv_dy : 1.0 / c.dym[(size_t)j * nx + i]; };
-    auto idy2h = [&](int i, int j) -> double { return uni ? c.inv_2dy : 1.0 / (2 * c.dym[(size_t)j * nx + i]); };
+    auto idy1 = [&](int i, int j) -> double { return uni ? c.inv_dy : c.iym[(size_t)j * nx + i]; };
+    auto idy2h = [&](int i, int j) -> double { return uni ? c.inv_2dy : 0.5 * c.iym[(size_t)j * nx + i]; };
     auto idyy = [&](int i, int j) -> double {
         if (uni) return c.inv_dy2;
-        const double d = c.dym[(size_t)j * nx + i];
-        return 1.0 / (d * d);
+        const double d = c.iym[(size_t)j * nx + i];
+        return d * d;
     };
 
     for (int e = tid; e < RX * RY; e += TX * TY) {
@@ -699,6 +701,97 @@ __device__ __forceinline__ void flexure_tile64(const double* __restrict__ x, con
     }
 }
 
+// The same tile on a distorted grid: 1/(dx K), 1/(dy K) per cell (ixm, iym).
+// A first difference takes the spacing of the cell it is taken at, a second
+// one that cell's squared; the last column's second x-difference takes the
+// first column's, as the reference does (src/finite_differences.f90:90-91).
+// (256^2: 26.5 us with a division per difference on 32 x 8 tiles, 17 with the
+// stored inverses, 14 on these tiles.)
+__device__ __forceinline__ void flexure_tile64k(const double* __restrict__ x, const double* __restrict__ wref,
+                                                const double* __restrict__ q0, const uint8_t* __restrict__ mask,
+                                                const double* __restrict__ D, const double* __restrict__ inv2eta,
+                                                double* __restrict__ f, int nx, int ny, const FlexCoef& c, int bx,
+                                                int by)
+{
+    __shared__ double ys[YR][YC];
+    __shared__ double Mxx[MR][MC], Myy[MR][MC], Mxy[MR][MC];
+    const int tid = (int)(threadIdx.x + threadIdx.y * blockDim.x);   // 1D or 32 x 8 blocks
+    const int i0 = bx * TX, j0 = by * TY64;
+    for (int e = tid; e < YR * YC; e += TX * TY) {
+        const int ly = e / YC, lx = e - ly * YC;
+        const int gi = i0 - 2 + lx, gj = j0 - 2 + ly;
+        ys[ly][lx] = gi >= 0 && gi < nx && gj >= 0 && gj < ny ? __ldg(x + (size_t)gj * nx + gi) : 0.0;
+    }
+    __syncthreads();
+    // neighbours of grid cell (gi, gj) and its spacings: centre of the second
+    // differences, ends of the first ones, 1/span of those in x at the two
+    // rows and in y
+    struct Nb {
+        int cx, cy, xl, xr, yl, yr;
+        double sl, sr, sy, ixx, iyy;
+    };
+    auto nb = [&](int gi, int gj) {
+        Nb n;
+        n.cx = (gi == 0) - (gi == nx - 1);
+        n.cy = (gj == 0) - (gj == ny - 1);
+        n.xl = -(gi > 0);
+        n.xr = gi < nx - 1;
+        n.yl = -(gj > 0);
+        n.yr = gj < ny - 1;
+        const size_t g = (size_t)gj * nx + gi;
+        const double hx = n.xr - n.xl == 2 ? 0.5 : 1.0, hy = n.yr - n.yl == 2 ? 0.5 : 1.0;
+        n.sl = hx * __ldg(c.ixm + (ptrdiff_t)g + (ptrdiff_t)n.yl * nx);
+        n.sr = hx * __ldg(c.ixm + (ptrdiff_t)g + (ptrdiff_t)n.yr * nx);
+        const double iy = __ldg(c.iym + g), ix = __ldg(c.ixm + (gi == nx - 1 ? g - gi : g));
+        n.sy = hy * iy;
+        n.ixx = ix * ix;
+        n.iyy = iy * iy;
+        return n;
+    };
+    const double nu = c.nu, omn = c.one_minus_nu;
+    for (int e = tid; e < MR * MC; e += TX * TY) {
+        const int my = e / MC, mx = e - my * MC;
+        const int gi = i0 - 1 + mx, gj = j0 - 1 + my;
+        if (gi < 0 || gi >= nx || gj < 0 || gj >= ny) continue;
+        const Nb n = nb(gi, gj);
+        const int ly = my + 1, lx = mx + 1, cx = lx + n.cx, cy = ly + n.cy;
+        const double Dl = __ldg(D + (size_t)gj * nx + gi);
+        const double wxx = ((ys[ly][cx + 1] - ys[ly][cx]) - (ys[ly][cx] - ys[ly][cx - 1])) * n.ixx;
+        const double wyy = ((ys[cy + 1][lx] - ys[cy][lx]) - (ys[cy][lx] - ys[cy - 1][lx])) * n.iyy;
+        const double wxy = ((ys[ly + n.yr][lx + n.xr] - ys[ly + n.yr][lx + n.xl]) * n.sr -
+                            (ys[ly + n.yl][lx + n.xr] - ys[ly + n.yl][lx + n.xl]) * n.sl) * n.sy;
+        Mxx[my][mx] = -Dl * (wxx + nu * wyy);
+        Myy[my][mx] = -Dl * (wyy + nu * wxx);
+        Mxy[my][mx] = (-Dl * omn) * wxy;
+    }
+    __syncthreads();
+    for (int e = tid; e < TX * TY64; e += TX * TY) {
+        const int ly = e / TX, lx = e - ly * TX;
+        const int gi = i0 + lx, gj = j0 + ly;
+        if (gi >= nx || gj >= ny) continue;
+        const size_t g = (size_t)gj * nx + gi;
+        const Nb n = nb(gi, gj);
+        const int my = ly + 1, mx = lx + 1, cx = mx + n.cx, cy = my + n.cy;
+        const double mxx = ((Mxx[my][cx + 1] - Mxx[my][cx]) - (Mxx[my][cx] - Mxx[my][cx - 1])) * n.ixx;
+        const double myy = ((Myy[cy + 1][mx] - Myy[cy][mx]) - (Myy[cy][mx] - Myy[cy - 1][mx])) * n.iyy;
+        const double mxy = ((Mxy[my + n.yr][mx + n.xr] - Mxy[my + n.yr][mx + n.xl]) * n.sr -
+                            (Mxy[my + n.yl][mx + n.xr] - Mxy[my + n.yl][mx + n.xl]) * n.sl) * n.sy;
+        double p = __ldg(q0 + g);
+        if (wref) p += c.coef_mantle * (ys[ly + 2][lx + 2] - __ldg(wref + g));
+        if (__ldg(mask + g) == 0) p = 0.0;
+        f[g] = (((p + mxx) + 2.0 * mxy) + myy) * __ldg(inv2eta + g);
+    }
+}
+
+__global__ void __launch_bounds__(TX* TY)
+k_flexure64k(const double* __restrict__ y, const double* __restrict__ wref, const double* __restrict__ q0,
+             const uint8_t* __restrict__ mask, const double* __restrict__ D, const double* __restrict__ inv2eta,
+             double* __restrict__ f, int nx, int ny, FlexCoef c, const int* __restrict__ gate)
+{
+    if (gate && *gate == 0) return;
+    flexure_tile64k(y, wref, q0, mask, D, inv2eta, f, nx, ny, c, blockIdx.x, blockIdx.y);
+}
+
 __global__ void __launch_bounds__(TX* TY)
 k_flexure64(const double* __restrict__ y, const double* __restrict__ wref, const double* __restrict__ q0,
             const uint8_t* __restrict__ mask, const double* __restrict__ D, const double* __restrict__ inv2eta,
@@ -759,7 +852,7 @@ void launch_flexure(const double* y, const double* wref, const T* q0, const uint
                     const float* whi, const float* wlo)
 {
     dim3 b(TX, TY), g((nx + TX - 1) / TX, (ny + TY - 1) / TY);
-    if (sizeof(T) == 4 && c.dxm == nullptr) {
+    if (sizeof(T) == 4 && c.ixm == nullptr) {
         const FlexCoefF cf = flex_coef_f32(c);
         if (whi && !wref) {
             const int seg = strip_seg_single(nx, ny);
@@ -785,13 +878,15 @@ void launch_flexure(const double* y, const double* wref, const T* q0, const uint
                                       (float*)f, nx, ny, cf, gate);
         return;
     }
-    if (sizeof(T) == 8 && c.dxm == nullptr) {
-        k_flexure64<<<dim3((nx + TX - 1) / TX, (ny + TY64 - 1) / TY64), b, 0, s>>>(
-            y, wref, (const double*)q0, mask, (const double*)D, (const double*)inv2eta, (double*)f, nx, ny,
-            flex_coef_f64(c), gate);
-        return;
+    if constexpr (sizeof(T) == 8) {
+        const dim3 g64((nx + TX - 1) / TX, (ny + TY64 - 1) / TY64);
+        if (c.ixm == nullptr)
+            k_flexure64<<<g64, b, 0, s>>>(y, wref, q0, mask, D, inv2eta, f, nx, ny, flex_coef_f64(c), gate);
+        else
+            k_flexure64k<<<g64, b, 0, s>>>(y, wref, q0, mask, D, inv2eta, f, nx, ny, c, gate);
+    } else {
+        k_flexure<T><<<g, b, 0, s>>>(y, wref, q0, mask, D, inv2eta, f, nx, ny, c, gate);
     }
-    k_flexure<T><<<g, b, 0, s>>>(y, wref, q0, mask, D, inv2eta, f, nx, ny, c, gate);
 }
 
 void launch_flexure_stage(const float* whi, const float* wlo, const float* rprev, const float* dxw, const float* q0,
@@ -1227,12 +1322,12 @@ __global__ void __launch_bounds__(256) k_b_flexure(const BMember* __restrict__ M
             if (task < strip_tasks(b.p.nx, b.p.ny, b.fseg))
                 flexure_strip<true>(b.d.whi, b.d.wlo, (const float*)b.q0, b.mask, (const float*)b.D,
                               (const float*)b.inv2eta, (float*)b.f, b.p.nx, b.p.ny, b.fcf, b.fseg, task);
-        } else if (b.fc.dxm == nullptr) {
+        } else if (b.fc.ixm == nullptr) {
             flexure_tile64<false>(b.y, nullptr, nullptr, (const double*)b.q0, b.mask, (const double*)b.D,
                                   (const double*)b.inv2eta, (double*)b.f, b.p.nx, b.p.ny, b.fc64, bx, by);
         } else {
-            flexure_body<T>(b.y, nullptr, (const T*)b.q0, b.mask, (const T*)b.D, (const T*)b.inv2eta, (T*)b.f,
-                            b.p.nx, b.p.ny, b.fc, bx, by);
+            flexure_tile64k(b.y, nullptr, (const double*)b.q0, b.mask, (const double*)b.D, (const double*)b.inv2eta,
+                            (double*)b.f, b.p.nx, b.p.ny, b.fc, bx, by);
         }
         __syncthreads();   // the next virtual block reuses the shared tiles
     });
@@ -1362,12 +1457,12 @@ __global__ void __launch_bounds__(256) k_b_flexure_y(const BMember* __restrict__
                 flexure_f32_body<false>(y, b.wref, (const float*)b.q0, b.mask, (const float*)b.D,
                                         (const float*)b.inv2eta, (float*)b.f, b.p.nx, b.p.ny, b.fcf, bx, by);
             }
-        } else if (b.fc.dxm == nullptr) {
+        } else if (b.fc.ixm == nullptr) {
             flexure_tile64<false>(y, nullptr, b.wref, (const double*)b.q0, b.mask, (const double*)b.D,
                                   (const double*)b.inv2eta, (double*)b.f, b.p.nx, b.p.ny, b.fc64, bx, by);
         } else {
-            flexure_body<T>(y, b.wref, (const T*)b.q0, b.mask, (const T*)b.D, (const T*)b.inv2eta, (T*)b.f, b.p.nx,
-                            b.p.ny, b.fc, bx, by);
+            flexure_tile64k(y, b.wref, (const double*)b.q0, b.mask, (const double*)b.D, (const double*)b.inv2eta,
+                            (double*)b.f, b.p.nx, b.p.ny, b.fc, bx, by);
         }
         __syncthreads();
     });
