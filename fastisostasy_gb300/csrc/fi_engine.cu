@@ -25,7 +25,7 @@
 #include <type_traits>
 
 #include "fi_engine.h"
-#include "fi_fft.cuh"
+#include "fi_lines.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -146,7 +146,7 @@ __device__ __forceinline__ void tmark(unsigned long long* tr)
 // ---------------------------------------------------------------------------
 // Phase A: one item = output rows j0 .. j0+RA-1 (full width).
 // ---------------------------------------------------------------------------
-template <typename T, int RA, int FM>
+template <typename T, int RA>
 __device__ void phase_a(const EngineArgs& g, int j0, int stage, float sdf_in, unsigned char* smem,
                         const EngTw<T>& tw)
 {
@@ -288,7 +288,7 @@ __device__ void phase_a(const EngineArgs& g, int j0, int stage, float sdf_in, un
     }
     __syncthreads();
     tmark(g.trace);
-    C2* r = block_fft<T, true, FM>(b0, b1, g.p.row.d, RA, hh, tw.row, -1);
+    C2* r = block_fft<T, true>(b0, b1, g.p.row.d, RA, hh, tw.row, -1);
     const C2* rtw = tw.rtw;
     // column-major: the strided stores do not hold the block up, and phase B
     // then reads each spectrum column contiguously
@@ -314,7 +314,7 @@ __device__ void phase_a(const EngineArgs& g, int j0, int stage, float sdf_in, un
 // inverse column FFT.  Columns come contiguous from the column-major copy
 // phase A wrote; the result goes back row-major for the row passes of C.
 // ---------------------------------------------------------------------------
-template <typename T, int FM>
+template <typename T>
 __device__ void phase_b(const EngineArgs& g, int k0, int CB, unsigned char* smem, const EngTw<T>& tw)
 {
     typedef typename vec2<T>::type C2;
@@ -330,7 +330,7 @@ __device__ void phase_b(const EngineArgs& g, int k0, int CB, unsigned char* smem
     }
     __syncthreads();
     tmark(g.trace);
-    C2* r = block_fft<T, true, FM>(b0, b1, g.p.col.d, CB, ny, tw.col, -1);
+    C2* r = block_fft<T, true>(b0, b1, g.p.col.d, CB, ny, tw.col, -1);
     const T* mA = g.mA_T<T>();
     const T* mB = g.mB_T<T>();
     const int half = ny / 2 + 1;
@@ -366,7 +366,7 @@ __device__ void phase_b(const EngineArgs& g, int k0, int CB, unsigned char* smem
     __syncthreads();
     tmark(g.trace);
     C2* other = (r == b0) ? b1 : b0;
-    C2* q = block_fft<T, true, FM>(r, other, g.p.col.d, CB, ny, tw.col, +1);
+    C2* q = block_fft<T, true>(r, other, g.p.col.d, CB, ny, tw.col, +1);
     for (int e = tid; e < CB * ny; e += nt) {
         const int c = CB == 1 ? 0 : e % CB, l = CB == 1 ? e : e / CB;
         const int k = k0 + c;
@@ -379,7 +379,7 @@ __device__ void phase_b(const EngineArgs& g, int k0, int CB, unsigned char* smem
 // ---------------------------------------------------------------------------
 // Phase C: inverse row real-FFT of rows j0 .. j0+RC-1 -> raw (scaled 1/(nx ny)).
 // ---------------------------------------------------------------------------
-template <typename T, int RC, int FM>
+template <typename T, int RC>
 __device__ void phase_c(const EngineArgs& g, int j0, T* out, unsigned char* smem, const EngTw<T>& tw)
 {
     typedef typename vec2<T>::type C2;
@@ -405,7 +405,7 @@ __device__ void phase_c(const EngineArgs& g, int j0, T* out, unsigned char* smem
     }
     __syncthreads();
     tmark(g.trace);
-    C2* r = block_fft<T, true, FM>(b0, b1, g.p.row.d, RC, hh, tw.row, +1);
+    C2* r = block_fft<T, true>(b0, b1, g.p.row.d, RC, hh, tw.row, +1);
     T scale;
     if constexpr (std::is_same<T, float>::value) scale = g.norm_scale_f;
     else scale = g.norm_scale;
@@ -416,6 +416,293 @@ __device__ void phase_c(const EngineArgs& g, int j0, T* out, unsigned char* smem
         v.x *= scale;
         v.y *= scale;
         *reinterpret_cast<C2*>(out + (size_t)j * nx + 2 * m) = v;
+    }
+    __syncthreads();
+    tmark(g.trace);
+}
+
+// ---------------------------------------------------------------------------
+// The phases where both lengths have a register line (FM == FFT_LINES): rows
+// transform in their warps, a column pair on its own few warps under a named
+// barrier, points in registers from the load to the store; the stencil is two
+// passes over the stage state's float pair (moments, then f), each thread
+// walking down a column, instead of five over its differences.  An update of
+// ten RK4 steps at 512^2 897 -> 660 us, at 256^2 600 -> 478.
+// ---------------------------------------------------------------------------
+enum { FFT_ANY = 0, FFT_LINES = 1 };   // FM
+
+template <int RA> __host__ __device__ inline size_t lines_a_bytes(int nx)
+{
+    return ((size_t)2 * (RA + 4) + 3 * (RA + 2)) * nx * sizeof(float);
+}
+template <int RA> __host__ __device__ inline size_t lines_tab_off(int nx, int h, int ny, int CB)
+{
+    const size_t a = lines_a_bytes<RA>(nx) + (size_t)RA * line_room(h, true) * sizeof(float2);
+    const size_t b = (size_t)CB * line_room(ny, true) * sizeof(float2);
+    return ((a > b ? a : b) + 15) & ~(size_t)15;
+}
+// row and column lengths of the line phases (their instances below)
+inline bool engine_line_rows(int h) { return h == 128 || h == 192 || h == 256; }
+inline bool engine_line_cols(int n) { return n == 256 || n == 384 || n == 512; }
+
+template <int RA, int H>
+__device__ __forceinline__ void engine_rows_fwd(float2* zb, const EngTw<float>& tw)
+{
+    constexpr int E = LineShape<float, H>::E, TH = LineShape<float, H>::threads, ROOM = line_smem<float, H>();
+    const int line = threadIdx.x / TH, t = threadIdx.x % TH;
+    if (line >= RA) return;   // whole warps
+    float2* b = zb + (size_t)line * ROOM;
+    float2 v[E];
+#pragma unroll
+    for (int m = 0; m < E; ++m) v[m] = b[t + TH * m];
+    line_fft<float, H, -1, 1, true>(v, b, tw.row, t);
+    __syncwarp();
+#pragma unroll
+    for (int m = 0; m < E; ++m) b[line_pad<E>(t + TH * m)] = v[m];
+}
+
+template <int RA> __device__ void phase_a_lines(const EngineArgs& g, int j0, int stage, float sdf, unsigned char* smem,
+                                                const EngTw<float>& tw)
+{
+    const int nx = g.p.nx, ny = g.p.ny, hh = g.p.h;
+    const int tid = threadIdx.x, ngrp = (int)blockDim.x / nx, grp = tid / nx, i = tid - grp * nx;
+    float* yh = reinterpret_cast<float*>(smem);
+    float* yl = yh + (RA + 4) * nx;
+    float* Mxx = yl + (RA + 4) * nx;
+    float* Myy = Mxx + (RA + 2) * nx;
+    float* Mxy = Myy + (RA + 2) * nx;
+    float2* zb = reinterpret_cast<float2*>(smem + lines_a_bytes<RA>(nx));
+    const int room = line_room(hh, true);
+    const float* rprev = stage > 0 ? (const float*)g.raw[stage - 1] : nullptr;
+    __shared__ float s_cmf;
+    float cf[4] = {0.f, 0.f, 0.f, 0.f};
+    if (tid == 0 && rprev) {   // corner values; their mean after the state has been requested (see phase_a)
+        const size_t last = (size_t)(ny - 1) * nx;
+        const float* q[4] = {rprev, rprev + last + nx - 1, rprev + last, rprev + nx - 1};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(cf[c]) : "l"(q[c]));
+    }
+    // the stage state x + sdf raw as a float pair, rows j0 - 2 .. j0 + RA + 1
+    if (grp < ngrp) {
+#pragma unroll
+        for (int q = 0; q < RA + 4; ++q) {
+            const int r = grp + q * ngrp, gj = j0 - 2 + r;
+            if (r >= RA + 4 || gj < 0 || gj >= ny) continue;
+            const size_t c = (size_t)gj * nx + i;
+            float hi = g.xhi[c], lo = g.xlo[c];
+            if (rprev) {
+                const float inc = sdf * rprev[c];
+                const float sm = hi + inc, bb = sm - hi;
+                const float er = (hi - (sm - bb)) + (inc - bb);
+                const float l2 = lo + er;
+                hi = sm + l2;
+                lo = l2 - (hi - sm);
+            }
+            yh[r * nx + i] = hi;
+            yl[r * nx + i] = lo;
+        }
+    }
+    if (tid == 0) s_cmf = rprev ? (float)corner_mean((double)cf[0], (double)cf[1], (double)cf[2], (double)cf[3]) : 0.f;
+    __syncthreads();
+    tmark(g.trace);
+    const bool left = i == 0, right = i == nx - 1;
+    const int ic = left ? 1 : right ? nx - 2 : i;       // centre of the second differences in x
+    const int il = left ? 0 : i - 1, ir = right ? nx - 1 : i + 1;
+    const float cx = left || right ? g.fcf.inv_dx : g.fcf.inv_2dx;
+    if (grp < ngrp) {
+        // moments of grid rows j0 - 1 .. j0 + RA; one-sided second differences
+        // are the central ones one cell inside
+        const int run = (RA + 2 + ngrp - 1) / ngrp;
+        int m0 = grp * run, m1 = m0 + run < RA + 2 ? m0 + run : RA + 2;
+        if (j0 == 0 && m0 == 0) m0 = 1;
+        if (m1 > ny + 1 - j0) m1 = ny + 1 - j0;
+        const float nu = g.fcf.nu, omn = g.fcf.one_minus_nu;
+        float w0 = 0.f, w1 = 0.f, w2, x1 = 0.f, x2, h0 = 0.f, h1 = 0.f, h2, l0 = 0.f, l1 = 0.f, l2;
+        auto row = [&](int j, float& w, float& x, float& h, float& l) {   // (rows beyond the grid are not used)
+            const int o = ((j < 0 ? 0 : j < ny ? j : ny - 1) - j0 + 2) * nx + ic;
+            const float ha = yh[o - 1], hb = yh[o], hc = yh[o + 1], la = yl[o - 1], lb = yl[o], lc = yl[o + 1];
+            const float dA = (hb - ha) + (lb - la), dB = (hc - hb) + (lc - lb);
+            x = (dB - dA) * g.fcf.inv_dx2;
+            w = (left ? dA : right ? dB : dA + dB) * cx;
+            h = left ? ha : right ? hc : hb;
+            l = left ? la : right ? lc : lb;
+        };
+        if (m0 < m1) {
+            row(j0 + m0 - 2, w0, x1, h0, l0);
+            row(j0 + m0 - 1, w1, x1, h1, l1);
+        }
+        for (int m = m0; m < m1; ++m) {
+            const int j = j0 - 1 + m, o = m * nx + i;
+            const float Dl = __ldg((const float*)g.D + (size_t)j * nx + i);
+            row(j + 1, w2, x2, h2, l2);
+            float wxy, wyy;
+            if (j == 0 || j == ny - 1) {
+                wxy = (j == 0 ? w2 - w1 : w1 - w0) * g.fcf.inv_dy;
+                const int c = ((j == 0 ? 1 : ny - 2) - j0 + 2) * nx + i;
+                wyy = (((yh[c + nx] - yh[c]) + (yl[c + nx] - yl[c])) - ((yh[c] - yh[c - nx]) + (yl[c] - yl[c - nx]))) *
+                      g.fcf.inv_dy2;
+            } else {
+                wxy = (w2 - w0) * g.fcf.inv_2dy;
+                wyy = (((h2 - h1) + (l2 - l1)) - ((h1 - h0) + (l1 - l0))) * g.fcf.inv_dy2;
+            }
+            Mxx[o] = -Dl * (x1 + nu * wyy);
+            Myy[o] = -Dl * (wyy + nu * x1);
+            Mxy[o] = (-Dl * omn) * wxy;
+            w0 = w1; w1 = w2; x1 = x2;
+            h0 = h1; h1 = h2; l0 = l1; l1 = l2;
+        }
+    }
+    __syncthreads();
+    tmark(g.trace);
+    if (grp < ngrp) {
+        const float cmd = sdf * s_cmf;
+        const int run = (RA + ngrp - 1) / ngrp;
+        const int oa = grp * run, ob = oa + run < RA ? oa + run : RA;
+        for (int o = oa; o < ob && j0 + o < ny; ++o) {
+            const int j = j0 + o, r = (o + 1) * nx;
+            const size_t c = (size_t)j * nx + i;
+            const float load = __ldg((const float*)g.q0 + c), ie = __ldg((const float*)g.inv2eta + c);
+            const float wh = __ldg(g.wrefhi + c), wl = __ldg(g.wreflo + c);
+            const uint32_t on = __ldg(g.mask + c);
+            const float mx_xx = ((Mxx[r + ic + 1] - 2.f * Mxx[r + ic]) + Mxx[r + ic - 1]) * g.fcf.inv_dx2;
+            const float qu = (Mxy[r - nx + ir] - Mxy[r - nx + il]) * cx, qd = (Mxy[r + nx + ir] - Mxy[r + nx + il]) * cx;
+            float mxy, my_yy;
+            if (j == 0 || j == ny - 1) {
+                const float qc = (Mxy[r + ir] - Mxy[r + il]) * cx;
+                mxy = (j == 0 ? qd - qc : qc - qu) * g.fcf.inv_dy;
+                const int k = ((j == 0 ? 1 : ny - 2) - j0 + 1) * nx + i;
+                my_yy = ((Myy[k + nx] - 2.f * Myy[k]) + Myy[k - nx]) * g.fcf.inv_dy2;
+            } else {
+                mxy = (qd - qu) * g.fcf.inv_2dy;
+                my_yy = ((Myy[r + nx + i] - 2.f * Myy[r + i]) + Myy[r - nx + i]) * g.fcf.inv_dy2;
+            }
+            const int y = (o + 2) * nx + i;
+            float dy = (yh[y] - wh) + (yl[y] - wl);
+            if (rprev) dy -= cmd;
+            const float p = on ? load + g.fcf.coef_mantle * dy : 0.f;
+            // the real row packed as complex pairs
+            reinterpret_cast<float*>(zb + (size_t)o * room)[i] = (((p + mx_xx) + 2.f * mxy) + my_yy) * ie;
+        }
+    }
+    __syncthreads();
+    tmark(g.trace);
+    switch (hh) {
+    case 128: engine_rows_fwd<RA, 128>(zb, tw); break;
+    case 192: engine_rows_fwd<RA, 192>(zb, tw); break;
+    case 256: engine_rows_fwd<RA, 256>(zb, tw); break;
+    }
+    __syncthreads();
+    tmark(g.trace);
+    // real split, column-major, the RA rows of a column in one segment
+    float2* ST = (float2*)g.ST;
+    const int pad = (line_points(hh, true) & (line_points(hh, true) - 1)) == 0 ? line_points(hh, true) : 16;
+    for (int e = tid; e < RA * (hh / 2); e += blockDim.x) {
+        const int o = e % RA, k = e / RA, j = j0 + o;
+        if (j >= ny) continue;
+        const float2* Z = zb + (size_t)o * room;
+        const float2 Zk = Z[k + k / pad];
+        if (k == 0) {
+            const float2 Zm = Z[hh / 2 + hh / 2 / pad];
+            ST[j] = make_float2(Zk.x + Zk.y, 0.f);
+            ST[(size_t)hh * ny + j] = make_float2(Zk.x - Zk.y, 0.f);
+            ST[(size_t)(hh / 2) * ny + j] = make_float2(Zm.x, -Zm.y);
+        } else {
+            const float2 Zc = Z[hh - k + (hh - k) / pad];
+            const float2 Ev = make_float2(0.5f * (Zk.x + Zc.x), 0.5f * (Zk.y - Zc.y));
+            const float2 O = make_float2(0.5f * (Zk.y + Zc.y), 0.5f * (Zc.x - Zk.x));
+            const float2 W = cmul(tw.rtw[k], O);
+            ST[(size_t)k * ny + j] = cadd(Ev, W);
+            ST[(size_t)(hh - k) * ny + j] = make_float2(Ev.x - W.x, W.y - Ev.y);
+        }
+    }
+    __syncthreads();
+    tmark(g.trace);
+}
+
+template <int CB, int N>
+__device__ __forceinline__ void engine_cols(const EngineArgs& g, int k0, unsigned char* smem, const EngTw<float>& tw)
+{
+    constexpr int E = LineShape<float, N>::E, TH = LineShape<float, N>::threads, ROOM = line_smem<float, N>();
+    constexpr int SY = CB * TH;
+    static_assert(SY % 32 == 0, "whole warps");
+    if ((int)threadIdx.x >= SY) return;   // whole warps
+    const int c = threadIdx.x % CB, t = threadIdx.x / CB, k = k0 + c;
+    const bool live = k <= g.p.h;
+    float2* b = reinterpret_cast<float2*>(smem) + (size_t)c * ROOM;
+    const float2* ST = (const float2*)g.ST + (size_t)k * N;
+    const float* mA = (const float*)g.mA;
+    const float* mB = (const float*)g.mB;
+    float2 v[E];
+    float fa[E];
+#pragma unroll
+    for (int m = 0; m < E; ++m) {
+        v[m] = live ? ST[t + TH * m] : make_float2(0.f, 0.f);
+        fa[m] = (live && g.even) ? __ldg(mA + (size_t)k * N + t + TH * m) : 0.f;
+    }
+    line_fft<float, N, -1, SY, true>(v, b, tw.col, t);
+    if (g.even) {
+#pragma unroll
+        for (int m = 0; m < E; ++m) v[m] = cscale(v[m], fa[m]);
+    } else {
+        line_sync<SY>();
+#pragma unroll
+        for (int m = 0; m < E; ++m) b[line_pad<E>(t + TH * m)] = v[m];
+        line_sync<SY>();
+#pragma unroll
+        for (int m = 0; m < E; ++m) {
+            if (!live) continue;
+            const int l = t + TH * m, lm = l == 0 ? 0 : N - l;
+            const size_t ia = (size_t)k * N + l, ib = (size_t)k * N + lm;
+            const float2 Fa = v[m], Fb = b[line_pad<E>(lm)];
+            const float H_kl = Fb.x - Fa.y, H_mkml = Fb.x + Fa.y, H_mkl = Fa.x + Fb.y, H_kml = Fa.x - Fb.y;
+            const float G_kl = __ldg(mA + ia) * H_kl, G_kml = __ldg(mA + ib) * H_kml;
+            const float G_mkl = __ldg(mB + ia) * H_mkl, G_mkml = __ldg(mB + ib) * H_mkml;
+            v[m] = make_float2(0.5f * (G_kml + G_mkl), 0.5f * (G_mkml - G_kl));
+        }
+    }
+    line_fft<float, N, +1, SY, true>(v, b, tw.col, t);
+    if (!live) return;
+    float2* S = (float2*)g.S;
+#pragma unroll
+    for (int m = 0; m < E; ++m) S[(size_t)(t + TH * m) * g.p.sp + k] = v[m];
+}
+
+template <int CB> __device__ void phase_b_lines(const EngineArgs& g, int k0, unsigned char* smem, const EngTw<float>& tw)
+{
+    switch (g.p.ny) {
+    case 256: engine_cols<CB, 256>(g, k0, smem, tw); break;
+    case 384: engine_cols<CB, 384>(g, k0, smem, tw); break;
+    case 512: engine_cols<CB, 512>(g, k0, smem, tw); break;
+    }
+    __syncthreads();
+    tmark(g.trace);
+}
+
+template <int RC, int H>
+__device__ __forceinline__ void engine_rows_inv(const EngineArgs& g, int j0, float* out, unsigned char* smem,
+                                                const EngTw<float>& tw)
+{
+    constexpr int E = LineShape<float, H>::E, TH = LineShape<float, H>::threads, ROOM = line_smem<float, H>();
+    const int line = threadIdx.x / TH, t = threadIdx.x % TH, j = j0 + line;
+    if (line >= RC) return;   // whole warps
+    const bool live = j < g.p.ny;
+    const float2* X = (const float2*)g.S + (size_t)(live ? j : 0) * g.p.sp;
+    float2 v[E];
+    line_rows_inv<float, H, 1, true>([&](int k) { return X[k]; }, v, reinterpret_cast<float2*>(smem) + (size_t)line * ROOM,
+                                     tw.row, tw.rtw, t, live);
+    if (!live) return;
+#pragma unroll
+    for (int m = 0; m < E; ++m)
+        *reinterpret_cast<float2*>(out + (size_t)j * g.p.nx + 2 * (t + TH * m)) = cscale(v[m], g.norm_scale_f);
+}
+
+template <int RC> __device__ void phase_c_lines(const EngineArgs& g, int j0, float* out, unsigned char* smem,
+                                                const EngTw<float>& tw)
+{
+    switch (g.p.h) {
+    case 128: engine_rows_inv<RC, 128>(g, j0, out, smem, tw); break;
+    case 192: engine_rows_inv<RC, 192>(g, j0, out, smem, tw); break;
+    case 256: engine_rows_inv<RC, 256>(g, j0, out, smem, tw); break;
     }
     __syncthreads();
     tmark(g.trace);
@@ -458,8 +745,8 @@ __device__ __forceinline__ bool grid_barrier(const EngineArgs& g, unsigned& targ
     return s_bar_ok != 0;
 }
 
-// FM: the block-FFT index mode, FFT_POW2 when both transform lengths are
-// powers of two, else FFT_ANY
+// FM: FFT_LINES where both transform lengths have a line phase, else FFT_ANY
+// (shared-memory stages)
 template <typename T, int RA, int FM>
 __global__ void __launch_bounds__(EngShape<RA>::threads, EngShape<RA>::per_sm) k_engine_rk4(EngineArgs g)
 {
@@ -485,7 +772,8 @@ __global__ void __launch_bounds__(EngShape<RA>::threads, EngShape<RA>::per_sm) k
     typedef typename vec2<T>::type C2;
     EngTw<T> tw;
     {
-        C2* tab = reinterpret_cast<C2*>(smem + engine_tab_off<T, RA>(nx, g.p.h, ny, g.CB));
+        C2* tab = reinterpret_cast<C2*>(smem + (FM == FFT_LINES ? lines_tab_off<RA>(nx, g.p.h, ny, g.CB)
+                                                                 : engine_tab_off<T, RA>(nx, g.p.h, ny, g.CB)));
         const C2* srow = etw<T>(g.p.row);
         const C2* scol = etw<T>(g.p.col);
         const C2* srtw = ertw<T>(g.p);
@@ -536,16 +824,24 @@ __global__ void __launch_bounds__(EngShape<RA>::threads, EngShape<RA>::per_sm) k
         const bool last = s_last != 0;
         TRACE();
         for (int stage = 0; stage < 4; ++stage) {
-            for (int it = blockIdx.x; it < na; it += gridDim.x)
-                phase_a<T, RA, FM>(g, it * RA, stage, s_sdf[stage], smem, tw);
+            for (int it = blockIdx.x; it < na; it += gridDim.x) {
+                if constexpr (FM == FFT_LINES) phase_a_lines<RA>(g, it * RA, stage, s_sdf[stage], smem, tw);
+                else phase_a<T, RA>(g, it * RA, stage, s_sdf[stage], smem, tw);
+            }
             TRACE();
             if (!grid_barrier(g, bar_target)) return;
             TRACE();
-            for (int it = blockIdx.x; it < nb; it += gridDim.x) phase_b<T, FM>(g, it * g.CB, g.CB, smem, tw);
+            for (int it = blockIdx.x; it < nb; it += gridDim.x) {
+                if constexpr (FM == FFT_LINES) phase_b_lines<EngShape<RA>::cb>(g, it * g.CB, smem, tw);
+                else phase_b<T>(g, it * g.CB, g.CB, smem, tw);
+            }
             TRACE();
             if (!grid_barrier(g, bar_target)) return;
             TRACE();
-            for (int it = blockIdx.x; it < nc; it += gridDim.x) phase_c<T, RC, FM>(g, it * RC, (T*)g.raw[stage], smem, tw);
+            for (int it = blockIdx.x; it < nc; it += gridDim.x) {
+                if constexpr (FM == FFT_LINES) phase_c_lines<RC>(g, it * RC, (float*)g.raw[stage], smem, tw);
+                else phase_c<T, RC>(g, it * RC, (T*)g.raw[stage], smem, tw);
+            }
             TRACE();
             if (!grid_barrier(g, bar_target)) return;
             TRACE();
@@ -655,6 +951,10 @@ template <typename T, int RA, int FM> int engine_config_shape(const Plan2D& p, i
     const int cb = EngShape<RA>::cb;
     *CB = cb;
     *smem = engine_smem_bytes<T, RA>(p, cb);
+    if (FM == FFT_LINES) {
+        if (p.nx > EngShape<RA>::threads) return 0;   // a thread owns a column
+        *smem = lines_tab_off<RA>(p.nx, p.h, p.ny, cb) + engine_tab_count<T>(p.h, p.ny) * 2 * sizeof(T) + 64;
+    }
     if (*smem > (size_t)optin) return 0;
     {
         // the limit is a property of the kernel, shared by every handle:
@@ -691,6 +991,8 @@ template <typename T, int RA, int FM> int engine_config_shape(const Plan2D& p, i
     return 1;
 }
 
+bool engine_has_lines(const Plan2D& p) { return engine_line_rows(p.h) && engine_line_cols(p.ny); }
+
 template <typename T> int engine_config(const Plan2D& p, int* grid, int* CB, size_t* smem, int* RA, int* P2)
 {
     // The plain FP64 form is FP64-throughput bound; it runs faster as the
@@ -707,13 +1009,13 @@ template <typename T> int engine_config(const Plan2D& p, int* grid, int* CB, siz
         const int v = atoi(ev);
         if (v == 2 || v == 4) ra = v;
     }
-    const int p2 = ((p.h & (p.h - 1)) == 0 && (p.ny & (p.ny - 1)) == 0) ? 1 : 0;
+    const int p2 = engine_has_lines(p) ? 1 : 0;
     *P2 = p2;
     if constexpr (sizeof(T) == 4) {
         auto shape = [&](int r) {
-            if (r == 4) return p2 ? engine_config_shape<T, 4, FFT_POW2>(p, nsm, optin, grid, CB, smem)
+            if (r == 4) return p2 ? engine_config_shape<T, 4, FFT_LINES>(p, nsm, optin, grid, CB, smem)
                                   : engine_config_shape<T, 4, FFT_ANY>(p, nsm, optin, grid, CB, smem);
-            return p2 ? engine_config_shape<T, 2, FFT_POW2>(p, nsm, optin, grid, CB, smem)
+            return p2 ? engine_config_shape<T, 2, FFT_LINES>(p, nsm, optin, grid, CB, smem)
                       : engine_config_shape<T, 2, FFT_ANY>(p, nsm, optin, grid, CB, smem);
         };
         if (ra == 4 && shape(4)) {
@@ -741,9 +1043,9 @@ template <typename T> cudaError_t engine_launch(const EngineArgs& g, int grid, s
         attr[0].val.cooperative = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        if (g.ra == 4) return g.p2 ? cudaLaunchKernelEx(&cfg, k_engine_rk4<T, 4, FFT_POW2>, g)
+        if (g.ra == 4) return g.p2 ? cudaLaunchKernelEx(&cfg, k_engine_rk4<T, 4, FFT_LINES>, g)
                                    : cudaLaunchKernelEx(&cfg, k_engine_rk4<T, 4, FFT_ANY>, g);
-        return g.p2 ? cudaLaunchKernelEx(&cfg, k_engine_rk4<T, 2, FFT_POW2>, g)
+        return g.p2 ? cudaLaunchKernelEx(&cfg, k_engine_rk4<T, 2, FFT_LINES>, g)
                     : cudaLaunchKernelEx(&cfg, k_engine_rk4<T, 2, FFT_ANY>, g);
     }
 }

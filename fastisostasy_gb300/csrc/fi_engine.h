@@ -34,7 +34,7 @@ struct EngineArgs {
     int nsteps;
     int CB;                          // spectrum columns per phase-B item
     int ra;                          // rows per stencil item (kernel shape: 2 or 4)
-    int p2;                          // both transform lengths are powers of two
+    int p2;                          // both transform lengths have a line phase
     double spy;
     double norm_scale;               // 1 / (nx*ny*1.) as the reference normalises
     float norm_scale_f;              // the same in float
@@ -53,6 +53,8 @@ struct EngineArgs {
 // memory, rows per stencil item and transform index mode of the engine for
 // this transform plan; 0 if it cannot run.
 template <typename T> int engine_config(const Plan2D& p, int* grid, int* CB, size_t* smem, int* RA, int* P2);
+// whether both transform lengths have the engine's line phases
+bool engine_has_lines(const Plan2D& p);
 template <typename T> cudaError_t engine_launch(const EngineArgs& g, int grid, size_t smem, cudaStream_t s);
 void split_hilo(const double* x, float* hi, float* lo, size_t n, cudaStream_t s);
 // split plus dxw = (hi - wrhi) + (lo - wrlo) (the kernel sequence's mixed RK4 stages)

@@ -163,19 +163,21 @@ template <typename T, typename C2, int SIGN> __device__ __forceinline__ void rdf
     c = mk2<T>(m.x + s1 * d.y, m.y - s1 * d.x);
 }
 
-// Barrier among the threads of a line: a warp barrier where a line never
-// leaves a warp (WARP), else the block's.
-template <bool WARP> __device__ __forceinline__ void line_sync()
+// Barrier among the threads of a line: 1 a warp barrier where a line never
+// leaves a warp, 0 the block's, n > 1 named barrier 1 of n threads (lines that
+// only those threads of a block work on).
+template <int SYNC> __device__ __forceinline__ void line_sync()
 {
-    if (WARP) __syncwarp();
-    else __syncthreads();
+    if (SYNC == 1) __syncwarp();
+    else if (SYNC == 0) __syncthreads();
+    else asm volatile("bar.sync 1, %0;" ::"n"(SYNC) : "memory");
 }
 
 // Stages from sub-transform size Ns on.  v: this thread's points t + T m;
 // sm: the line's shared memory; tw: exp(-2 pi i k / N).  Every thread of the
 // block calls it (threads without a line pass live = false: they only keep
 // the barriers).
-template <typename T, int N, int SIGN, bool WARP, bool TWSH, int Ns>
+template <typename T, int N, int SIGN, int WARP, bool TWSH, int Ns>
 __device__ __forceinline__ void line_stages(typename vec2<T>::type* v, typename vec2<T>::type* sm,
                                             const typename vec2<T>::type* __restrict__ tw, int t)
 {
@@ -230,7 +232,7 @@ __device__ __forceinline__ void line_stages(typename vec2<T>::type* v, typename 
 }
 
 // TWSH: the twiddles are in shared memory
-template <typename T, int N, int SIGN, bool WARP, bool TWSH = false>
+template <typename T, int N, int SIGN, int WARP, bool TWSH = false>
 __device__ __forceinline__ void line_fft(typename vec2<T>::type* v, typename vec2<T>::type* sm,
                                          const typename vec2<T>::type* __restrict__ tw, int t)
 {
@@ -246,7 +248,7 @@ __device__ __forceinline__ void line_fft(typename vec2<T>::type* v, typename vec
 // with E = (Z[k] + conj Z[H-k])/2 and W = w^k (Z[k] - conj Z[H-k])/(2i),
 // X[k] = E + W and X[H-k] = conj(E - W).
 // load(i): samples i and i + 1 of the row (i even); store(k, X[k]).
-template <typename T, int H, bool WARP, bool TWSH = false, typename Load, typename Store>
+template <typename T, int H, int WARP, bool TWSH = false, typename Load, typename Store>
 __device__ __forceinline__ void line_rows_fwd(Load load, Store store, typename vec2<T>::type* sm,
                                               const typename vec2<T>::type* __restrict__ tw,
                                               const typename vec2<T>::type* __restrict__ rtw, int t, bool live)
@@ -290,7 +292,7 @@ __device__ __forceinline__ void line_rows_fwd(Load load, Store store, typename v
 // packed real row: with s = X[k] + conj X[H-k] and u = conj(w^k) (X[k] -
 // conj X[H-k]), z[k] = s + i u and z[H-k] = conj(s) + i conj(u).
 // X(k): the spectrum value k.
-template <typename T, int H, bool WARP, bool TWSH = false, typename Load>
+template <typename T, int H, int WARP, bool TWSH = false, typename Load>
 __device__ __forceinline__ void line_rows_inv(Load X,
                                               typename vec2<T>::type* v, typename vec2<T>::type* sm,
                                               const typename vec2<T>::type* __restrict__ tw,
