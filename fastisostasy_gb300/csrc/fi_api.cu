@@ -312,6 +312,7 @@ struct fi_handle {
     double* weq_raw = nullptr;           // LV-ELRA convolution output
     void* conv_in = nullptr;             // convolution input (T)
     double *we_raw = nullptr, *dz_raw = nullptr, *corners = nullptr;
+    bool conv_ready = false;             // convolution plan, buffers and kernel spectra exist (ensure_conv)
     int* out_rows = nullptr;
     double* dH = nullptr;                // ice-grid thickness on the device
     double* dpack = nullptr;             // packed outputs
@@ -436,16 +437,40 @@ int upload_T(fi_handle* h, void* dst, const std::vector<double>& v)
     return upload(h, dst, v.data(), v.size() * sizeof(double));
 }
 
+// exp(-2 pi i t / n), t < n, rounded from long double.  The sine and cosine of
+// long doubles are software on some hosts (a microsecond each), so only an
+// eighth (a quarter, a half) of the circle is evaluated where n divides by it.
+void unit_roots(int n, double2* t64, float2* t32)
+{
+    const int parts = n % 8 == 0 ? 8 : n % 4 == 0 ? 4 : n % 2 == 0 ? 2 : 1;
+    const int last = parts == 1 ? n - 1 : n / parts;
+    std::vector<long double> c(last + 1), s(last + 1);
+    for (int t = 0; t <= last; ++t) {
+        const long double a = 2.0L * 3.14159265358979323846264338327950288L * (long double)t / (long double)n;
+        c[t] = cosl(a);
+        s[t] = sinl(a);
+    }
+    for (int t = 0; t < n; ++t) {
+        // reflect the angle into the evaluated part, undoing the reflections on its cosine and sine
+        int u = t;
+        bool neg_s = false, neg_c = false, swap = false;
+        if (parts >= 2 && 2 * u > n) { u = n - u; neg_s = true; }
+        if (parts >= 4 && 4 * u > n) { u = n / 2 - u; neg_c = true; }
+        if (parts >= 8 && 8 * u > n) { u = n / 4 - u; swap = true; }
+        long double co = swap ? s[u] : c[u], si = swap ? c[u] : s[u];
+        if (neg_c) co = -co;
+        if (neg_s) si = -si;
+        t64[t] = make_double2((double)co, (double)-si);
+        t32[t] = make_float2((float)co, (float)-si);
+    }
+}
+
 int make_len(fi_handle* h, int n, FftLen& L)
 {
     L.d = factorize(n);
     std::vector<double2> t64(n);
     std::vector<float2> t32(n);
-    for (int t = 0; t < n; ++t) {
-        long double a = -2.0L * 3.14159265358979323846264338327950288L * (long double)t / (long double)n;
-        t64[t] = make_double2((double)cosl(a), (double)sinl(a));
-        t32[t] = make_float2((float)cosl(a), (float)sinl(a));
-    }
+    unit_roots(n, t64.data(), t32.data());
     double2* d64;
     float2* d32;
     int rc;
@@ -465,13 +490,9 @@ int make_plan(fi_handle* h, int nx, int ny, Plan2D& P)
     P.sp = ((P.h + 1) + 7) / 8 * 8;
     int rc;
     if ((rc = make_len(h, P.h, P.row)) || (rc = make_len(h, ny, P.col))) return rc;
-    std::vector<double2> r64(P.h + 1);
-    std::vector<float2> r32(P.h + 1);
-    for (int k = 0; k <= P.h; ++k) {
-        long double a = -2.0L * 3.14159265358979323846264338327950288L * (long double)k / (long double)nx;
-        r64[k] = make_double2((double)cosl(a), (double)sinl(a));
-        r32[k] = make_float2((float)cosl(a), (float)sinl(a));
-    }
+    std::vector<double2> r64(nx);   // its first nx/2 + 1 entries
+    std::vector<float2> r32(nx);
+    unit_roots(nx, r64.data(), r32.data());
     double2* d64;
     float2* d32;
     if ((rc = dalloc(h, &d64, (P.h + 1) * sizeof(double2))) || (rc = dalloc(h, &d32, (P.h + 1) * sizeof(float2))))
@@ -573,10 +594,8 @@ void host_fields(fi_handle* h)
     // kappa, GE and GN cell by cell on the device (host loops as the fallback
     // for a failed launch are not kept: a device error is reported)
     h->kappa.assign(n, 0.0);
-    h->GE.assign(n, 0.0);
-    h->GN.assign(n, 0.0);
     h->init_rc = init_fields_device(h->nx, h->ny, h->dx, h->dy, PI_LIT, sp(1.e-12), sp(9.81), p.r_earth, p.m_earth,
-                                    kRn, kGe, h->kappa.data(), h->GE.data(), h->GN.data(), h->s);
+                                    kRn, kGe, h->kappa.data(), nullptr, nullptr, h->s);
     // He, D and (method 3) eta_eff, R on the device: src/fastisostasy.f90:240-443
     if (!h->init_rc) {
         RheoParams P;
@@ -869,6 +888,66 @@ template <typename T> void tune_conv_shapes(fi_handle* h)
     h->pconv_run.ct = best_ct;
     std::lock_guard<std::mutex> lk(mu);
     cache.push_back({key, Shape{best_rb, best_rt, best_cb, best_ct}});
+}
+
+// The page-locked staging buffer of fi_update.
+int ensure_pin(fi_handle* h)
+{
+    if (h->hpin) return FI_OK;
+    if (cudaMallocHost((void**)&h->hpin, h->hpin_elems * sizeof(double)) != cudaSuccess)
+        return fail(h, FI_E_OOM, "cudaMallocHost failed");
+    return FI_OK;
+}
+
+// The elastic and geoid Green's functions on the host.
+int ensure_green(fi_handle* h)
+{
+    if (!h->GE.empty() && !h->GN.empty()) return FI_OK;
+    std::vector<double> ge(h->n), gn(h->n), kap(h->n);
+    if (init_fields_device(h->nx, h->ny, h->dx, h->dy, PI_LIT, sp(1.e-12), sp(9.81), h->p.r_earth, h->p.m_earth, kRn, kGe,
+                           kap.data(), ge.data(), gn.data(), h->s))
+        return fail(h, FI_E_CUDA, "device init of the Green's functions failed");
+    if (h->GE.empty()) h->GE.swap(ge);
+    if (h->GN.empty()) h->GN.swap(gn);
+    return FI_OK;
+}
+
+// The convolution side of a domain: transform plan on the doubled grid,
+// buffers, kernel spectra.  Built with the domain where an update convolves
+// (elastic displacement, geoid, LV-ELRA), else only when fi_convolve or
+// fi_set_kernels asks for it: two FP64 transforms of the doubled grid and
+// three buffers of its size were half of a small domain's set-up.
+int ensure_conv(fi_handle* h)
+{
+    if (h->conv_ready) return FI_OK;
+    int rc;
+    if ((rc = ensure_green(h))) return rc;
+    const size_t n = h->n, c2 = 2 * tsz(h);
+    if ((rc = make_plan(h, h->Px, h->Py, h->pconv))) return rc;
+#define AL(ptr, bytes) if ((rc = dalloc(h, &(ptr), (bytes)))) return rc
+    AL(h->S2, (size_t)h->Py * h->pconv.sp * c2);
+    AL(h->KS[0], (size_t)h->Py * h->pconv.sp * c2);
+    AL(h->KS[1], (size_t)h->Py * h->pconv.sp * c2);
+    if (h->p.method == 2) { AL(h->KS[2], (size_t)h->Py * h->pconv.sp * c2); }
+    AL(h->conv_in, n * tsz(h));
+    AL(h->we_raw, n * 8); AL(h->dz_raw, n * 8); AL(h->corners, 12 * sizeof(double));
+    AL(h->out_rows, (h->ny + 2) * sizeof(int));
+#undef AL
+    std::vector<int> rows(h->ny + 2);
+    for (int j = 0; j < h->ny; ++j) rows[j] = h->ny / 2 - 1 + j;   // crop, src/convolutions.f90:29-55
+    rows[h->ny] = 0;
+    rows[h->ny + 1] = 2 * h->ny - 2;
+    if ((rc = upload(h, h->out_rows, rows.data(), rows.size() * sizeof(int)))) return rc;
+    h->pconv_run = h->pconv;
+    const char* nt = getenv("FI_NO_TUNE");
+    if ((h->p.include_elastic || h->p.heterogeneous_ssh) && !(nt && nt[0] == '1')) {
+        if (mixed(h)) tune_conv_shapes<float>(h);
+        else tune_conv_shapes<double>(h);
+    }
+    if ((rc = kernel_spectrum(h, h->GE, 0)) || (rc = kernel_spectrum(h, h->GN, 1))) return rc;
+    if (h->p.method == 2 && (rc = kernel_spectrum(h, h->GV, 2))) return rc;
+    h->conv_ready = true;
+    return FI_OK;
 }
 
 // ---- device pipelines ------------------------------------------------------
@@ -1491,6 +1570,9 @@ int read_status(fi_handle* h, Ctl* hc)
 }  // namespace
 
 // ============================================================================
+int fi_create_handle(const fi_params* pin, int nx_ice, int ny_ice, double dx, double dy, const double* K_or_null,
+                     bool staging, fi_handle** out);
+
 extern "C" {
 
 int fi_version(void) { return 1; }
@@ -1596,6 +1678,17 @@ int fi_padded_dims(const fi_params* p, int nx_ice, int ny_ice, double dx, double
 
 int fi_create(const fi_params* pin, int nx_ice, int ny_ice, double dx, double dy, const double* K_or_null,
               fi_handle** out)
+{
+    return fi_create_handle(pin, nx_ice, ny_ice, dx, dy, K_or_null, true, out);
+}
+
+}   // extern "C"
+
+// staging: with the page-locked staging buffer of fi_update (the solve server
+// drives its handles without it: allocating and freeing page-locked memory
+// took 0.3 ms of each request and held up the device's other work)
+int fi_create_handle(const fi_params* pin, int nx_ice, int ny_ice, double dx, double dy, const double* K_or_null,
+                     bool staging, fi_handle** out)
 {
     ApiRange nr("fi_create");
     if (!pin || !out) return FI_E_ARG;
@@ -1710,32 +1803,15 @@ int fi_create(const fi_params* pin, int nx_ice, int ny_ice, double dx, double dy
     // convolution plan: any even size >= 2n-1 gives the reference's linear convolution
     h->Px = nice_even_at_least(2 * h->nx - 1);
     h->Py = nice_even_at_least(2 * h->ny - 1);
-    if (h->Px == 2 * h->nx - 2 + 2 && false) {}
-    if ((rc = make_plan(h, h->Px, h->Py, h->pconv))) return rc;
-    AL(h->S2, (size_t)h->Py * h->pconv.sp * c2);
-    AL(h->KS[0], (size_t)h->Py * h->pconv.sp * c2);
-    AL(h->KS[1], (size_t)h->Py * h->pconv.sp * c2);
-    if (p.method == 2) { AL(h->KS[2], (size_t)h->Py * h->pconv.sp * c2); }
-    AL(h->conv_in, nT);
-    AL(h->we_raw, n * 8); AL(h->dz_raw, n * 8); AL(h->corners, 12 * sizeof(double));
     if (p.method != 3) {
         AL(h->weq, n * 8);
         if (p.method == 2) { AL(h->weq_raw, n * 8); }
-    }
-    AL(h->out_rows, (h->ny + 2) * sizeof(int));
-    {
-        std::vector<int> rows(h->ny + 2);
-        for (int j = 0; j < h->ny; ++j) rows[j] = h->ny / 2 - 1 + j;   // crop, src/convolutions.f90:29-55
-        rows[h->ny] = 0;
-        rows[h->ny + 1] = 2 * h->ny - 2;
-        if ((rc = upload(h, h->out_rows, rows.data(), rows.size() * sizeof(int)))) return rc;
     }
     AL(h->dH, nice_ * 8);
     const int nout = 11;
     AL(h->dpack, nice_ * nout * 8);
     h->hpin_elems = nice_ * nout;
-    if (cudaMallocHost((void**)&h->hpin, h->hpin_elems * sizeof(double)) != cudaSuccess)
-        return fail(h, FI_E_OOM, "cudaMallocHost failed");
+    if (staging && (rc = ensure_pin(h))) return rc;
     AL(h->gsrc, 8 * sizeof(double*));
     AL(h->gmsrc, 3 * sizeof(uint8_t*));
     {
@@ -1826,18 +1902,12 @@ int fi_create(const fi_params* pin, int nx_ice, int ny_ice, double dx, double dy
 #undef AL2
     }
     if ((rc = upload_static(h))) return rc;
-    h->pconv_run = h->pconv;
-    if ((p.include_elastic || p.heterogeneous_ssh) && !(getenv("FI_NO_TUNE") && getenv("FI_NO_TUNE")[0] == '1')) {
-        if (mixed(h)) tune_conv_shapes<float>(h);
-        else tune_conv_shapes<double>(h);
-    }
     if (p.method == 3 && !h->engine_ok && !h->clu_ok && !(getenv("FI_NO_TUNE") && getenv("FI_NO_TUNE")[0] == '1')) {
         if (mixed(h)) tune_rhs_shapes<float>(h);
         else tune_rhs_shapes<double>(h);
         CK(cudaGetLastError());
     }
-    if ((rc = kernel_spectrum(h, h->GE, 0)) || (rc = kernel_spectrum(h, h->GN, 1))) return rc;
-    if (p.method == 2 && (rc = kernel_spectrum(h, h->GV, 2))) return rc;
+    if ((p.include_elastic || p.heterogeneous_ssh || p.method == 2) && (rc = ensure_conv(h))) return rc;
     // zero_init_state (src/fastisostasy.f90:505-548): z_bed background 1e6
     {
         std::vector<double> bg(n, 1e6);
@@ -1853,6 +1923,8 @@ int fi_create(const fi_params* pin, int nx_ice, int ny_ice, double dx, double dy
     CK(cudaStreamSynchronize(h->s));
     return FI_OK;
 }
+
+extern "C" {
 
 int fi_destroy(fi_handle* h)
 {
@@ -2002,6 +2074,7 @@ int fi_set_kernels(fi_handle* h, const double* GE, const double* GN)
 {
     if (!h) return FI_E_ARG;
     int rc;
+    if ((rc = ensure_conv(h))) return rc;
     if (GE) { h->GE.assign(GE, GE + h->n); if ((rc = kernel_spectrum(h, h->GE, 0))) return rc; }
     if (GN) { h->GN.assign(GN, GN + h->n); if ((rc = kernel_spectrum(h, h->GN, 1))) return rc; }
     return FI_OK;
@@ -2145,6 +2218,7 @@ int fi_update(fi_handle* h, const double* H_ice, double time, fi_bsl* bsl, fi_ou
     if (!h->state_ready) return fail(h, FI_E_STATE, "fi_update before fi_init_state");
     const size_t ni = (size_t)h->nx_ice * h->ny_ice;
     int rc;
+    if ((rc = ensure_pin(h))) return rc;
     auto pinned = [&](const void* ptr) {
         if (!ptr) return false;
         for (const auto& e : h->pin_seen)
@@ -2322,8 +2396,11 @@ int fi_get_field(fi_handle* h, int which, double* out)
     case FI_FIELD_ETA_EFF: hv = &h->eta_eff; break;
     case FI_FIELD_R: hv = &h->R; break;
     case FI_FIELD_MASKACTIVE: msk = d.mactive; break;
-    case FI_FIELD_GE: hv = &h->GE; break;
-    case FI_FIELD_GN: hv = &h->GN; break;
+    case FI_FIELD_GE:
+    case FI_FIELD_GN:
+        if (const int rc = ensure_green(h)) return rc;
+        hv = which == FI_FIELD_GE ? &h->GE : &h->GN;
+        break;
     default: return fail(h, FI_E_ARG, "unknown field %d", which);
     }
     if (hv) { memcpy(out, hv->data(), n * 8); return FI_OK; }
@@ -2395,7 +2472,7 @@ int fi_convolve(fi_handle* h, int kernel, const double* in, double* out)
     if (!h || !in || !out || kernel < 0 || kernel > 1) return FI_E_ARG;
     const size_t n = h->n;
     int rc;
-    if ((rc = upload(h, h->we_raw, in, n * 8))) return rc;
+    if ((rc = ensure_conv(h)) || (rc = upload(h, h->we_raw, in, n * 8))) return rc;
     if (mixed(h)) {
         cast_from_double<float>((float*)h->conv_in, h->we_raw, n, h->s);
         conv<float>(h, kernel, h->dz_raw, h->corners);

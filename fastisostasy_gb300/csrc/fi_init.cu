@@ -45,6 +45,7 @@ __global__ void k_init_fields(double* __restrict__ kappa, double* __restrict__ G
         const double q = (j <= jc) ? mu_y * (j - 1) : mu_y * (ny - j + 1);
         // products and sums unfused (no FMA contraction), as on the host
         kappa[e] = sqrt(__dadd_rn(__dmul_rn(pp, pp), __dmul_rn(q, q)));   // x**0.5, correctly rounded
+        if (!GE) continue;
         const double x = (i - 1 - mx) * dx, y = (j - 1 - mx) * dx;
         const double r = sqrt(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)));
         GE[e] = __dmul_rn(__dmul_rn(ge_value_dev(r), ge_scale), __dmul_rn(dx, dx)) / __dmul_rn(g_lit, (r > dx ? r : dx));
@@ -61,21 +62,22 @@ int init_fields_device(int nx, int ny, double dx, double dy, double pi_lit, doub
     const size_t n = (size_t)nx * ny;
     double* buf = nullptr;
     // stream-ordered: set-up of one handle never waits for other handles' work
-    if (cudaMallocAsync((void**)&buf, 3 * n * sizeof(double), s) != cudaSuccess) return 1;
+    const bool green = GE && GN;
+    if (cudaMallocAsync((void**)&buf, (green ? 3 : 1) * n * sizeof(double), s) != cudaSuccess) return 1;
     int rc = 0;
-    if (cudaMemcpyToSymbolAsync(c_ge_rn, ge_rn, 42 * sizeof(float), 0, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-        cudaMemcpyToSymbolAsync(c_ge_v, ge_v, 42 * sizeof(float), 0, cudaMemcpyHostToDevice, s) != cudaSuccess)
+    if (green && (cudaMemcpyToSymbolAsync(c_ge_rn, ge_rn, 42 * sizeof(float), 0, cudaMemcpyHostToDevice, s) != cudaSuccess ||
+        cudaMemcpyToSymbolAsync(c_ge_v, ge_v, 42 * sizeof(float), 0, cudaMemcpyHostToDevice, s) != cudaSuccess))
         rc = 1;
     if (!rc) {
         const double mu_x = 2.0 * pi_lit / ((nx - 1) * dx), mu_y = 2.0 * pi_lit / ((ny - 1) * dy);
         int blocks = (int)((n + 255) / 256);
         if (blocks > 152 * 16) blocks = 152 * 16;
-        k_init_fields<<<blocks, 256, 0, s>>>(buf, buf + n, buf + 2 * n, nx, ny, dx, mu_x, mu_y, ge_scale, g_lit,
+        k_init_fields<<<blocks, 256, 0, s>>>(buf, green ? buf + n : nullptr, green ? buf + 2 * n : nullptr, nx, ny, dx, mu_x, mu_y, ge_scale, g_lit,
                                              r_earth, m_earth);
         if (cudaGetLastError() != cudaSuccess ||
             cudaMemcpyAsync(kappa, buf, n * sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaMemcpyAsync(GE, buf + n, n * sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaMemcpyAsync(GN, buf + 2 * n, n * sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+            (green && (cudaMemcpyAsync(GE, buf + n, n * sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+                       cudaMemcpyAsync(GN, buf + 2 * n, n * sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess)) ||
             cudaStreamSynchronize(s) != cudaSuccess)
             rc = 1;
     }

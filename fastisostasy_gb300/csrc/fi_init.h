@@ -7,7 +7,8 @@ namespace fi {
 
 // kappa (calc_kappa), GE and GN (elastic and geoid Green's functions) of a
 // padded (nx, ny) domain into host arrays; the 42-entry elastic table as the
-// single-precision values of the reference.  Returns 0 on success.
+// single-precision values of the reference.  GE and GN may both be null (not
+// computed then).  Returns 0 on success.
 int init_fields_device(int nx, int ny, double dx, double dy, double pi_lit, double ge_scale, double g_lit,
                        double r_earth, double m_earth, const float* ge_rn, const float* ge_v, double* kappa,
                        double* GE, double* GN, cudaStream_t s);

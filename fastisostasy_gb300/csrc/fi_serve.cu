@@ -38,6 +38,10 @@
 
 #include "../../include/fi_gpu.h"
 
+// fi_create without fi_update's staging buffer (fi_api.cu)
+int fi_create_handle(const fi_params* pin, int nx_ice, int ny_ice, double dx, double dy, const double* K_or_null,
+                     bool staging, fi_handle** out);
+
 namespace {
 
 constexpr int kDepth = 2;     // updates queued ahead per running request
@@ -135,7 +139,7 @@ int start(fi_server* s, Req* r)
 {
     size_t free0 = 0, total = 0;
     cudaMemGetInfo(&free0, &total);
-    int rc = fi_create(&r->p, r->nxi, r->nyi, r->dx, r->dy, nullptr, &r->h);
+    int rc = fi_create_handle(&r->p, r->nxi, r->nyi, r->dx, r->dy, nullptr, false, &r->h);
     if (rc) return rc;
     rc = fi_set_fields(r->h, r->D.empty() ? nullptr : r->D.data(), r->eta.empty() ? nullptr : r->eta.data(),
                        r->R.empty() ? nullptr : r->R.data(), r->mask.empty() ? nullptr : r->mask.data());

@@ -77,3 +77,16 @@ def test_convolution_on_lines(nx, ny, precision):
     for k, G in ((0, dom.field("GE")), (1, dom.field("GN"))):
         assert rel(dom.convolve(k, x), linear_convolution(G, x)) <= TOL[precision]
     dom.close()
+
+
+def test_convolution_of_a_domain_that_does_not_convolve():
+    """Green's functions and spectra made on demand equal those of a domain whose updates use them."""
+    got = []
+    for name in ("test2c", "test1d"):
+        dom, p = _domain(name, 48, 48, 0)
+        assert bool(p["include_elastic"] or p["heterogeneous_ssh"]) == (name == "test2c")
+        x = np.random.default_rng(1).standard_normal((48, 48)) * 1e7
+        got.append([dom.convolve(0, x), dom.convolve(1, x), dom.field("GE"), dom.field("GN")])
+        dom.close()
+    for a, b in zip(*got):
+        assert rel(a, b) <= 1e-13
