@@ -1011,7 +1011,7 @@ void rhs_stage64(fi_handle* h, const double* rprev, double a, double* raw_out)
 }
 
 // One RHS of the mixed true-stage Tsit5 at a stage state given as a float
-// pair with its dxw (rhs with the column-strip stencil in stage mode).
+// pair with its dxw (the tile stencil in stage mode).
 void rhs_tpair(fi_handle* h, const float* hi, const float* lo, const float* dw, float* raw_out, const int* gate)
 {
     typedef vec2<float>::type C2;
@@ -2439,7 +2439,7 @@ int fi_lvelva(fi_handle* h, const double* w, const double* canom_full, double* d
     if (mixed(h)) {
         q0_from_cf<float>((float*)h->q0, tmp, h->d.mactive, h->p.g, n, h->s);
         if (h->p.method == 3 && h->fc.ixm == nullptr) {
-            // uniform spacing: w as a float pair through the column-strip
+            // uniform spacing: w as a float pair through the tile
             // stencil, as the mixed reference-compatible Tsit5 evaluates it
             float* pair;
             if ((rc = dalloc(h, &pair, 2 * n * sizeof(float)))) return rc;
@@ -2596,13 +2596,13 @@ struct fi_batch {
     bool true_stages = false;            // members run Tsit5 with true stages (stage_mode 1)
     std::vector<BMember> hM;             // host copy of the member descriptors
     std::vector<int> hoff;               // host copy of the virtual-block offsets (4 x (nm + 1))
-    int shape[4] = {0, 0, 16, 8};        // rows / columns per transform block (0: single-domain shape), strip rows, waves
+    int shape[4] = {0, 0, 16, 8};        // rows / columns per transform block (0: single-domain shape), tile rows, waves
 };
 
 // Per-member transform and stencil shapes, the virtual-block offsets and
 // the resident grids of the batched launches; uploads the descriptors.
 // RB / CB <= 0: the single-domain shapes.
-int batch_shape(fi_batch* b, int RB, int CB, int fseg, int waves)
+int batch_shape(fi_batch* b, int RB, int CB, int waves)
 {
     const int n = b->nl();
     if (n == 0) return 0;
@@ -2635,9 +2635,11 @@ int batch_shape(fi_batch* b, int RB, int CB, int fseg, int waves)
         BMember& m = b->hM[i];
         if (m.lines & 1) m.RB = b->rows_threads / rhs_line_threads(m.p.h, b->mixed);
         if (m.lines & 2) m.CB = b->cols_threads / rhs_line_threads(m.p.ny, b->mixed);
-        m.fseg = fseg;
-        const int fblk = b->mixed ? (!b->true_stages || m.yhi ? batch_flexure_blocks(m.p.nx, m.p.ny, m.fseg)
-                                                              : m.fgx * ((m.p.ny + 7) / 8))
+        // stencil tiles: the FP64 state of true stages without the pairs has its own
+        const bool pair = b->mixed && (!b->true_stages || m.yhi);
+        m.fgx = pair ? (m.p.nx + 63) / 64 : (m.p.nx + 31) / 32;
+        const int fblk = pair ? batch_flexure_tiles32(m.p.nx, m.p.ny)
+                       : b->mixed ? m.fgx * ((m.p.ny + 7) / 8)
                                   : batch_flexure_tiles64(m.p.nx, m.p.ny);
         const int rblk = (m.p.ny + m.RB - 1) / m.RB;
         const int cblk = (m.p.h + 1 + m.CB - 1) / m.CB;
@@ -2679,7 +2681,6 @@ int batch_shape(fi_batch* b, int RB, int CB, int fseg, int waves)
     }
     b->shape[0] = RB;
     b->shape[1] = CB;
-    b->shape[2] = fseg;
     b->shape[3] = waves;
     return 0;
 }
@@ -2928,7 +2929,6 @@ int fi_batch_create(fi_handle* const* hs, int n, fi_batch** out)
             m.wrhi = h->wrefhi; m.wrlo = h->wreflo;
         }
         m.even = h->even;
-        m.fgx = (m.p.nx + 31) / 32;
         m.red_nblk = ts_grid(h->n);
         m.d = h->d;
         m.atol = h->p.atol;
@@ -2962,7 +2962,7 @@ int fi_batch_create(fi_handle* const* hs, int n, fi_batch** out)
     if (const char* e = getenv("FI_BATCH_RB")) { const int v = atoi(e); if (v >= 1 && v <= 16) RB = v; }
     if (const char* e = getenv("FI_BATCH_CB")) { const int v = atoi(e); if (v >= 1 && v <= 16) CB = v; }
     if (const char* e = getenv("FI_BATCH_WAVES")) waves = atoi(e);
-    if (batch_shape(b, RB, CB, 16, waves)) {
+    if (batch_shape(b, RB, CB, waves)) {
         batch_free(b);
         return FI_E_CUDA;
     }
@@ -3041,19 +3041,18 @@ int fi_batch_autotune(fi_batch* b, int32_t* chosen4)
     auto time_of = [&](int part) { return b->mixed ? batch_time_rhs<float>(b, part, 3) : batch_time_rhs<double>(b, part, 3); };
     int sh[4] = {b->shape[0], b->shape[1], b->shape[2], b->shape[3]};
     auto try_shape = [&](const int* c, int part, float* t) -> int {
-        const int rc = batch_shape(b, c[0], c[1], c[2], c[3]);
+        const int rc = batch_shape(b, c[0], c[1], c[3]);
         if (rc == 2) { *t = 1e30f; return 0; }   // does not fit
         if (rc || batch_all_lists(b)) return 1;
         *t = time_of(part);
         return *t < 0 ? 1 : 0;
     };
-    // coordinate descent: stencil rows per task, transform rows, transform
-    // columns, then waves over the whole RHS
-    const int seg_c[3] = {8, 16, 32}, rb_c[4] = {2, 4, 8, 16}, cb_c[5] = {1, 2, 4, 8, 16}, wv_c[4] = {2, 4, 8, 16};
+    // coordinate descent: transform rows, transform columns, then waves over
+    // the whole RHS
+    const int rb_c[4] = {2, 4, 8, 16}, cb_c[5] = {1, 2, 4, 8, 16}, wv_c[4] = {2, 4, 8, 16};
     struct Axis { int idx, part, nc; const int* c; };
-    const Axis axes[4] = {{2, 1, 3, seg_c}, {0, 2, 4, rb_c}, {1, 3, 5, cb_c}, {3, 0, 4, wv_c}};
+    const Axis axes[3] = {{0, 2, 4, rb_c}, {1, 3, 5, cb_c}, {3, 0, 4, wv_c}};
     for (const Axis& ax : axes) {
-        if (ax.idx == 2 && (!b->mixed || b->true_stages)) continue;   // column strips: mixed reference stages only
         int best_v = sh[ax.idx];
         float best_t = 1e30f;
         for (int k = 0; k < ax.nc; ++k) {
@@ -3065,7 +3064,7 @@ int fi_batch_autotune(fi_batch* b, int32_t* chosen4)
         }
         sh[ax.idx] = best_v;
     }
-    if (batch_shape(b, sh[0], sh[1], sh[2], sh[3])) return FI_E_CUDA;
+    if (batch_shape(b, sh[0], sh[1], sh[3])) return FI_E_CUDA;
     if (cudaStreamSynchronize(b->s) != cudaSuccess) return FI_E_CUDA;
     if (chosen4)
         for (int k = 0; k < 4; ++k) chosen4[k] = sh[k];

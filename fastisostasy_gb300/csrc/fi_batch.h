@@ -44,7 +44,6 @@ struct BMember {
     int RB, CB;               // rows per row block, columns per column block
     int lines;                // transforms on register lines: bit 0 rows, bit 1 columns
     int fgx;                  // flexure blocks along x (tiles)
-    int fseg;                 // output rows per flexure warp task (mixed column strips)
     int red_nblk;             // blocks of the reduction kernels
     double norm_scale;        // 1 / (nx*ny*1.) as the reference normalises
     float norm_scale_f;       // the same in float: no FP64 division per thread
@@ -81,8 +80,8 @@ inline BList blist(const int* base, int nm, int kind)
     return L;
 }
 
-// Virtual blocks of the mixed batched flexure (8 column-strip warp tasks each).
-int batch_flexure_blocks(int nx, int ny, int seg);
+// Virtual blocks of the mixed batched flexure (64 x 16 tiles of the pair).
+int batch_flexure_tiles32(int nx, int ny);
 // ... and of the FP64 one (32 x 16 tiles).
 int batch_flexure_tiles64(int nx, int ny);
 

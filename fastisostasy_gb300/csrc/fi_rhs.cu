@@ -3,10 +3,12 @@
 // src/convolutions.f90:59-91).
 //
 // RHS = four kernels:
-//   k_flexure      finite-difference flexure moments and load -> f      (one pass over the grid)
-//   k_rows_fwd     real FFT of every row of f -> half spectrum S
-//   k_cols_hartley column FFT, multiply by 1/(kappa R) in the Hartley basis, inverse column FFT
-//   k_rows_inv     inverse real FFT of the rows, scaled by 1/(nx*ny) -> raw
+//   k_flexure*     finite-difference flexure moments and load -> f (one pass over the grid)
+//   rows_fwd       real FFT of every row of f -> half spectrum S
+//   cols_hartley   column FFT, multiply by 1/(kappa R) in the Hartley basis, inverse column FFT
+//   rows_inv       inverse real FFT of the rows, scaled by 1/(nx*ny) -> raw
+// The transforms of lengths that have a register line are in fi_lines*.cu;
+// the shared-memory forms here take every other length.
 // The corner boundary condition and the sec_per_year factor are applied by
 // whichever kernel consumes raw (it reads the four corner values).
 //
@@ -194,20 +196,12 @@ k_flexure(const double* __restrict__ y, const double* __restrict__ wref, const T
 // mantle term y - w_ref.  Central and second differences are rebuilt
 // exactly from them: y[i+1]-y[i-1] = dX[i]+dX[i-1],
 // y[i+1]-2y[i]+y[i-1] = dX[i]-dX[i-1].
-// HILO: the state arrives as a float pair y = hi + lo (whi, wlo) instead of
-// doubles, and the first differences are (hi[i+1]-hi[i]) + (lo[i+1]-lo[i]),
-// all in float (no mantle term in this form).
-template <bool HILO>
 __device__ __forceinline__ void flexure_f32_body(const double* __restrict__ y, const double* __restrict__ wref,
                                                  const float* __restrict__ q0, const uint8_t* __restrict__ mask,
                                                  const float* __restrict__ D, const float* __restrict__ inv2eta,
-                                                 float* __restrict__ f, int nx, int ny, FlexCoefF c, int bx, int by,
-                                                 const float* __restrict__ whi = nullptr,
-                                                 const float* __restrict__ wlo = nullptr)
+                                                 float* __restrict__ f, int nx, int ny, FlexCoefF c, int bx, int by)
 {
-    __shared__ double ys[HILO ? 1 : RY][HILO ? 1 : RX];
-    __shared__ float yh[HILO ? RY : 1][HILO ? RX : 1];
-    __shared__ float yl[HILO ? RY : 1][HILO ? RX : 1];
+    __shared__ double ys[RY][RX];
     __shared__ float dX[RY][RX];
     __shared__ float dY[RY][RX];
     __shared__ float Wx[RY][RX];
@@ -231,23 +225,13 @@ __device__ __forceinline__ void flexure_f32_body(const double* __restrict__ y, c
             const int gi = i0 + lx, gj = j0 + ly;
             const bool in = gi >= 0 && gi < nx && gj >= 0 && gj < ny;
             Ds[ly][lx] = in ? D[(size_t)gj * nx + gi] : 0.f;
-            if constexpr (HILO) {
-                yh[ly][lx] = in ? whi[(size_t)gj * nx + gi] : 0.f;
-                yl[ly][lx] = in ? wlo[(size_t)gj * nx + gi] : 0.f;
-            } else {
-                ys[ly][lx] = in ? y[(size_t)gj * nx + gi] : 0.0;
-            }
+            ys[ly][lx] = in ? y[(size_t)gj * nx + gi] : 0.0;
         }
     __syncthreads();
     for (int ly = ty; ly < RY; ly += TY)
         for (int lx = tx; lx < RX; lx += TX) {
-            if constexpr (HILO) {
-                if (lx < RX - 1) dX[ly][lx] = (yh[ly][lx + 1] - yh[ly][lx]) + (yl[ly][lx + 1] - yl[ly][lx]);
-                if (ly < RY - 1) dY[ly][lx] = (yh[ly + 1][lx] - yh[ly][lx]) + (yl[ly + 1][lx] - yl[ly][lx]);
-            } else {
-                if (lx < RX - 1) dX[ly][lx] = (float)(ys[ly][lx + 1] - ys[ly][lx]);
-                if (ly < RY - 1) dY[ly][lx] = (float)(ys[ly + 1][lx] - ys[ly][lx]);
-            }
+            if (lx < RX - 1) dX[ly][lx] = (float)(ys[ly][lx + 1] - ys[ly][lx]);
+            if (ly < RY - 1) dY[ly][lx] = (float)(ys[ly + 1][lx] - ys[ly][lx]);
         }
     __syncthreads();
     for (int ly = ty; ly < RY; ly += TY)
@@ -309,23 +293,22 @@ __device__ __forceinline__ void flexure_f32_body(const double* __restrict__ y, c
     float p = 0.f;
     if (own_m) {
         p = own_q;
-        if constexpr (!HILO) {
-            if (wref) p += c.coef_mantle * (float)(ys[ly][lx] - wref[e]);
-        }
+        if (wref) p += c.coef_mantle * (float)(ys[ly][lx] - wref[e]);
     }
     f[e] = (((p + mx_xx) + 2.f * mxy_xy) + my_yy) * own_ie;
 }
 
 // ---------------------------------------------------------------------------
-// Flexure by column strips (mixed form, uniform spacing, the state as a
-// float pair).  One warp task = SW output columns [SW g, SW g + SW) by `seg`
-// output rows [seg s, seg s + seg): lane l holds column SW g - 2 + l and
-// walks down the rows with the vertical stencil window in registers, taking
-// x-neighbours by warp shuffles, so there is no shared memory and no block
-// barrier.  Moments of row m are formed when input row m + 2 has been read,
-// f of row o when moments of row o + 2 exist (the one-sided formulas of the
-// first and last rows reach two rows further than the interior ones); the
-// arithmetic is that of flexure_f32_body<true>, term by term.
+// Flexure by column strips (mixed form, uniform spacing, the FP64 state: its
+// first differences taken in double and rounded, as in flexure_f32_body, and
+// with wref the mantle term coef_mantle (y - wref) at masked cells).  One
+// warp task = SW output columns [SW g, SW g + SW) by `seg` output rows
+// [seg s, seg s + seg): lane l holds column SW g - 2 + l and walks down the
+// rows with the vertical stencil window in registers, taking x-neighbours by
+// warp shuffles, so there is no shared memory and no block barrier.  Moments
+// of row m are formed when input row m + 2 has been read, f of row o when
+// moments of row o + 2 exist (the one-sided formulas of the first and last
+// rows reach two rows further than the interior ones).
 // ---------------------------------------------------------------------------
 constexpr int SW = 28;                     // output columns per warp task
 
@@ -334,30 +317,12 @@ __device__ __forceinline__ int strip_tasks(int nx, int ny, int seg)
     return ((nx + SW - 1) / SW) * ((ny + seg - 1) / seg);
 }
 
-// PAIR: the state as a float pair (whi + wlo), no mantle term; else the
-// FP64 state y, its first differences taken in double and rounded (as
-// flexure_f32_body<false>), and with wref the mantle term
-// coef_mantle (y - wref) at masked cells.
-// STG (with PAIR): an RK stage state y = x + sdf (rprev - cm) formed on the
-// fly from the pair x = whi + wlo and the previous stage's raw RHS rprev
-// (null at the first stage), with the mantle term
-// coef_mantle (dxw + sdf (rprev - cm)) at masked cells, where
-// dxw = (whi - w_ref,hi) + (wlo - w_ref,lo) is kept per cell beside the pair:
-// the arithmetic of the step engine's phase A, term by term, and no FP64
-// instruction.  (Loading every field one row ahead, as the state already is,
-// takes 78 registers instead of 64 and ran 35 % slower at 2048^2: the walk
-// is bound by warps in flight, not by the distance of each warp's loads.)
-template <bool PAIR, bool STG = false>
-__device__ __forceinline__ void flexure_strip(const float* __restrict__ whi, const float* __restrict__ wlo,
+__device__ __forceinline__ void flexure_strip(const double* __restrict__ y, const double* __restrict__ wref,
                                               const float* __restrict__ q0, const uint8_t* __restrict__ mask,
                                               const float* __restrict__ D, const float* __restrict__ inv2eta,
                                               float* __restrict__ f, int nx, int ny, const FlexCoefF& c, int seg,
-                                              int task, const double* __restrict__ y = nullptr,
-                                              const double* __restrict__ wref = nullptr,
-                                              const float* __restrict__ rprev = nullptr, float sdf = 0.f,
-                                              float cmdf = 0.f, const float* __restrict__ dxw = nullptr)
+                                              int task)
 {
-    static_assert(PAIR || !STG, "stage states are formed from the float pair");
     const unsigned FULL = 0xffffffffu;
     const int ncg = (nx + SW - 1) / SW;
     const int g = task % ncg, sg = task / ncg;
@@ -369,9 +334,7 @@ __device__ __forceinline__ void flexure_strip(const float* __restrict__ whi, con
     const bool edge = g == 0 || g == ncg - 1;   // warp-uniform: a lane may sit on x = 0 or x = nx - 1
     const int o0 = sg * seg, o1 = min(o0 + seg, ny);
     const int cc = cin ? col : 0;
-    float hp = 0.f, lp = 0.f;                           // pair of row r - 1
-    float rp = 0.f;                                     // rprev of row r - 1 (STG)
-    double yp = 0.0;                                    // FP64 state of row r - 1 (!PAIR)
+    double yp = 0.0;                                    // state of row r - 1
     float Wx1 = 0.f, Wx2 = 0.f, Wx3 = 0.f;              // Wx of rows r-1, r-2, r-3
     float wxx1 = 0.f, wxx2 = 0.f;                       // wxx of rows r-1, r-2
     float dY1 = 0.f, dY2 = 0.f, dY3 = 0.f, dY4 = 0.f;   // dY of rows r-1 .. r-4 (dY_j = y_{j+1} - y_j)
@@ -380,74 +343,21 @@ __device__ __forceinline__ void flexure_strip(const float* __restrict__ whi, con
     float mx0 = 0.f, mx1 = 0.f, mx2 = 0.f;                         // mx_xx of rows m .. m-2
     // the next row's loads are issued one iteration ahead
     int r = o0 - 4;
-    const bool stg = STG && rprev != nullptr;   // uniform
-    auto ld_pair = [&](int rr, float& h, float& l, double& yy, float& rv) {
-        if (cin && rr >= 0 && rr < ny) {
-            const size_t e = (size_t)rr * nx + cc;
-            if constexpr (PAIR) {
-                h = __ldg(whi + e);
-                l = __ldg(wlo + e);
-                if (stg) rv = __ldg(rprev + e);
-            } else {
-                yy = __ldg(y + e);
-            }
-        } else {
-            h = 0.f;
-            l = 0.f;
-            yy = 0.0;
-            rv = 0.f;
-        }
-    };
-    float hn = 0.f, ln = 0.f, rn = 0.f;
-    double yn = 0.0;
-    ld_pair(r, hn, ln, yn, rn);
-    // the fields of input row rr that are used at rows m = rr - 2 (D) and
-    // o = rr - 4 (mask, load, 1/(2 eta), and with STG dxw and rprev)
-    auto ld_rest = [&](int rr, float& Dv, uint32_t& mv, float& qv, float& iev, float& dv, float& rov) {
-        const int mm = rr - 2, oo = rr - 4;
-        const bool mr = cin && mm >= 0 && mm < ny;
-        Dv = mr ? __ldg(D + (size_t)mm * nx + cc) : 0.f;
-        const bool orr = outl && oo >= o0 && oo < o1;
-        const size_t ee = orr ? (size_t)oo * nx + cc : 0;
-        mv = orr ? (uint32_t)__ldg(mask + ee) : 0u;
-        qv = orr ? __ldg(q0 + ee) : 0.f;
-        iev = orr ? __ldg(inv2eta + ee) : 0.f;
-        if constexpr (STG) {
-            dv = orr ? __ldg(dxw + ee) : 0.f;
-            rov = (orr && stg) ? __ldg(rprev + ee) : 0.f;
-        }
-    };
+    auto ld = [&](int rr) { return cin && rr >= 0 && rr < ny ? __ldg(y + (size_t)rr * nx + cc) : 0.0; };
+    double yn = ld(r);
     for (; r < o1 + 4; ++r) {
-        const float h = hn, l = ln, rv = rn;
         const double yv = yn;
-        ld_pair(r + 1, hn, ln, yn, rn);
+        yn = ld(r + 1);
         const int m = r - 2, o = r - 4;
         const bool orow = outl && o >= o0 && o < o1;
         const size_t eo = orow ? (size_t)o * nx + cc : 0;
-        float Dm, oq, oie, od = 0.f, orv = 0.f;
-        uint32_t om;
-        if constexpr (STG) {
-            ld_rest(r, Dm, om, oq, oie, od, orv);
-        } else {
-            const bool mrow = cin && m >= 0 && m < ny;
-            Dm = mrow ? __ldg(D + (size_t)m * nx + cc) : 0.f;
-            om = orow ? __ldg(mask + eo) : (uint8_t)0;
-            oq = orow ? __ldg(q0 + eo) : 0.f;
-            oie = orow ? __ldg(inv2eta + eo) : 0.f;
-        }
+        const bool mrow = cin && m >= 0 && m < ny;
+        const float Dm = mrow ? __ldg(D + (size_t)m * nx + cc) : 0.f;
+        const uint32_t om = orow ? (uint32_t)__ldg(mask + eo) : 0u;
+        const float oq = orow ? __ldg(q0 + eo) : 0.f, oie = orow ? __ldg(inv2eta + eo) : 0.f;
         // row r: first differences, Wx, wxx
-        float dX;
-        if constexpr (PAIR) {
-            const float hr = __shfl_down_sync(FULL, h, 1), lr = __shfl_down_sync(FULL, l, 1);
-            dX = (hr - h) + (lr - l);
-            if constexpr (STG) {
-                const float rr = __shfl_down_sync(FULL, rv, 1);
-                if (stg) dX += sdf * (rr - rv);
-            }
-        } else {
-            const double yr = __shfl_down_sync(FULL, yv, 1);
-            dX = (float)(yr - yv);
-        }
+        const double yr = __shfl_down_sync(FULL, yv, 1);
+        const float dX = (float)(yr - yv);
         const float dXm = __shfl_up_sync(FULL, dX, 1);
         float Wx, wxx;
         if (edge) {
@@ -458,18 +368,7 @@ __device__ __forceinline__ void flexure_strip(const float* __restrict__ whi, con
             Wx = (dX + dXm) * c.inv_2dx;
             wxx = (dX - dXm) * c.inv_dx2;
         }
-        float dYn;   // dY of row r - 1
-        if constexpr (PAIR) {
-            dYn = (h - hp) + (l - lp);
-            if constexpr (STG) {
-                if (stg) dYn += sdf * (rv - rp);
-                rp = rv;
-            }
-        } else {
-            dYn = (float)(yv - yp);
-        }
-        hp = h;
-        lp = l;
+        const float dYn = (float)(yv - yp);   // dY of row r - 1
         yp = yv;
         dY4 = dY3; dY3 = dY2; dY2 = dY1; dY1 = dYn;
         // moments of row m = r - 2 (Wx1..3 are still those of rows r-1..r-3)
@@ -521,30 +420,10 @@ __device__ __forceinline__ void flexure_strip(const float* __restrict__ whi, con
                 my_yy = ((My1 - 2.f * My2) + My3) * c.inv_dy2;
             }
             float p = om ? oq : 0.f;
-            if constexpr (!PAIR) {
-                if (om && wref) p += c.coef_mantle * (float)(__ldg(y + eo) - __ldg(wref + eo));
-            }
-            if constexpr (STG) {
-                if (om) {
-                    float dy = od;
-                    if (stg) dy += sdf * (orv - cmdf);
-                    p = oq + c.coef_mantle * dy;
-                }
-            }
+            if (om && wref) p += c.coef_mantle * (float)(__ldg(y + eo) - __ldg(wref + eo));
             f[eo] = (((p + mx2) + 2.f * mxy_xy) + my_yy) * oie;
         }
     }
-}
-
-__global__ void __launch_bounds__(256)
-k_flexure_strip(const float* __restrict__ whi, const float* __restrict__ wlo, const float* __restrict__ q0,
-                const uint8_t* __restrict__ mask, const float* __restrict__ D, const float* __restrict__ inv2eta,
-                float* __restrict__ f, int nx, int ny, FlexCoefF c, int seg, const int* __restrict__ gate)
-{
-    if (gate && *gate == 0) return;
-    const int task = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (task >= strip_tasks(nx, ny, seg)) return;   // whole warps
-    flexure_strip<true>(whi, wlo, q0, mask, D, inv2eta, f, nx, ny, c, seg, task);
 }
 
 __global__ void __launch_bounds__(256)
@@ -555,30 +434,7 @@ k_flexure_strip_y(const double* __restrict__ y, const double* __restrict__ wref,
     if (gate && *gate == 0) return;
     const int task = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (task >= strip_tasks(nx, ny, seg)) return;   // whole warps
-    flexure_strip<false>(nullptr, nullptr, q0, mask, D, inv2eta, f, nx, ny, c, seg, task, y, wref);
-}
-
-// RK4 stage RHS from the float pair of x: stage scale sdf = (a h) spy with h
-// the step size in the control block, cm the corner mean of rprev; thread 0
-// forms both (the only FP64 instructions of the kernel).
-__global__ void __launch_bounds__(256)
-k_flexure_strip_stage(const float* __restrict__ whi, const float* __restrict__ wlo, const float* __restrict__ rprev,
-                      const float* __restrict__ dxw, const float* __restrict__ q0, const uint8_t* __restrict__ mask,
-                      const float* __restrict__ D, const float* __restrict__ inv2eta, float* __restrict__ f, int nx,
-                      int ny, FlexCoefF c, int seg, const Ctl* __restrict__ ctl, double a, double spy,
-                      const int* __restrict__ gate)
-{
-    if (gate && *gate == 0) return;
-    __shared__ float s_sc[2];
-    if (threadIdx.x == 0) {
-        s_sc[0] = rprev ? (float)(a * ctl->h * spy) : 0.f;
-        s_sc[1] = rprev ? (float)corner_mean_of(rprev, nx, ny) : 0.f;
-    }
-    __syncthreads();
-    const int task = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (task >= strip_tasks(nx, ny, seg)) return;   // whole warps
-    flexure_strip<true, true>(whi, wlo, q0, mask, D, inv2eta, f, nx, ny, c, seg, task, nullptr, nullptr, rprev,
-                              s_sc[0], s_sc[1], dxw);
+    flexure_strip(y, wref, q0, mask, D, inv2eta, f, nx, ny, c, seg, task);
 }
 
 // rows per warp task for a single domain: enough tasks to fill the GPU
@@ -834,17 +690,199 @@ k_flexure_f32(const double* __restrict__ y, const double* __restrict__ wref, con
               float* __restrict__ f, int nx, int ny, FlexCoefF c, const int* __restrict__ gate)
 {
     if (gate && *gate == 0) return;
-    flexure_f32_body<false>(y, wref, q0, mask, D, inv2eta, f, nx, ny, c, blockIdx.x, blockIdx.y);
+    flexure_f32_body(y, wref, q0, mask, D, inv2eta, f, nx, ny, c, blockIdx.x, blockIdx.y);
 }
 
-__global__ void __launch_bounds__(TX* TY)
-k_flexure_f32_hilo(const float* __restrict__ whi, const float* __restrict__ wlo, const float* __restrict__ q0,
-                   const uint8_t* __restrict__ mask, const float* __restrict__ D, const float* __restrict__ inv2eta,
-                   float* __restrict__ f, int nx, int ny, FlexCoefF c, const int* __restrict__ gate)
+// ---------------------------------------------------------------------------
+// Mixed stencil by tiles (uniform spacing), the state as a float pair x =
+// whi + wlo.  With rprev (the previous stage's raw RHS) the RK stage state
+// x + sdf (rprev - cm) is formed on the way into the tile, sdf = (a h) spy
+// with h the step size in the control block and cm the corner mean of rprev
+// (thread 0 has the only FP64 instructions).  With dxw = x - w_ref the load
+// takes the mantle term coef_mantle (dxw + sdf (rprev - cm)) at masked cells.
+// Moments come from the tile, f from the moments.  64 x 16 outputs, 256 threads as four groups of
+// 64 columns: a thread keeps its column in every pass, walks down it with the
+// vertical window in registers, and has some fifteen independent loads in
+// flight where column strips (a warp per 28 columns, shuffles for the
+// x-neighbours) had one row's and waited on them: 2048^2 54.1 -> 43.9 us, 512 x
+// 1024 16.8 -> 10.6 us an RK4 stage.  The tile is bound by instruction issue:
+// with cell indices divided out per element it issued 304 a cell and took
+// 50.9 us at 2048^2.
+// The grid is even in both directions, so the last tile has two columns and
+// two rows at least, which the one-sided forms at the far edges need.
+// ---------------------------------------------------------------------------
+constexpr int TXF = 64, TYF = 16, NGF = 4, YRF = TYF + 4, YCF = TXF + 4, MRF = TYF + 2, MCF = TXF + 2;
+
+__device__ __forceinline__ void flexure_tile(const float* __restrict__ whi, const float* __restrict__ wlo,
+                                             const float* __restrict__ rprev, const float* __restrict__ dxw,
+                                             const float* __restrict__ q0, const uint8_t* __restrict__ mask,
+                                             const float* __restrict__ D, const float* __restrict__ inv2eta,
+                                             float* __restrict__ f, int nx, int ny, const FlexCoefF& c, int bx, int by,
+                                             const Ctl* __restrict__ ctl = nullptr, double a = 0.0, double spy = 0.0)
+{
+    __shared__ float2 ys[YRF][YCF];
+    __shared__ float Mxx[MRF][MCF], Myy[MRF][MCF], Mxy[MRF][MCF];
+    __shared__ float s_sc[2];
+    const int tid = threadIdx.x + threadIdx.y * blockDim.x, tx = tid % TXF, grp = tid / TXF;
+    const int i0 = bx * TXF, j0 = by * TYF;
+    const int gi = i0 + tx;                            // this thread's column
+    const bool col = gi < nx;
+    if (tid == 0) {
+        s_sc[0] = rprev ? (float)(a * ctl->h * spy) : 0.f;
+        s_sc[1] = rprev ? (float)corner_mean_of(rprev, nx, ny) : 0.f;
+    }
+    // the state: this column's rows grp, grp + 4, ..; the four halo columns by
+    // the first 80 threads
+    constexpr int NL = YRF / NGF;
+    float2 xv[NL + 1];
+    float rv[NL + 1];
+    const int hr = tid / 4, hc = tid % 4, hx = hc < 2 ? hc : TXF + hc;   // halo element: row, tile column
+    {
+        const int ha = i0 - 2 + hx;
+#pragma unroll
+        for (int q = 0; q <= NL; ++q) {
+            const int r = q < NL ? grp + NGF * q : hr, i = q < NL ? gi : ha, j = j0 - 2 + r;
+            const bool in = (q < NL || tid < 4 * YRF) && i >= 0 && i < nx && j >= 0 && j < ny;
+            const int g = in ? j * nx + i : 0;
+            xv[q] = in ? make_float2(__ldg(whi + g), __ldg(wlo + g)) : make_float2(0.f, 0.f);
+            rv[q] = in && rprev ? __ldg(rprev + g) : 0.f;
+        }
+    }
+    __syncthreads();
+    const float sdf = s_sc[0], cm = s_sc[1];
+#pragma unroll
+    for (int q = 0; q <= NL; ++q) {
+        float2 v = xv[q];
+        if (rprev) {   // two-sum of the pair and the increment (its corner mean drops out of every difference)
+            const float inc = sdf * rv[q];
+            const float sm = v.x + inc, bb = sm - v.x;
+            const float er = (v.x - (sm - bb)) + (inc - bb);
+            const float l2 = v.y + er;
+            v.x = sm + l2;
+            v.y = l2 - (v.x - sm);
+        }
+        if (q < NL) ys[grp + NGF * q][tx + 2] = v;
+        else if (tid < 4 * YRF) ys[hr][hx] = v;
+    }
+    __syncthreads();
+    auto dif = [](float2 p, float2 q) { return (q.x - p.x) + (q.y - p.y); };
+    // moments of grid rows j0 - 1 .. j0 + 16, a run per group, walking down
+    // three rows of this column
+    const bool left = gi == 0, right = gi == nx - 1;
+    const int lc = tx + 2 + (left ? 1 : right ? -1 : 0);   // centre of the second x-differences (tile column)
+    const float sx = left || right ? c.inv_dx : c.inv_2dx;
+    if (col) {
+        constexpr int RUN = (MRF + NGF - 1) / NGF;
+        int m0 = grp * RUN, m1 = min(m0 + RUN, MRF);
+        if (j0 == 0 && m0 == 0) m0 = 1;
+        m1 = min(m1, ny + 1 - j0);
+        float w0 = 0.f, w1 = 0.f, w2, x1 = 0.f, x2;
+        float2 y0, y1, y2;
+        auto row = [&](int r, float& w, float& x, float2& y) {   // tile row r
+            const float2 p = ys[r][lc - 1], q = ys[r][lc], s = ys[r][lc + 1];
+            const float dA = dif(p, q), dB = dif(q, s);
+            x = (dB - dA) * c.inv_dx2;
+            w = (left ? dA : right ? dB : dA + dB) * sx;
+            y = left ? p : right ? s : q;
+        };
+        if (m0 < m1) {
+            row(m0, w0, x1, y0);
+            row(m0 + 1, w1, x1, y1);
+        }
+        const float* Dp = D + (j0 - 1) * nx + gi;
+#pragma unroll
+        for (int q = 0; q < RUN; ++q) {
+            const int m = m0 + q, j = j0 - 1 + m;
+            if (m >= m1) break;
+            const float Dl = __ldg(Dp + m * nx);
+            row(m + 2, w2, x2, y2);
+            float wxy, wyy;
+            if (j == 0 || j == ny - 1) {
+                wxy = (j == 0 ? w2 - w1 : w1 - w0) * c.inv_dy;
+                const int r = (j == 0 ? 1 : ny - 2) - j0 + 2;
+                wyy = (dif(ys[r][tx + 2], ys[r + 1][tx + 2]) - dif(ys[r - 1][tx + 2], ys[r][tx + 2])) * c.inv_dy2;
+            } else {
+                wxy = (w2 - w0) * c.inv_2dy;
+                wyy = (dif(y1, y2) - dif(y0, y1)) * c.inv_dy2;
+            }
+            Mxx[m][tx + 1] = -Dl * (x1 + c.nu * wyy);
+            Myy[m][tx + 1] = -Dl * (wyy + c.nu * x1);
+            Mxy[m][tx + 1] = (-Dl * c.one_minus_nu) * wxy;
+            w0 = w1; w1 = w2; x1 = x2; y0 = y1; y1 = y2;
+        }
+    }
+    // and of the two columns beside the tile
+    if (tid >= TXF * NGF - 2 * MRF) {
+        const int e = tid - (TXF * NGF - 2 * MRF), m = e / 2, mx = e % 2 ? MCF - 1 : 0;
+        const int i = i0 - 1 + mx, j = j0 - 1 + m;
+        if (i >= 0 && i < nx && j >= 0 && j < ny) {
+            const int lx = mx + 1, ly = m + 1;
+            const int cx = lx + (i == 0) - (i == nx - 1), cy = ly + (j == 0) - (j == ny - 1);
+            const int xl = lx - (i > 0), xr = lx + (i < nx - 1), yl = ly - (j > 0), yr = ly + (j < ny - 1);
+            const float hxs = xr - xl == 2 ? c.inv_2dx : c.inv_dx, hys = yr - yl == 2 ? c.inv_2dy : c.inv_dy;
+            const float Dl = __ldg(D + j * nx + i);
+            const float wxx = (dif(ys[ly][cx], ys[ly][cx + 1]) - dif(ys[ly][cx - 1], ys[ly][cx])) * c.inv_dx2;
+            const float wyy = (dif(ys[cy][lx], ys[cy + 1][lx]) - dif(ys[cy - 1][lx], ys[cy][lx])) * c.inv_dy2;
+            const float wxy = (dif(ys[yr][xl], ys[yr][xr]) * hxs - dif(ys[yl][xl], ys[yl][xr]) * hxs) * hys;
+            Mxx[m][mx] = -Dl * (wxx + c.nu * wyy);
+            Myy[m][mx] = -Dl * (wyy + c.nu * wxx);
+            Mxy[m][mx] = (-Dl * c.one_minus_nu) * wxy;
+        }
+    }
+    // the output rows' operands, requested before the barrier
+    constexpr int RO = TYF / NGF;
+    float qv[RO], iv[RO], dv[RO], ov[RO];
+    uint32_t on[RO];
+    const int o0 = grp * RO, ge = (j0 + o0) * nx + gi;
+#pragma unroll
+    for (int q = 0; q < RO; ++q) {
+        const bool in = col && j0 + o0 + q < ny;
+        const int g = in ? ge + q * nx : 0;
+        qv[q] = in ? __ldg(q0 + g) : 0.f;
+        iv[q] = in ? __ldg(inv2eta + g) : 0.f;
+        dv[q] = in && dxw ? __ldg(dxw + g) : 0.f;
+        ov[q] = in && rprev ? __ldg(rprev + g) : 0.f;
+        on[q] = in ? (uint32_t)__ldg(mask + g) : 0u;
+    }
+    __syncthreads();
+    if (!col) return;
+    const int mc = tx + 1, cc = mc + (left ? 1 : right ? -1 : 0), cl = mc - (left ? 0 : 1), cr = mc + (right ? 0 : 1);
+    // output row o is row o + 1 of the moments
+    float q0v = (Mxy[o0][cr] - Mxy[o0][cl]) * sx, q1v = (Mxy[o0 + 1][cr] - Mxy[o0 + 1][cl]) * sx;
+    float y0 = Myy[o0][mc], y1 = Myy[o0 + 1][mc];
+#pragma unroll
+    for (int q = 0; q < RO; ++q) {
+        const int o = o0 + q, j = j0 + o, m = o + 1;
+        if (j >= ny) break;
+        const float q2v = (Mxy[m + 1][cr] - Mxy[m + 1][cl]) * sx, y2 = Myy[m + 1][mc];
+        const float mxx = ((Mxx[m][cc + 1] - 2.f * Mxx[m][cc]) + Mxx[m][cc - 1]) * c.inv_dx2;
+        float mxy, myy;
+        if (j == 0 || j == ny - 1) {
+            mxy = (j == 0 ? q2v - q1v : q1v - q0v) * c.inv_dy;
+            const int r = (j == 0 ? 1 : ny - 2) - j0 + 1;
+            myy = ((Myy[r + 1][mc] - 2.f * Myy[r][mc]) + Myy[r - 1][mc]) * c.inv_dy2;
+        } else {
+            mxy = (q2v - q0v) * c.inv_2dy;
+            myy = ((y2 - 2.f * y1) + y0) * c.inv_dy2;
+        }
+        float dy = dv[q];
+        if (rprev) dy += sdf * (ov[q] - cm);
+        const float p = on[q] ? (dxw ? qv[q] + c.coef_mantle * dy : qv[q]) : 0.f;
+        f[ge + q * nx] = (((p + mxx) + 2.f * mxy) + myy) * iv[q];
+        q0v = q1v; q1v = q2v; y0 = y1; y1 = y2;
+    }
+}
+
+__global__ void __launch_bounds__(TXF* NGF)
+k_flexure_tile(const float* __restrict__ whi, const float* __restrict__ wlo, const float* __restrict__ rprev,
+               const float* __restrict__ dxw, const float* __restrict__ q0, const uint8_t* __restrict__ mask,
+               const float* __restrict__ D, const float* __restrict__ inv2eta, float* __restrict__ f, int nx, int ny,
+               FlexCoefF c, const Ctl* __restrict__ ctl, double a, double spy, const int* __restrict__ gate)
 {
     if (gate && *gate == 0) return;
-    flexure_f32_body<true>(nullptr, nullptr, q0, mask, D, inv2eta, f, nx, ny, c, blockIdx.x, blockIdx.y, whi, wlo);
+    flexure_tile(whi, wlo, rprev, dxw, q0, mask, D, inv2eta, f, nx, ny, c, blockIdx.x, blockIdx.y, ctl, a, spy);
 }
+static dim3 tile_grid(int nx, int ny) { return dim3((nx + TXF - 1) / TXF, (ny + TYF - 1) / TYF); }
 
 template <typename T>
 void launch_flexure(const double* y, const double* wref, const T* q0, const uint8_t* mask, const T* D,
@@ -855,10 +893,9 @@ void launch_flexure(const double* y, const double* wref, const T* q0, const uint
     if (sizeof(T) == 4 && c.ixm == nullptr) {
         const FlexCoefF cf = flex_coef_f32(c);
         if (whi && !wref) {
-            const int seg = strip_seg_single(nx, ny);
-            const int tasks = ((nx + SW - 1) / SW) * ((ny + seg - 1) / seg);
-            k_flexure_strip<<<(tasks + 7) / 8, 256, 0, s>>>(whi, wlo, (const float*)q0, mask, (const float*)D,
-                                                            (const float*)inv2eta, (float*)f, nx, ny, cf, seg, gate);
+            k_flexure_tile<<<tile_grid(nx, ny), TXF * NGF, 0, s>>>(whi, wlo, nullptr, nullptr, (const float*)q0, mask,
+                                                                   (const float*)D, (const float*)inv2eta, (float*)f,
+                                                                   nx, ny, cf, nullptr, 0.0, 0.0, gate);
             return;
         }
         // the FP64 state by column strips (the shared-memory tile form is
@@ -894,11 +931,8 @@ void launch_flexure_stage(const float* whi, const float* wlo, const float* rprev
                           const FlexCoef& c, const Ctl* ctl, double a, double spy, cudaStream_t s,
                           const int* gate)
 {
-    const FlexCoefF cf = flex_coef_f32(c);
-    const int seg = strip_seg_single(nx, ny);
-    const int tasks = ((nx + SW - 1) / SW) * ((ny + seg - 1) / seg);
-    k_flexure_strip_stage<<<(tasks + 7) / 8, 256, 0, s>>>(whi, wlo, rprev, dxw, q0, mask, D, inv2eta, f, nx, ny, cf,
-                                                          seg, ctl, a, spy, gate);
+    k_flexure_tile<<<tile_grid(nx, ny), TXF * NGF, 0, s>>>(whi, wlo, rprev, dxw, q0, mask, D, inv2eta, f, nx, ny,
+                                                           flex_coef_f32(c), ctl, a, spy, gate);
 }
 
 // ---------------------------------------------------------------------------
@@ -1316,12 +1350,9 @@ __global__ void __launch_bounds__(256) k_b_flexure(const BMember* __restrict__ M
         const BMember& b = M[m];
         const int bx = local % b.fgx, by = local / b.fgx;
         if constexpr (sizeof(T) == 4) {
-            // mixed members have uniform spacing and carry now%w as a float
-            // pair: column strips, 8 warp tasks per virtual block
-            const int task = local * 8 + (int)threadIdx.y;   // 32 x 8 block: warp = threadIdx.y
-            if (task < strip_tasks(b.p.nx, b.p.ny, b.fseg))
-                flexure_strip<true>(b.d.whi, b.d.wlo, (const float*)b.q0, b.mask, (const float*)b.D,
-                              (const float*)b.inv2eta, (float*)b.f, b.p.nx, b.p.ny, b.fcf, b.fseg, task);
+            // mixed members have uniform spacing and carry now%w as a float pair
+            flexure_tile(b.d.whi, b.d.wlo, nullptr, nullptr, (const float*)b.q0, b.mask, (const float*)b.D,
+                         (const float*)b.inv2eta, (float*)b.f, b.p.nx, b.p.ny, b.fcf, bx, by);
         } else if (b.fc.ixm == nullptr) {
             flexure_tile64<false>(b.y, nullptr, nullptr, (const double*)b.q0, b.mask, (const double*)b.D,
                                   (const double*)b.inv2eta, (double*)b.f, b.p.nx, b.p.ny, b.fc64, bx, by);
@@ -1408,11 +1439,15 @@ template <typename T> void batch_grids(size_t rows_smem, size_t cols_smem, int r
 
 template <typename T> void batch_flexure(const BMember* M, BList L, int nblk, cudaStream_t s)
 {
-    // 256 threads: the tile body reads them as TX x TY, the strip body as 8 warps
+    // 256 threads: the FP64 tiles read them as TX x TY, the mixed one as 4 x 64
     k_b_flexure<T><<<nblk, dim3(TX, TY), 0, s>>>(M, L);
 }
 int batch_flexure_tiles64(int nx, int ny) { return ((nx + TX - 1) / TX) * ((ny + TY64 - 1) / TY64); }
-int batch_flexure_blocks(int nx, int ny, int seg) { return (((nx + SW - 1) / SW) * ((ny + seg - 1) / seg) + 7) / 8; }
+int batch_flexure_tiles32(int nx, int ny)
+{
+    const dim3 g = tile_grid(nx, ny);
+    return (int)(g.x * g.y);
+}
 template <typename T>
 void batch_rows_fwd(const BMember* M, BList L, int nblk, int threads, size_t smem, cudaStream_t s)
 {
@@ -1433,9 +1468,9 @@ void batch_rows_inv(const BMember* M, BList L, int nblk, int threads, size_t sme
 }
 
 // True stages: the RHS at stage state y (stage 0: x, 1-5: the stage buffer,
-// 6: x2) with the mantle term at that state: mixed members by column strips
-// over the float pair of the stage state (stage 0: of x) and its dxw, FP64
-// members (and mixed ones without the pairs) by shared-memory tiles.
+// 6: x2) with the mantle term at that state: mixed members over
+// the float pair of the stage state (stage 0: of x) and its dxw, mixed ones
+// without the pairs and FP64 members over the FP64 state.
 template <typename T>
 __global__ void __launch_bounds__(256) k_b_flexure_y(const BMember* __restrict__ M, BList L, int stage)
 {
@@ -1445,16 +1480,12 @@ __global__ void __launch_bounds__(256) k_b_flexure_y(const BMember* __restrict__
         const double* y = stage == 0 ? b.d.x : (stage == 6 ? b.d.ts_x2 : b.yst);
         if constexpr (sizeof(T) == 4) {
             if (b.yhi) {
-                const int task = local * 8 + (int)threadIdx.y;   // 32 x 8 block: warp = threadIdx.y
-                if (task < strip_tasks(b.p.nx, b.p.ny, b.fseg)) {
-                    const bool s0 = stage == 0;
-                    flexure_strip<true, true>(s0 ? b.xhi : b.yhi, s0 ? b.xlo : b.ylo, (const float*)b.q0, b.mask,
-                                              (const float*)b.D, (const float*)b.inv2eta, (float*)b.f, b.p.nx,
-                                              b.p.ny, b.fcf, b.fseg, task, nullptr, nullptr, nullptr, 0.f, 0.f,
-                                              s0 ? b.xdw : b.ydw);
-                }
+                const bool s0 = stage == 0;
+                flexure_tile(s0 ? b.xhi : b.yhi, s0 ? b.xlo : b.ylo, nullptr, s0 ? b.xdw : b.ydw, (const float*)b.q0,
+                             b.mask, (const float*)b.D, (const float*)b.inv2eta, (float*)b.f, b.p.nx, b.p.ny, b.fcf,
+                             bx, by);
             } else {
-                flexure_f32_body<false>(y, b.wref, (const float*)b.q0, b.mask, (const float*)b.D,
+                flexure_f32_body(y, b.wref, (const float*)b.q0, b.mask, (const float*)b.D,
                                         (const float*)b.inv2eta, (float*)b.f, b.p.nx, b.p.ny, b.fcf, bx, by);
             }
         } else if (b.fc.ixm == nullptr) {
