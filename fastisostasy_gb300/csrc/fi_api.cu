@@ -723,7 +723,7 @@ template <typename T> void tune_rhs_shapes(fi_handle* h)
     int best_rb = 0, best_cb = 0, best_rt = 0, best_ct = 0;
     float tr = 1e30f, tc = 1e30f;
     // (register lines fix the threads of a line: only the lines per block are tried)
-    const int lr = rhs_line_threads(p.h, sizeof(T) == 4), lc = rhs_line_threads(p.ny, sizeof(T) == 4);
+    const int lr = rhs_line_threads(p.h, p, sizeof(T) == 4), lc = rhs_line_threads(p.ny, p, sizeof(T) == 4);
     for (int rb : {1, 2, 4, 8, 16, 32}) {
         if (lr ? rb * lr > 512 || rb * lr < 32 : rb > 8 || 2 * (size_t)rb * p.h * sizeof(C2) > (size_t)optin) continue;
         for (int rt : {128, 256, 512, 1024}) {
@@ -847,7 +847,7 @@ template <typename T> void tune_conv_shapes(fi_handle* h)
     const double scale = 1.0 / ((double)h->Px * (double)h->Py);
     int best_rb = 0, best_cb = 0, best_rt = 0, best_ct = 0;
     float tr = 1e30f, tc = 1e30f;
-    const int lr = rhs_line_threads(p.h, sizeof(T) == 4), lc = rhs_line_threads(p.ny, sizeof(T) == 4);
+    const int lr = rhs_line_threads(p.h, p, sizeof(T) == 4), lc = rhs_line_threads(p.ny, p, sizeof(T) == 4);
     for (int rb : {1, 2, 4, 8, 16, 32}) {
         if (lr ? rb * lr > 512 || rb * lr < 32 : rb > 4 || 2 * (size_t)rb * p.h * sizeof(C2) > (size_t)optin) continue;
         for (int rt : {128, 256, 512, 1024}) {
@@ -2615,7 +2615,7 @@ int batch_shape(fi_batch* b, int RB, int CB, int waves)
     auto shape_of = [&](BMember& m, int& rt, int& ct) {
         m.RB = RB > 0 ? RB : rhs_rows_per_block(m.p.h);
         m.CB = CB > 0 ? CB : (b->mixed ? rhs_cols_per_block<float>(m.p.ny) : rhs_cols_per_block<double>(m.p.ny));
-        const int lr = rhs_line_threads(m.p.h, b->mixed), lc = rhs_line_threads(m.p.ny, b->mixed);
+        const int lr = rhs_line_threads(m.p.h, m.p, b->mixed), lc = rhs_line_threads(m.p.ny, m.p, b->mixed);
         m.lines = (lr > 0 ? 1 : 0) | (lc > 0 ? 2 : 0);
         auto line_block = [](int lines, int th) {
             int t = lines * th;
@@ -2633,8 +2633,8 @@ int batch_shape(fi_batch* b, int RB, int CB, int waves)
     }
     for (int i = 0; i < n; ++i) {
         BMember& m = b->hM[i];
-        if (m.lines & 1) m.RB = b->rows_threads / rhs_line_threads(m.p.h, b->mixed);
-        if (m.lines & 2) m.CB = b->cols_threads / rhs_line_threads(m.p.ny, b->mixed);
+        if (m.lines & 1) m.RB = b->rows_threads / rhs_line_threads(m.p.h, m.p, b->mixed);
+        if (m.lines & 2) m.CB = b->cols_threads / rhs_line_threads(m.p.ny, m.p, b->mixed);
         // stencil tiles: the FP64 state of true stages without the pairs has its own
         const bool pair = b->mixed && (!b->true_stages || m.yhi);
         m.fgx = pair ? (m.p.nx + 63) / 64 : (m.p.nx + 31) / 32;

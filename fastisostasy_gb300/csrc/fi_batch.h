@@ -88,7 +88,7 @@ int batch_flexure_tiles64(int nx, int ny);
 // Block shapes of the single-domain launches (shared with the batched ones).
 int rhs_rows_per_block(int h);
 int rhs_threads_for(int work);
-int rhs_line_threads(int n, bool f32);      // threads of a register line of n points, 0: none
+int rhs_line_threads(int n, const Plan2D& p, bool f32);   // threads of a register line of n points, 0: none
 size_t rhs_line_bytes(int n, bool f32);     // its shared memory
 template <typename T> int rhs_cols_per_block(int ny);
 int reduce_grid(size_t n);

@@ -164,7 +164,7 @@ template <typename T>
 bool lines_rows_fwd(const T* in, int in_pitch, int in_width, int nrows_in, typename vec2<T>::type* S, const Plan2D& p,
                     cudaStream_t s, const int* gate)
 {
-    if (!line_threads<T>(p.h) || p.h > 2048) return false;
+    if (!line_threads<T>(p.h, (long long)p.h * p.ny) || p.h > 2048) return false;
 #define FI_GO(N)                                                                                     \
     FI_LAUNCH(k_lines_rows_fwd, N, (p.rb > 0 ? p.rb : line_default<T, N, false>()), nrows_in, in, in_pitch, in_width, \
               nrows_in, S, p, gate)
@@ -177,7 +177,7 @@ template <typename T>
 bool lines_rows_inv(const typename vec2<T>::type* S, T* out, const Plan2D& p, double scale, cudaStream_t s,
                     const int* gate)
 {
-    if (!line_threads<T>(p.h) || p.h > 2048) return false;
+    if (!line_threads<T>(p.h, (long long)p.h * p.ny) || p.h > 2048) return false;
 #define FI_GO(N)                                                                                            \
     FI_LAUNCH(k_lines_rows_inv, N, (p.rb > 0 ? p.rb : line_default<T, N, false>()), p.ny, S, p.ny, out, p.nx, p, \
               (T)scale, gate)
@@ -190,7 +190,7 @@ template <typename T>
 bool lines_cols_hartley(typename vec2<T>::type* S, const T* mA, const T* mB, int even, const Plan2D& p, cudaStream_t s,
                         const int* gate)
 {
-    if (!line_threads<T>(p.ny) || p.ny > 2048) return false;
+    if (!line_threads<T>(p.ny, (long long)p.h * p.ny) || p.ny > 2048) return false;
 #define FI_GO(N) \
     FI_LAUNCH(k_lines_cols, N, (p.cb > 0 ? p.cb : line_default<T, N, true>()), p.h + 1, S, mA, mB, even, p, gate)
     FI_LINE_SWITCH(p.ny, FI_GO)
@@ -202,7 +202,7 @@ template <typename T>
 bool lines_cols_conv(typename vec2<T>::type* S, const typename vec2<T>::type* K, int nrows_in, int n_out,
                      const Plan2D& p, cudaStream_t s)
 {
-    if (!line_threads<T>(p.ny) || n_out != nrows_in + 2) return false;
+    if (!line_threads<T>(p.ny, (long long)p.h * p.ny) || n_out != nrows_in + 2) return false;
 #define FI_GO(N) \
     FI_LAUNCH(k_lines_cols_conv, N, (p.cb > 0 ? p.cb : line_default<T, N, true>()), p.h + 1, S, K, nrows_in, p)
     FI_LINE_SWITCH(p.ny, FI_GO)
@@ -216,7 +216,7 @@ template <typename T>
 bool lines_conv_rows_inv(const typename vec2<T>::type* S, int n_out, double* out, int nx, int ny, int i_off,
                          double* corners, int corner_col1, const Plan2D& p, double scale, cudaStream_t s)
 {
-    if (!line_threads<T>(p.h) || p.h > 2048) return false;
+    if (!line_threads<T>(p.h, (long long)p.h * p.ny) || p.h > 2048) return false;
 #define FI_GO(N)                                                                                              \
     FI_LAUNCH(k_lines_conv_rows_inv, N, (p.rb > 0 ? p.rb : line_default<T, N, false>()), n_out, S, n_out, out, nx, ny, \
               i_off, corners, corner_col1, p, (T)scale)

@@ -29,8 +29,17 @@ inline bool has_line(int n)
     const int m = n % 3 == 0 ? n / 3 : n;
     return (m & (m - 1)) == 0 && n >= (n % 3 == 0 ? 24 : 16) && n <= 4096;
 }
-template <typename T> inline int line_threads(int n)
+// `points` (the transform's h x ny): double lines of 3 2^k points hold twelve
+// a thread, so 152 SMs have a warp in every quarter from 233,000 points on,
+// and each warp a serial chain of FP64 instructions three times as long as
+// the shared-memory stages'.  Rows forward / columns / rows inverse, lines
+// against stages: 96^2 16.7 / 24.9 / 16.7 against 10.7 / 18.6 / 10.5 us, 384^2
+// (74,000 points) 19.9 / 31.2 / 20.8 against 18.3 / 27.0 / 16.7, 768^2 (295,000)
+// 30.9 / 51.7 / 31.1 against 37.6 / 57.8 / 35.2, 768 x 384 (147,000) 21.4 /
+// 32.6 / 21.7 against 24.8 / 33.9 / 23.3.
+template <typename T> inline int line_threads(int n, long long points)
 {
+    if (sizeof(T) == 8 && n % 3 == 0 && points < 1 << 17) return 0;
     return has_line(n) ? n / line_points(n, sizeof(T) == 4) : 0;
 }
 // points of shared memory of one line (line_smem)
@@ -155,7 +164,7 @@ __device__ __forceinline__ void cols_hartley_lines(typename vec2<T>::type* __res
 #define FI_LINE_SWITCH(n, FN) \
     switch (n) {              \
     case 16: FN(16); break;   \
-    case 24: FN(24); break;   \
+    case 24: if constexpr (sizeof(T) == 4) { FN(24); } break;   /* no double plan of 131,072 points has it */ \
     case 48: FN(48); break;   \
     case 96: FN(96); break;   \
     case 192: FN(192); break; \

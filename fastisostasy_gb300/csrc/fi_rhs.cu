@@ -1332,12 +1332,13 @@ void launch_conv_rows_inv(const typename vec2<T>::type* S, int n_out, double* ou
 int rhs_rows_per_block(int h) { return rows_per_block(h); }
 int rhs_threads_for(int work) { return threads_for(work); }
 template <typename T> int rhs_cols_per_block(int ny) { return cols_per_block<T>(ny); }
-int rhs_line_threads(int n, bool f32)
+int rhs_line_threads(int n, const Plan2D& p, bool f32)
 {
     // the batched kernels carry every line length they take; one that a
     // single domain would transform on lines has to be among them, or the
     // member would not get the bits it gets alone
-    return f32 ? line_threads<float>(n) : line_threads<double>(n);
+    const long long points = (long long)p.h * p.ny;
+    return f32 ? line_threads<float>(n, points) : line_threads<double>(n, points);
 }
 size_t rhs_line_bytes(int n, bool f32) { return f32 ? line_bytes<float>(n) : line_bytes<double>(n); }
 template int rhs_cols_per_block<float>(int);

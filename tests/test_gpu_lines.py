@@ -37,6 +37,14 @@ def test_rate_on_lines(nx, ny, even, precision):
     _check_rate(nx, ny, even, precision)
 
 
+@pytest.mark.parametrize("nx,ny,even", [(384, 768, False), (768, 384, True), (192, 1536, True), (1536, 192, False),
+                                        (512, 768, True), (340, 768, False)])
+def test_rate_on_double_lines_of_three_times_a_power(nx, ny, even):
+    """FP64 lines of 3 2^k points, taken from 131,072 points of the half
+    spectrum on (the last size has a few less)."""
+    _check_rate(nx, ny, even, 0)
+
+
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("nx,ny,even", [(70, 44, True), (50, 98, False), (154, 26, False), (34, 250, True),
                                         (122, 142, False)])
