@@ -21,6 +21,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 
 #include "fi_fft.cuh"
 
@@ -462,11 +463,29 @@ static int strip_seg_single(int nx, int ny)
 // quarter nothing covers its loads, shuffles and addressing (FP64 pipe 39 %).
 // STAGE: y = x + sc rprev; `off` = sc times the corner mean of rprev, which the
 // differences drop and the mantle term takes off.
+// R output rows of a tile: 16, or fewer where that fills the chip better.  A
+// tile costs R + 2 rows of moments and R of outputs one after the other on its
+// SM, which the rounds of tiles multiply (the last term: what a round cannot
+// overlap of its first loads).  Plain / distorted, 16, 8, 4 rows: 122^2 12.9,
+// 10.2, 8.4 / 15.6, 10.5, 8.7 us; 192^2 13.1, 10.1, 10.2 / 15.9, 10.9, 11.7;
+// 256^2 12.8, 12.6, 13.5 / 15.9, 14.4, 16.0; 384^2 18.3, 18.1, 20.0 / 22.4,
+// 23.3, 26.2; 512^2 28.6, 26.5, 30.3 / 38.6, 36.4, 40.6.
 // ---------------------------------------------------------------------------
-constexpr int TY64 = 16;                              // 32 x 16 outputs, 32 x 8 threads
-constexpr int YR = TY64 + 4, YC = TX + 4, MR = TY64 + 2, MC = TX + 2;
+constexpr int TY64 = 16;                              // 32 x R outputs, 32 x 8 threads
+constexpr int YC = TX + 4, MC = TX + 2;
+static int tile64_rows(int nx, int ny)
+{
+    int best = 16;
+    long long least = -1;
+    for (int r : {16, 8, 4}) {
+        const long long tiles = (long long)((nx + TX - 1) / TX) * ((ny + r - 1) / r);
+        const long long cost = (tiles + 151) / 152 * (2 * r + 2) + r / 2;
+        if (least < 0 || cost < least) { least = cost; best = r; }
+    }
+    return best;
+}
 
-template <bool STAGE>
+template <bool STAGE, int R>
 __device__ __forceinline__ void flexure_tile64(const double* __restrict__ x, const double* __restrict__ rprev,
                                                const double* __restrict__ wref, const double* __restrict__ q0,
                                                const uint8_t* __restrict__ mask, const double* __restrict__ D,
@@ -474,13 +493,13 @@ __device__ __forceinline__ void flexure_tile64(const double* __restrict__ x, con
                                                int ny, const FlexCoef64& c, int bx, int by, double sc = 0.0,
                                                double off = 0.0)
 {
-    __shared__ double ys[YR][YC];
-    __shared__ double Mxx[MR][MC], Myy[MR][MC], Mxy[MR][MC];
+    __shared__ double ys[R + 4][YC];
+    __shared__ double Mxx[R + 2][MC], Myy[R + 2][MC], Mxy[R + 2][MC];
     const int tid = (int)(threadIdx.x + threadIdx.y * blockDim.x);   // 1D or 32 x 8 blocks
-    const int i0 = bx * TX, j0 = by * TY64;
+    const int i0 = bx * TX, j0 = by * R;
     // tiles that touch no edge of the grid carry none of the one-sided forms
-    const bool inner = i0 >= 2 && i0 + TX + 2 <= nx && j0 >= 2 && j0 + TY64 + 2 <= ny;
-    for (int e = tid; e < YR * YC; e += TX * TY) {
+    const bool inner = i0 >= 2 && i0 + TX + 2 <= nx && j0 >= 2 && j0 + R + 2 <= ny;
+    for (int e = tid; e < (R + 4) * YC; e += TX * TY) {
         const int ly = e / YC, lx = e - ly * YC;
         const int gi = i0 - 2 + lx, gj = j0 - 2 + ly;
         double v = 0.0;
@@ -493,7 +512,7 @@ __device__ __forceinline__ void flexure_tile64(const double* __restrict__ x, con
     }
     __syncthreads();
     if (inner) {
-        for (int e = tid; e < MR * MC; e += TX * TY) {
+        for (int e = tid; e < (R + 2) * MC; e += TX * TY) {
             const int my = e / MC, mx = e - my * MC;
             const int ly = my + 1, lx = mx + 1;
             const double Dl = __ldg(D + (size_t)(j0 - 1 + my) * nx + (i0 - 1 + mx));
@@ -509,7 +528,7 @@ __device__ __forceinline__ void flexure_tile64(const double* __restrict__ x, con
             Mxy[my][mx] = Dl * wxy;
         }
     } else {
-        for (int e = tid; e < MR * MC; e += TX * TY) {
+        for (int e = tid; e < (R + 2) * MC; e += TX * TY) {
             const int my = e / MC, mx = e - my * MC;
             const int gi = i0 - 1 + mx, gj = j0 - 1 + my;
             if (gi < 0 || gi >= nx || gj < 0 || gj >= ny) continue;
@@ -529,7 +548,7 @@ __device__ __forceinline__ void flexure_tile64(const double* __restrict__ x, con
         }
     }
     __syncthreads();
-    for (int e = tid; e < TX * TY64; e += TX * TY) {
+    for (int e = tid; e < TX * R; e += TX * TY) {
         const int ly = e / TX, lx = e - ly * TX;
         const int gi = i0 + lx, gj = j0 + ly;
         if (!inner && (gi >= nx || gj >= ny)) continue;
@@ -563,17 +582,18 @@ __device__ __forceinline__ void flexure_tile64(const double* __restrict__ x, con
 // first column's, as the reference does (src/finite_differences.f90:90-91).
 // (256^2: 26.5 us with a division per difference on 32 x 8 tiles, 17 with the
 // stored inverses, 14 on these tiles.)
+template <int R>
 __device__ __forceinline__ void flexure_tile64k(const double* __restrict__ x, const double* __restrict__ wref,
                                                 const double* __restrict__ q0, const uint8_t* __restrict__ mask,
                                                 const double* __restrict__ D, const double* __restrict__ inv2eta,
                                                 double* __restrict__ f, int nx, int ny, const FlexCoef& c, int bx,
                                                 int by)
 {
-    __shared__ double ys[YR][YC];
-    __shared__ double Mxx[MR][MC], Myy[MR][MC], Mxy[MR][MC];
+    __shared__ double ys[R + 4][YC];
+    __shared__ double Mxx[R + 2][MC], Myy[R + 2][MC], Mxy[R + 2][MC];
     const int tid = (int)(threadIdx.x + threadIdx.y * blockDim.x);   // 1D or 32 x 8 blocks
-    const int i0 = bx * TX, j0 = by * TY64;
-    for (int e = tid; e < YR * YC; e += TX * TY) {
+    const int i0 = bx * TX, j0 = by * R;
+    for (int e = tid; e < (R + 4) * YC; e += TX * TY) {
         const int ly = e / YC, lx = e - ly * YC;
         const int gi = i0 - 2 + lx, gj = j0 - 2 + ly;
         ys[ly][lx] = gi >= 0 && gi < nx && gj >= 0 && gj < ny ? __ldg(x + (size_t)gj * nx + gi) : 0.0;
@@ -605,7 +625,7 @@ __device__ __forceinline__ void flexure_tile64k(const double* __restrict__ x, co
         return n;
     };
     const double nu = c.nu, omn = c.one_minus_nu;
-    for (int e = tid; e < MR * MC; e += TX * TY) {
+    for (int e = tid; e < (R + 2) * MC; e += TX * TY) {
         const int my = e / MC, mx = e - my * MC;
         const int gi = i0 - 1 + mx, gj = j0 - 1 + my;
         if (gi < 0 || gi >= nx || gj < 0 || gj >= ny) continue;
@@ -621,7 +641,7 @@ __device__ __forceinline__ void flexure_tile64k(const double* __restrict__ x, co
         Mxy[my][mx] = (-Dl * omn) * wxy;
     }
     __syncthreads();
-    for (int e = tid; e < TX * TY64; e += TX * TY) {
+    for (int e = tid; e < TX * R; e += TX * TY) {
         const int ly = e / TX, lx = e - ly * TX;
         const int gi = i0 + lx, gj = j0 + ly;
         if (gi >= nx || gj >= ny) continue;
@@ -639,24 +659,27 @@ __device__ __forceinline__ void flexure_tile64k(const double* __restrict__ x, co
     }
 }
 
+template <int R>
 __global__ void __launch_bounds__(TX* TY)
 k_flexure64k(const double* __restrict__ y, const double* __restrict__ wref, const double* __restrict__ q0,
              const uint8_t* __restrict__ mask, const double* __restrict__ D, const double* __restrict__ inv2eta,
              double* __restrict__ f, int nx, int ny, FlexCoef c, const int* __restrict__ gate)
 {
     if (gate && *gate == 0) return;
-    flexure_tile64k(y, wref, q0, mask, D, inv2eta, f, nx, ny, c, blockIdx.x, blockIdx.y);
+    flexure_tile64k<R>(y, wref, q0, mask, D, inv2eta, f, nx, ny, c, blockIdx.x, blockIdx.y);
 }
 
+template <int R>
 __global__ void __launch_bounds__(TX* TY)
 k_flexure64(const double* __restrict__ y, const double* __restrict__ wref, const double* __restrict__ q0,
             const uint8_t* __restrict__ mask, const double* __restrict__ D, const double* __restrict__ inv2eta,
             double* __restrict__ f, int nx, int ny, FlexCoef64 c, const int* __restrict__ gate)
 {
     if (gate && *gate == 0) return;
-    flexure_tile64<false>(y, nullptr, wref, q0, mask, D, inv2eta, f, nx, ny, c, blockIdx.x, blockIdx.y);
+    flexure_tile64<false, R>(y, nullptr, wref, q0, mask, D, inv2eta, f, nx, ny, c, blockIdx.x, blockIdx.y);
 }
 
+template <int R>
 __global__ void __launch_bounds__(TX* TY)
 k_flexure64_stage(const double* __restrict__ x, const double* __restrict__ rprev, const double* __restrict__ wref,
                   const double* __restrict__ q0, const uint8_t* __restrict__ mask, const double* __restrict__ D,
@@ -669,7 +692,17 @@ k_flexure64_stage(const double* __restrict__ x, const double* __restrict__ rprev
         s_sc[1] = s_sc[0] * corner_mean_of(rprev, nx, ny);
     }
     __syncthreads();
-    flexure_tile64<true>(x, rprev, wref, q0, mask, D, inv2eta, f, nx, ny, c, blockIdx.x, blockIdx.y, s_sc[0], s_sc[1]);
+    flexure_tile64<true, R>(x, rprev, wref, q0, mask, D, inv2eta, f, nx, ny, c, blockIdx.x, blockIdx.y, s_sc[0], s_sc[1]);
+}
+
+// fn(rows of a tile as a type, grid, block) with the rows tile64_rows takes
+template <typename F> static void tile64_launch(int nx, int ny, F fn)
+{
+    const int r = tile64_rows(nx, ny);
+    const dim3 g((nx + TX - 1) / TX, (ny + r - 1) / r), b(TX, TY);
+    if (r == 4) fn(std::integral_constant<int, 4>{}, g, b);
+    else if (r == 8) fn(std::integral_constant<int, 8>{}, g, b);
+    else fn(std::integral_constant<int, 16>{}, g, b);
 }
 
 void launch_flexure_stage64(const double* x, const double* rprev, const double* wref, const double* q0,
@@ -677,11 +710,13 @@ void launch_flexure_stage64(const double* x, const double* rprev, const double* 
                             const FlexCoef& c, const Ctl* ctl, double a, double spy, cudaStream_t s)
 {
     const FlexCoef64 cf = flex_coef_f64(c);
-    const dim3 b(TX, TY), g((nx + TX - 1) / TX, (ny + TY64 - 1) / TY64);
-    if (rprev)
-        k_flexure64_stage<<<g, b, 0, s>>>(x, rprev, wref, q0, mask, D, inv2eta, f, nx, ny, cf, ctl, a, spy);
-    else
-        k_flexure64<<<g, b, 0, s>>>(x, wref, q0, mask, D, inv2eta, f, nx, ny, cf, nullptr);
+    tile64_launch(nx, ny, [&](auto r, dim3 g, dim3 b) {
+        constexpr int R = decltype(r)::value;
+        if (rprev)
+            k_flexure64_stage<R><<<g, b, 0, s>>>(x, rprev, wref, q0, mask, D, inv2eta, f, nx, ny, cf, ctl, a, spy);
+        else
+            k_flexure64<R><<<g, b, 0, s>>>(x, wref, q0, mask, D, inv2eta, f, nx, ny, cf, nullptr);
+    });
 }
 
 __global__ void __launch_bounds__(TX* TY)
@@ -916,11 +951,13 @@ void launch_flexure(const double* y, const double* wref, const T* q0, const uint
         return;
     }
     if constexpr (sizeof(T) == 8) {
-        const dim3 g64((nx + TX - 1) / TX, (ny + TY64 - 1) / TY64);
-        if (c.ixm == nullptr)
-            k_flexure64<<<g64, b, 0, s>>>(y, wref, q0, mask, D, inv2eta, f, nx, ny, flex_coef_f64(c), gate);
-        else
-            k_flexure64k<<<g64, b, 0, s>>>(y, wref, q0, mask, D, inv2eta, f, nx, ny, c, gate);
+        tile64_launch(nx, ny, [&](auto r, dim3 g64, dim3 b64) {
+            constexpr int R = decltype(r)::value;
+            if (c.ixm == nullptr)
+                k_flexure64<R><<<g64, b64, 0, s>>>(y, wref, q0, mask, D, inv2eta, f, nx, ny, flex_coef_f64(c), gate);
+            else
+                k_flexure64k<R><<<g64, b64, 0, s>>>(y, wref, q0, mask, D, inv2eta, f, nx, ny, c, gate);
+        });
     } else {
         k_flexure<T><<<g, b, 0, s>>>(y, wref, q0, mask, D, inv2eta, f, nx, ny, c, gate);
     }
@@ -1355,10 +1392,10 @@ __global__ void __launch_bounds__(256) k_b_flexure(const BMember* __restrict__ M
             flexure_tile(b.d.whi, b.d.wlo, nullptr, nullptr, (const float*)b.q0, b.mask, (const float*)b.D,
                          (const float*)b.inv2eta, (float*)b.f, b.p.nx, b.p.ny, b.fcf, bx, by);
         } else if (b.fc.ixm == nullptr) {
-            flexure_tile64<false>(b.y, nullptr, nullptr, (const double*)b.q0, b.mask, (const double*)b.D,
+            flexure_tile64<false, TY64>(b.y, nullptr, nullptr, (const double*)b.q0, b.mask, (const double*)b.D,
                                   (const double*)b.inv2eta, (double*)b.f, b.p.nx, b.p.ny, b.fc64, bx, by);
         } else {
-            flexure_tile64k(b.y, nullptr, (const double*)b.q0, b.mask, (const double*)b.D, (const double*)b.inv2eta,
+            flexure_tile64k<TY64>(b.y, nullptr, (const double*)b.q0, b.mask, (const double*)b.D, (const double*)b.inv2eta,
                             (double*)b.f, b.p.nx, b.p.ny, b.fc, bx, by);
         }
         __syncthreads();   // the next virtual block reuses the shared tiles
@@ -1490,10 +1527,10 @@ __global__ void __launch_bounds__(256) k_b_flexure_y(const BMember* __restrict__
                                         (const float*)b.inv2eta, (float*)b.f, b.p.nx, b.p.ny, b.fcf, bx, by);
             }
         } else if (b.fc.ixm == nullptr) {
-            flexure_tile64<false>(y, nullptr, b.wref, (const double*)b.q0, b.mask, (const double*)b.D,
+            flexure_tile64<false, TY64>(y, nullptr, b.wref, (const double*)b.q0, b.mask, (const double*)b.D,
                                   (const double*)b.inv2eta, (double*)b.f, b.p.nx, b.p.ny, b.fc64, bx, by);
         } else {
-            flexure_tile64k(y, b.wref, (const double*)b.q0, b.mask, (const double*)b.D, (const double*)b.inv2eta,
+            flexure_tile64k<TY64>(y, b.wref, (const double*)b.q0, b.mask, (const double*)b.D, (const double*)b.inv2eta,
                             (double*)b.f, b.p.nx, b.p.ny, b.fc, bx, by);
         }
         __syncthreads();

@@ -28,3 +28,19 @@ def test_tile_edges(monkeypatch, nx, ny, par):
     for f in ("w", "z_bed"):
         assert rel(pair.dom.field(f), pair.orc.field(f)) <= 1e-5
     pair.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(6, 4), (32, 6), (34, 66), (66, 160), (224, 226), (322, 162), (512, 130)])
+@pytest.mark.parametrize("par", [dict(dt_method=1), dict(dt_method=2, stage_mode=1, dt_init=8.0, dt_max=8.0)],
+                         ids=["rk4", "tsit54-true"])
+def test_fp64_tile_rows(nx, ny, par):
+    """FP64 tiles of 4, 8 and 16 rows, with last tiles of two rows or columns;
+    the FP64 form's bound."""
+    pair = Pair(workload(nx, ny, nx + 9 * ny, nx != 34, **par), precision=0)
+    pair.init()
+    pair.step(2)
+    a, b = pair.dom.scalars(), pair.orc.scalars()
+    assert a["t"] == pair.t and a["n_accept"] == b["n_accept"] and a["n_reject"] == b["n_reject"]
+    for f in ("w", "z_bed"):
+        assert rel(pair.dom.field(f), pair.orc.field(f)) <= 1e-10
+    pair.close()
