@@ -32,36 +32,74 @@ __device__ __forceinline__ void absmax_bits(unsigned long long& m, double x)
     if (b <= kInfBits && b > m) m = b;
 }
 
-__device__ __forceinline__ double warp_sum(double v)
+// Reductions of a warp's (or its first W lanes') values.  An FP64 instruction
+// issues every 64 clocks per SM quarter, so the grid reductions of the small
+// kernels cost their FP64 instructions: maxima, all of them of non-negative
+// values, are taken on the bit patterns (NaN ignored, as fmax ignores it), two
+// sums share their rounds, half of the lanes each (the same tree, so the same
+// sums), and the second level has as many rounds as it has warps.
+template <int W> __device__ __forceinline__ double warp_sum(double v)
 {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ double warp_max(double v)
+__device__ __forceinline__ double max_nonneg(double a, double x)
 {
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-    return v;
+    unsigned long long m = abs_bits(a);
+    absmax_bits(m, x);
+    return __longlong_as_double((long long)m);
+}
+template <int W> __device__ __forceinline__ double warp_max(double v)
+{
+    unsigned long long m = 0ull;
+    absmax_bits(m, v);
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1) {
+        const unsigned long long u = __shfl_down_sync(0xffffffffu, m, o);
+        m = u > m ? u : m;
+    }
+    return __longlong_as_double((long long)m);
+}
+// a, b -> their sums over W lanes, in lane 0
+template <int W> __device__ __forceinline__ void warp_sum2(double& a, double& b)
+{
+    const bool up = threadIdx.x & (W / 2);
+    const double got = __shfl_xor_sync(0xffffffffu, up ? a : b, W / 2);
+    double mine = (up ? b : a) + got;
+#pragma unroll
+    for (int o = W / 4; o > 0; o >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, o);
+    a = mine;
+    b = __shfl_sync(0xffffffffu, mine, W / 2);
+}
+template <int NV, int W> __device__ __forceinline__ void warp_reduce(double (&v)[NV], const bool (&is_max)[NV])
+{
+    if constexpr (NV == 2) {
+        if (!is_max[0] && !is_max[1]) {
+            warp_sum2<W>(v[0], v[1]);
+            return;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NV; ++q) v[q] = is_max[q] ? warp_max<W>(v[q]) : warp_sum<W>(v[q]);
 }
 
-// Reduce NV values per thread across the block (sum or max per slot).
+// Reduce NV values per thread across the block of NT (sum or max per slot).
 template <int NV>
 __device__ __forceinline__ void block_reduce(double (&v)[NV], const bool (&is_max)[NV], double* sh)
 {
+    constexpr int NW = NT / 32;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int q = 0; q < NV; ++q) v[q] = is_max[q] ? warp_max(v[q]) : warp_sum(v[q]);
+    warp_reduce<NV, 32>(v, is_max);
     if (lane == 0) {
 #pragma unroll
         for (int q = 0; q < NV; ++q) sh[wid * NV + q] = v[q];
     }
     __syncthreads();
     if (wid == 0) {
-        const int nw = blockDim.x >> 5;
 #pragma unroll
-        for (int q = 0; q < NV; ++q) {
-            double a = (lane < nw) ? sh[lane * NV + q] : (is_max[q] ? 0.0 : 0.0);
-            v[q] = is_max[q] ? warp_max(a) : warp_sum(a);
-        }
+        for (int q = 0; q < NV; ++q) v[q] = lane < NW ? sh[lane * NV + q] : 0.0;
+        warp_reduce<NV, NW>(v, is_max);
     }
 }
 
@@ -93,7 +131,7 @@ __device__ bool grid_finish(double (&v)[NV], const bool (&is_max)[NV], double* p
         a[q] = 0.0;
         for (unsigned b = threadIdx.x; b < (unsigned)nblk; b += blockDim.x) {
             const double pb = ((volatile double*)partials)[(size_t)b * NV + q];
-            a[q] = is_max[q] ? fmax(a[q], pb) : a[q] + pb;
+            a[q] = is_max[q] ? max_nonneg(a[q], pb) : a[q] + pb;
         }
     }
     __syncthreads();
@@ -160,7 +198,7 @@ __device__ bool grid_finish_f(float (&vf)[NV], const bool (&is_max)[NV], double*
         a[q] = 0.0;
         for (unsigned b = threadIdx.x; b < (unsigned)nblk; b += blockDim.x) {
             const double pb = ((volatile double*)partials)[(size_t)b * NV + q];
-            a[q] = is_max[q] ? fmax(a[q], pb) : a[q] + pb;
+            a[q] = is_max[q] ? max_nonneg(a[q], pb) : a[q] + pb;
         }
     }
     __syncthreads();
@@ -620,8 +658,8 @@ __device__ __forceinline__ void ts_max_body(Dom d, const T* __restrict__ raw, do
             ts_x12(d.x[e], k, dt, x1, x2);
             d.ts_x2[e] = x2;         // kept for the error norm and the commit
             d.ts_dx[e] = x2 - x1;
-            v[0] = fmax(v[0], fabs(x1));
-            v[1] = fmax(v[1], fabs(x2));
+            v[0] = max_nonneg(v[0], x1);
+            v[1] = max_nonneg(v[1], x2);
         }
     }
     double tot[2];
@@ -950,8 +988,8 @@ __device__ __forceinline__ void dp_err_body(Dom d, const DPRaw<T>& r, double ato
             for (int q = 0; q < 7; ++q) a += c_dp_bs[q] * (((double)r.p[q][e] - cm[q]) * d.spy);
             const double x1 = d.x[e] + h * a, x2 = d.ts_x2[e];
             d.ts_dx[e] = x2 - x1;
-            v[0] = fmax(v[0], fabs(x1));
-            v[1] = fmax(v[1], fabs(x2));
+            v[0] = max_nonneg(v[0], x1);
+            v[1] = max_nonneg(v[1], x2);
         }
     } else {
         // x2 - x1 = h sum_r (a_{6 r} - bs_r) k_r in FP32; the float
