@@ -199,7 +199,12 @@ __device__ __forceinline__ void stage_fixed(const typename vec2<T>::type* __rest
 // step engine there 890 -> 740 us.)  The sums and differences are formed once,
 // in place in src, which the stage consumes.  Radix 5 and 7 keep their points
 // in registers (dft_odd): through this pass with its extra barrier a 100^2
-// update took 799 us against 711 of the direct sums, in registers 597.
+// update took 799 us against 711 of the direct sums, in registers 597.  In FP32
+// radices up to 23 form the sums and differences again for each output pair,
+// without that pass and barrier: an update of 66^2 (11) 899 -> 820 us, 190^2
+// (19) 1232 -> 1175, 92^2 (23) 895 -> 887; 116^2 (29) would take 966 against
+// 942, 122^2 (61) 1028 against 954.
+constexpr int ODD_ONE_PASS = 23;
 template <typename T, bool SH = false>
 __device__ void stage_odd(typename vec2<T>::type* __restrict__ src, typename vec2<T>::type* __restrict__ dst, int n,
                           int nl, int ls, int R, int Ns, const typename vec2<T>::type* __restrict__ tw, int sign,
@@ -210,6 +215,36 @@ __device__ void stage_odd(typename vec2<T>::type* __restrict__ src, typename vec
     const int tstep = n / (Ns * R);
     const int step = n / R;   // table stride of the R-th roots of unity
     const int hR = R / 2, nj = nl * NR;
+    if (sizeof(T) == 4 && R <= ODD_ONE_PASS) {
+        // sums and differences formed by each output pair for itself
+        for (int it = tid; it < nj * (hR + 1); it += nthr) {
+            const int q = it / nj, jl = it - q * nj;
+            const int line = jl / NR, j = jl - line * NR;
+            const C2* x = src + (size_t)line * ls + j;
+            const int jm = j % Ns;
+            C2* y = dst + (size_t)line * ls + (j - jm) * R + jm;
+            C2 P = x[0], Q = mk2<T>((T)0, (T)0);
+            int e = 0;   // r q mod R
+            for (int r = 1; r <= hR; ++r) {
+                e += q;
+                if (e >= R) e -= R;
+                const C2 w = tw_load<T, C2, SH>(tw, e * step, -1);   // (cos, -sin)
+                C2 a = x[r * NR], b = x[(R - r) * NR];
+                if (jm > 0) {
+                    a = cmul(a, tw_load<T, C2, SH>(tw, jm * r * tstep, sign));
+                    b = cmul(b, tw_load<T, C2, SH>(tw, jm * (R - r) * tstep, sign));
+                }
+                P.x += (a.x + b.x) * w.x;
+                P.y += (a.y + b.y) * w.x;
+                Q.x -= (a.x - b.x) * w.y;
+                Q.y -= (a.y - b.y) * w.y;
+            }
+            const C2 lo = mk2<T>(P.x + Q.y, P.y - Q.x), hi = mk2<T>(P.x - Q.y, P.y + Q.x);
+            y[q * Ns] = sign < 0 ? lo : hi;
+            if (q > 0) y[(R - q) * Ns] = sign < 0 ? hi : lo;
+        }
+        return;
+    }
     for (int it = tid; it < nj * hR; it += nthr) {
         const int r = it / nj + 1, jl = it - (r - 1) * nj;
         const int line = jl / NR, j = jl - line * NR;

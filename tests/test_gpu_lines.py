@@ -53,6 +53,13 @@ def test_rate_with_odd_radices(nx, ny, even, precision):
     _check_rate(nx, ny, even, precision)
 
 
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("nx,ny,even", [(66, 46, True), (46, 58, False), (76, 26, False), (136, 74, True)])
+def test_rate_with_primes_around_the_one_pass_limit(nx, ny, even, precision):
+    """11, 13, 17, 19 and 23 take one pass in the mixed form, 29 and 37 two."""
+    _check_rate(nx, ny, even, precision)
+
+
 def _check_rate(nx, ny, even, precision):
     dom, p = _domain("test1d", nx, ny, precision)
     rng = np.random.default_rng(nx + ny)
