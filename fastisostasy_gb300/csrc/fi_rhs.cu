@@ -740,9 +740,9 @@ k_flexure_f32(const double* __restrict__ y, const double* __restrict__ wref, con
 // vertical window in registers, and has some fifteen independent loads in
 // flight where column strips (a warp per 28 columns, shuffles for the
 // x-neighbours) had one row's and waited on them: 2048^2 54.1 -> 43.9 us, 512 x
-// 1024 16.8 -> 10.6 us an RK4 stage.  The tile is bound by instruction issue:
-// with cell indices divided out per element it issued 304 a cell and took
-// 50.9 us at 2048^2.
+// 1024 16.8 -> 10.6 us an RK4 stage.  It issues 224 instructions a cell and
+// keeps the issue slots 65 % busy; with cell indices divided out per element
+// it issued 304 and took 50.9 us at 2048^2.
 // The grid is even in both directions, so the last tile has two columns and
 // two rows at least, which the one-sided forms at the far edges need.
 // ---------------------------------------------------------------------------
