@@ -3033,8 +3033,10 @@ int fi_batch_autotune(fi_batch* b, int32_t* chosen4)
             for (int k = 0; k < 4; ++k) chosen4[k] = b->shape[k];
         return FI_OK;
     }
-    // the stencil of the reference stages reads now%w's float pair
-    for (fi_handle* h : b->hs) {
+    // the pairs that the stencils of the loop members read (a member with a
+    // cluster of its own is not timed, and has no dxw)
+    for (int i : b->loop) {
+        fi_handle* h = b->hs[i];
         if (h->d.whi) split_hilo(h->d.w, h->d.whi, h->d.wlo, h->n, b->s);
         if (h->yhi) split_hilo_dxw(h->d.x, h->xhi, h->xlo, h->wrefhi, h->wreflo, h->dxw, h->n, b->s);
     }
