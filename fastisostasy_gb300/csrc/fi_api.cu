@@ -28,6 +28,7 @@
 #include "fi_engine.h"
 #include "fi_init.h"
 #include "fi_kernels.h"
+#include "fi_shapes.h"
 #include "fi_batch.h"
 #include "fi_state.h"
 
@@ -2610,20 +2611,16 @@ int batch_shape(fi_batch* b, int RB, int CB, int waves)
     const size_t c2 = b->mixed ? sizeof(float2) : sizeof(double2);
     b->rows_threads = b->cols_threads = 0;
     b->rows_smem = b->cols_smem = 0;
-    // threads of a transform block: the most any member's shape asks for; a
-    // member on register lines then takes as many lines as they make
+    // threads of a transform block: the most any member's shape asks for, a
+    // power of two as all of them are; a member on register lines then takes
+    // as many lines as they make
     auto shape_of = [&](BMember& m, int& rt, int& ct) {
         m.RB = RB > 0 ? RB : rhs_rows_per_block(m.p.h);
         m.CB = CB > 0 ? CB : (b->mixed ? rhs_cols_per_block<float>(m.p.ny) : rhs_cols_per_block<double>(m.p.ny));
         const int lr = rhs_line_threads(m.p.h, m.p, b->mixed), lc = rhs_line_threads(m.p.ny, m.p, b->mixed);
         m.lines = (lr > 0 ? 1 : 0) | (lc > 0 ? 2 : 0);
-        auto line_block = [](int lines, int th) {
-            int t = lines * th;
-            while (t > 512) t /= 2;
-            return t < th ? th : t < 32 ? 32 : t;
-        };
-        rt = lr > 0 ? line_block(m.RB, lr) : rhs_threads_for(m.RB * m.p.h / 4);
-        ct = lc > 0 ? line_block(m.CB, lc) : rhs_threads_for(m.CB * m.p.ny / 4);
+        rt = lr > 0 ? line_block(m.RB, lr, 512) : rhs_threads_for(m.RB * m.p.h / 4);
+        ct = lc > 0 ? line_block(m.CB, lc, 512) : rhs_threads_for(m.CB * m.p.ny / 4);
     };
     for (int i = 0; i < n; ++i) {
         int rt, ct;

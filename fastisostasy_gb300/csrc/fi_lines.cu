@@ -4,6 +4,7 @@
 #include <mutex>
 
 #include "fi_lines.cuh"
+#include "fi_shapes.h"
 
 #ifndef FI_LINES_T   // one translation unit per precision (fi_lines64.cu)
 #define FI_LINES_T float
@@ -124,16 +125,6 @@ template <typename K> void line_smem_limit(K kern, size_t bytes, size_t* cur)
     std::lock_guard<std::mutex> lk(mu);
     if (bytes <= *cur) return;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess) *cur = bytes;
-}
-
-// Threads of a block of `lines` lines of th threads: whole warps, no more
-// than the kernel's limit.
-int line_block(int lines, int th, int most)
-{
-    int n = lines * th;
-    while (n > most) n /= 2;
-    if (n < th) n = th;
-    return n < 32 ? 32 : n;
 }
 
 }  // namespace

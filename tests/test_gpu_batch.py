@@ -67,3 +67,21 @@ def check(sizes, precision, stage_mode, autotune):
 def test_cluster_members_beside_loop_members(stage_mode, autotune):
     """64^2 and 128^2 fit a cluster, 384^2 (register lines) and 200^2 (none) do not."""
     check([(64, 64), (384, 384), (128, 128), (200, 200)], 1, stage_mode, autotune)
+
+
+@pytest.mark.parametrize("autotune", [False, True])
+def test_fp64_members_on_lines_of_three_times_a_power(autotune):
+    """Row lines of 8, 16 and 32 threads in one block (96, 192 and 384 points,
+    each on a grid large enough for FP64 lines of that kind)."""
+    check([(192, 1368), (384, 684), (768, 342)], 0, 0, autotune)
+
+
+@pytest.mark.parametrize("rows,cols", [(3, 5), (5, 3), (1, 1), (16, 16), (7, 6)])
+@pytest.mark.parametrize("precision,sizes", [(0, [(64, 2048), (128, 64), (40, 48)]),
+                                             (1, [(64, 2048), (512, 256), (384, 384), (200, 200)])])
+def test_any_rows_and_columns_a_block(monkeypatch, precision, sizes, rows, cols):
+    """Block shapes asked for by the environment that are no powers of two, over
+    lines of different lengths."""
+    monkeypatch.setenv("FI_BATCH_RB", str(rows))
+    monkeypatch.setenv("FI_BATCH_CB", str(cols))
+    check(sizes, precision, 0, False)
