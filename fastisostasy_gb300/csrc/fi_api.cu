@@ -2194,11 +2194,13 @@ int fi_metrics_json(fi_handle* h, char* buf, size_t len)
     const int n = snprintf(buf, len,
                            "{\"nx\": %d, \"ny\": %d, \"nx_ice\": %d, \"ny_ice\": %d, \"precision\": \"%s\", "
                            "\"method\": %d, \"dt_method\": %d, \"stage_mode\": %d, \"step_engine\": %s, "
+                           "\"stepper\": \"%s\", "
                            "\"updates\": %lld, \"t\": %.17g, \"dt\": %.17g, \"n_accept\": %lld, \"n_reject\": %lld, "
                            "\"n_attempt\": %lld, \"kernels_enqueued\": %lld, \"graphs_captured\": %d, "
                            "\"host_update_ms\": %.6f, \"status\": %d}",
                            h->nx, h->ny, h->nx_ice, h->ny_ice, mixed(h) ? "mixed" : "fp64", p.method, p.dt_method,
-                           p.stage_mode, h->engine_ok || h->clu_ok ? "true" : "false", h->updates, hc.t, hc.dt, hc.n_accept,
+                           p.stage_mode, h->engine_ok || h->clu_ok ? "true" : "false",
+                           h->clu_ok ? "cluster" : h->engine_ok ? "engine" : "kernels", h->updates, hc.t, hc.dt, hc.n_accept,
                            hc.n_reject, hc.n_attempt, h->launches, (int)h->graphs.size(), 1e3 * h->host_update_s,
                            hc.status);
     return (n < 0 || (size_t)n >= len) ? FI_E_SIZE : FI_OK;

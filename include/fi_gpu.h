@@ -167,9 +167,12 @@ int fi_update_async(fi_handle* h, const double* d_H_ice, double time, fi_bsl* bs
 int fi_synchronize(fi_handle* h);
 /* Run metrics of a handle (no reference counterpart; the reference has no
  * instrumentation beyond gprof): one JSON object, NUL-terminated, in buf —
- * grid, form, integrator, updates made, model time and step, accepted and
- * rejected steps, adaptive attempts (tsit54), kernels enqueued, CUDA graphs
- * captured, host time inside the update calls, device status.  Waits for
+ * grid, form, integrator, what makes its steps ("stepper": "cluster", one
+ * thread-block cluster; "engine", the grid-wide step engine; "kernels", one
+ * kernel a pass; "step_engine" is true for the first two), updates made, model
+ * time and step, accepted and rejected steps, adaptive attempts (tsit54),
+ * kernels enqueued, CUDA graphs captured, host time inside the update calls,
+ * device status.  Waits for
  * the handle's stream.  FI_E_SIZE when len is too small (1 KiB suffices).
  * With the environment variable FI_METRICS_FILE set, fi_destroy appends
  * this line to that file (a per-run metrics sink).  The host API calls

@@ -33,9 +33,10 @@ def ensemble_w(wls, precision, autotune):
         ens.update(t)
     ens.synchronize()
     w = [d.field("w") for d in ens.doms]
+    steppers = [d.metrics()["stepper"] for d in ens.doms]
     counts = [(d.scalars()["n_accept"], d.scalars()["n_reject"]) for d in ens.doms]
     ens.close()
-    return w, counts
+    return w, counts, steppers
 
 
 def alone_w(wl, precision):
@@ -50,9 +51,10 @@ def alone_w(wl, precision):
     return w, (sc["n_accept"], sc["n_reject"])
 
 
-def check(sizes, precision, stage_mode, autotune):
+def check(sizes, precision, stage_mode, autotune, clustered=False):
     wls = [member(nx, ny, stage_mode) for nx, ny in sizes]
-    got, counts = ensemble_w(wls, precision, autotune)
+    got, counts, steppers = ensemble_w(wls, precision, autotune)
+    assert "kernels" in steppers and (precision == 0 or not clustered or "cluster" in steppers)
     for wl, g, c in zip(wls, got, counts):
         w, ca = alone_w(wl, precision)
         assert c == ca and np.abs(w).max() > 0, wl.name
@@ -66,7 +68,7 @@ def check(sizes, precision, stage_mode, autotune):
 @pytest.mark.parametrize("stage_mode", [0, 1])
 def test_cluster_members_beside_loop_members(stage_mode, autotune):
     """64^2 and 128^2 fit a cluster, 384^2 (register lines) and 200^2 (none) do not."""
-    check([(64, 64), (384, 384), (128, 128), (200, 200)], 1, stage_mode, autotune)
+    check([(64, 64), (384, 384), (128, 128), (200, 200)], 1, stage_mode, autotune, clustered=True)
 
 
 @pytest.mark.parametrize("autotune", [False, True])
@@ -85,3 +87,11 @@ def test_any_rows_and_columns_a_block(monkeypatch, precision, sizes, rows, cols)
     monkeypatch.setenv("FI_BATCH_RB", str(rows))
     monkeypatch.setenv("FI_BATCH_CB", str(cols))
     check(sizes, precision, 0, False)
+
+
+@pytest.mark.parametrize("autotune", [False, True])
+@pytest.mark.parametrize("stage_mode", [0, 1])
+def test_small_members_in_the_loop(monkeypatch, stage_mode, autotune):
+    """Members that would fit a cluster, batched (and driven alone) without it."""
+    monkeypatch.setenv("FI_NO_CLUSTER", "1")
+    check([(40, 40), (56, 34), (192, 192), (128, 96)], 1, stage_mode, autotune)

@@ -1,0 +1,57 @@
+"""Which of the three steppers a mixed domain takes (one thread-block cluster,
+the grid-wide step engine, one kernel a pass), and the step engine against the
+oracle on each of its forms: register lines in its phases, and shared-memory
+stages for lengths without one.
+
+The bound is the mixed form's, 1e-5 of the largest displacement.
+"""
+import pytest
+
+from fastisostasy_gb300.isostasy import Domain
+from harness import Pair, rel
+from test_gpu_cluster import workload
+
+pytestmark = pytest.mark.gpu
+RK4, TSIT, TSIT_TRUE = dict(dt_method=1), dict(dt_method=2, stage_mode=0), dict(dt_method=2, stage_mode=1)
+SMALL = [(16, 16), (18, 18), (34, 34), (50, 50), (64, 64), (48, 80), (96, 96), (64, 20), (256, 32), (32, 256), (128, 192),
+         (192, 128), (384, 48), (192, 192), (128, 128)]
+
+
+@pytest.mark.parametrize("stepper,par,sizes", [
+    ("cluster", RK4, SMALL), ("cluster", TSIT, SMALL + [(256, 256)]), ("cluster", TSIT_TRUE, SMALL + [(256, 256)]),
+    ("engine", RK4, [(256, 256), (80, 60), (100, 100), (200, 200), (384, 384), (512, 512), (32, 512), (512, 128)]),
+    ("kernels", RK4, [(64, 1024), (1024, 512), (640, 640)]),
+    ("kernels", TSIT_TRUE, [(100, 100), (200, 200), (384, 384), (512, 128)]),
+], ids=["cluster-rk4", "cluster-tsit54", "cluster-tsit54-true", "engine-rk4", "kernels-rk4", "kernels-tsit54-true"])
+def test_stepper_of_a_size(stepper, par, sizes):
+    for nx, ny in sizes:
+        wl = workload(nx, ny, 1, True, **par)
+        dom = Domain(wl.params, nx, ny, wl.dx, precision=1)
+        assert dom.metrics()["stepper"] == stepper, (nx, ny)
+        dom.close()
+
+
+def check_engine(nx, ny, even):
+    pair = Pair(workload(nx, ny, 5 * nx + ny, even), precision=1)
+    m = pair.dom.metrics()
+    assert m["stepper"] == "engine" and m["step_engine"]
+    pair.init()
+    pair.step(2)
+    assert pair.dom.scalars()["t"] == pair.t and pair.dom.scalars()["n_accept"] == 20
+    for f in ("w", "z_bed"):
+        assert rel(pair.dom.field(f), pair.orc.field(f)) <= 1e-5
+    assert rel(pair.dom.field("dwdt"), pair.orc.field("dwdt")) <= 1e-4
+    pair.close()
+
+
+@pytest.mark.parametrize("even", [True, False])
+@pytest.mark.parametrize("nx,ny", [(256, 256), (384, 256), (256, 384), (384, 384), (512, 384), (384, 512)])
+def test_engine_on_lines(nx, ny, even):
+    check_engine(nx, ny, even)
+
+
+@pytest.mark.parametrize("nx,ny", [(50, 50), (66, 46), (100, 100), (122, 98), (76, 140), (200, 200), (464, 466)])
+def test_engine_without_lines(monkeypatch, nx, ny):
+    """Shared-memory stages, radices 5, 7 and larger primes among them, two and four rows a block."""
+    monkeypatch.setenv("FI_NO_CLUSTER", "1")
+    check_engine(nx, ny, nx != 100)
