@@ -28,7 +28,7 @@ def _nvcc():
 
 def sources():
     """Translation units, the longest to compile first."""
-    slow = ("fi_cluster_", "fi_rhs", "fi_lines")
+    slow = ("fi_cluster_", "fi_rhs", "fi_engine", "fi_lines")
     return sorted(glob.glob(os.path.join(CSRC, "*.cu")),
                   key=lambda p: (not os.path.basename(p).startswith(slow), p))
 

@@ -249,7 +249,7 @@ struct fi_handle {
     bool clu_ok = false;
     int clu_mode = 0, clu_nc = 0, clu_threads = 0, clu_stages = 0;
     size_t clu_smem = 0;
-    int eng_grid = 0, eng_CB = 1, eng_RA = 2, eng_P2 = 0;
+    int eng_grid = 0, eng_CB = 1, eng_RA = 2;
     size_t eng_smem = 0;
     float *xhi = nullptr, *xlo = nullptr, *wrefhi = nullptr, *wreflo = nullptr;
     float* dxw = nullptr;   // (xhi - wrefhi) + (xlo - wreflo): the kernel sequence's mixed RK4 stages
@@ -1152,7 +1152,6 @@ template <typename T> T* enqueue_engine(fi_handle* h, int nsteps)
     g.nsteps = nsteps;
     g.CB = h->eng_CB;
     g.ra = h->eng_RA;
-    g.p2 = h->eng_P2;
     g.spy = h->spy;
     g.norm_scale = 1.0 / (double)(float)((long long)h->nx * h->ny);
     g.norm_scale_f = (float)g.norm_scale;
@@ -1872,9 +1871,8 @@ int fi_create_handle(const fi_params* pin, int nx_ice, int ny_ice, double dx, do
         if ((want || tsit_any) && mixed(h) && !is_set("FI_NO_CLUSTER") && !is_set("FI_ENGINE_RA") &&
             !is_set("FI_ENGINE_BARRIER_PHANTOM")) {
             // RK4: from 256^2 on the grid-wide step engine is the faster one
-            // where both lengths have its line phases (256^2: 478 against 540
-            // us an update of ten steps; 192^2: 451 in the cluster, 620 of the
-            // engine without them)
+            // where both lengths have its line phases (256^2: 475 against 540
+            // us an update of ten steps; 192^2: 508 against 451 in the cluster)
             const bool grid_wide = p.dt_method == 1 && h->n >= 65536 && engine_has_lines(h->prhs);
             h->clu_mode = p.dt_method == 1 ? CLU_RK4 : p.stage_mode == 1 ? CLU_TSIT_TRUE : CLU_TSIT;
             h->clu_ok = !grid_wide && cluster_config(h->prhs, h->clu_mode, &h->clu_nc, &h->clu_threads, &h->clu_stages,
@@ -1883,10 +1881,8 @@ int fi_create_handle(const fi_params* pin, int nx_ice, int ny_ice, double dx, do
             if (h->clu_ok) { AL2(h->mAT, nk * tsz(h)); AL2(h->mBT, nk * tsz(h)); }
         }
         if (want && !h->clu_ok) {
-            int ok = mixed(h) ? engine_config<float>(h->prhs, &h->eng_grid, &h->eng_CB, &h->eng_smem, &h->eng_RA,
-                                                  &h->eng_P2)
-                              : engine_config<double>(h->prhs, &h->eng_grid, &h->eng_CB, &h->eng_smem, &h->eng_RA,
-                                                      &h->eng_P2);
+            int ok = mixed(h) ? engine_config<float>(h->prhs, &h->eng_grid, &h->eng_CB, &h->eng_smem, &h->eng_RA)
+                              : engine_config<double>(h->prhs, &h->eng_grid, &h->eng_CB, &h->eng_smem, &h->eng_RA);
             h->engine_ok = ok != 0;
             cudaGetLastError();
             if (h->engine_ok) {

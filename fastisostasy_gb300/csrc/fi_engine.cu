@@ -27,6 +27,14 @@
 #include "fi_engine.h"
 #include "fi_lines.cuh"
 
+// Translation units: the host code and the kernels on shared-memory stages
+// (0, this file), those on register lines (1, fi_engine_lines.cu), of grids
+// wider than a block (2, fi_engine_wide.cu) and with short lines (3,
+// fi_engine_short.cu).
+#ifndef FI_ENGINE_PART
+#define FI_ENGINE_PART 0
+#endif
+
 namespace cg = cooperative_groups;
 
 namespace fi {
@@ -50,8 +58,19 @@ template <int RA> struct EngShape {
     static constexpr int cb = RA == 4 ? 2 : 1;       // spectrum columns per phase-B item
 };
 
+// Form of a kernel (FM): transforms by shared-memory stages of any radix
+// (FFT_ANY) or of radices 2, 3, 4 and 8 only (FFT_23), or on register lines
+// (FFT_LINES, see phase_a_lines).  A kernel on lines has the lengths of one
+// kind: rows (columns) of 2^k or with FFT_ROW3 (FFT_COL3) of 3 2^k points, both
+// from SHORT_LINE points on or with FFT_SHORT any, and grids no wider or with
+// FFT_WIDE wider than its block.  What a domain does not need costs it
+// registers and instruction cache (an update of ten steps, all lengths in one
+// kernel / the 2^k ones / those from 128 points: 512^2 668 / 653 / 645 us,
+// 256^2 505 / 494 / 471; 324^2 with / without the odd radices 973 / 942).
+enum { FFT_ANY = 0, FFT_LINES = 1, FFT_ROW3 = 2, FFT_COL3 = 4, FFT_WIDE = 8, FFT_SHORT = 16, FFT_23 = 32 };
+
 // stage coefficients of RK4: y_s = x + a_s h k_{s-1}
-__constant__ double c_rk4_a[4] = {0.0, 0.5, 0.5, 1.0};
+static __constant__ double c_rk4_a[4] = {0.0, 0.5, 0.5, 1.0};
 
 template <typename T, int RA> struct PhaseAMem {
     // level-0 differences on RA+4 rows, moments on RA+2 rows, all full width
@@ -136,7 +155,7 @@ __device__ __forceinline__ unsigned long long gtimer()
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-__shared__ int s_trk;
+static __shared__ int s_trk;
 constexpr int kTraceLen = 256;
 __device__ __forceinline__ void tmark(unsigned long long* tr)
 {
@@ -146,7 +165,7 @@ __device__ __forceinline__ void tmark(unsigned long long* tr)
 // ---------------------------------------------------------------------------
 // Phase A: one item = output rows j0 .. j0+RA-1 (full width).
 // ---------------------------------------------------------------------------
-template <typename T, int RA>
+template <typename T, int RA, int FM>
 __device__ void phase_a(const EngineArgs& g, int j0, int stage, float sdf_in, unsigned char* smem,
                         const EngTw<T>& tw)
 {
@@ -288,7 +307,7 @@ __device__ void phase_a(const EngineArgs& g, int j0, int stage, float sdf_in, un
     }
     __syncthreads();
     tmark(g.trace);
-    C2* r = block_fft<T, true>(b0, b1, g.p.row.d, RA, hh, tw.row, -1);
+    C2* r = block_fft<T, true, FM == FFT_ANY>(b0, b1, g.p.row.d, RA, hh, tw.row, -1);
     const C2* rtw = tw.rtw;
     // column-major: the strided stores do not hold the block up, and phase B
     // then reads each spectrum column contiguously
@@ -314,7 +333,7 @@ __device__ void phase_a(const EngineArgs& g, int j0, int stage, float sdf_in, un
 // inverse column FFT.  Columns come contiguous from the column-major copy
 // phase A wrote; the result goes back row-major for the row passes of C.
 // ---------------------------------------------------------------------------
-template <typename T>
+template <typename T, int FM>
 __device__ void phase_b(const EngineArgs& g, int k0, int CB, unsigned char* smem, const EngTw<T>& tw)
 {
     typedef typename vec2<T>::type C2;
@@ -330,7 +349,7 @@ __device__ void phase_b(const EngineArgs& g, int k0, int CB, unsigned char* smem
     }
     __syncthreads();
     tmark(g.trace);
-    C2* r = block_fft<T, true>(b0, b1, g.p.col.d, CB, ny, tw.col, -1);
+    C2* r = block_fft<T, true, FM == FFT_ANY>(b0, b1, g.p.col.d, CB, ny, tw.col, -1);
     const T* mA = g.mA_T<T>();
     const T* mB = g.mB_T<T>();
     const int half = ny / 2 + 1;
@@ -366,7 +385,7 @@ __device__ void phase_b(const EngineArgs& g, int k0, int CB, unsigned char* smem
     __syncthreads();
     tmark(g.trace);
     C2* other = (r == b0) ? b1 : b0;
-    C2* q = block_fft<T, true>(r, other, g.p.col.d, CB, ny, tw.col, +1);
+    C2* q = block_fft<T, true, FM == FFT_ANY>(r, other, g.p.col.d, CB, ny, tw.col, +1);
     for (int e = tid; e < CB * ny; e += nt) {
         const int c = CB == 1 ? 0 : e % CB, l = CB == 1 ? e : e / CB;
         const int k = k0 + c;
@@ -379,7 +398,7 @@ __device__ void phase_b(const EngineArgs& g, int k0, int CB, unsigned char* smem
 // ---------------------------------------------------------------------------
 // Phase C: inverse row real-FFT of rows j0 .. j0+RC-1 -> raw (scaled 1/(nx ny)).
 // ---------------------------------------------------------------------------
-template <typename T, int RC>
+template <typename T, int RC, int FM>
 __device__ void phase_c(const EngineArgs& g, int j0, T* out, unsigned char* smem, const EngTw<T>& tw)
 {
     typedef typename vec2<T>::type C2;
@@ -405,7 +424,7 @@ __device__ void phase_c(const EngineArgs& g, int j0, T* out, unsigned char* smem
     }
     __syncthreads();
     tmark(g.trace);
-    C2* r = block_fft<T, true>(b0, b1, g.p.row.d, RC, hh, tw.row, +1);
+    C2* r = block_fft<T, true, FM == FFT_ANY>(b0, b1, g.p.row.d, RC, hh, tw.row, +1);
     T scale;
     if constexpr (std::is_same<T, float>::value) scale = g.norm_scale_f;
     else scale = g.norm_scale;
@@ -422,50 +441,91 @@ __device__ void phase_c(const EngineArgs& g, int j0, T* out, unsigned char* smem
 }
 
 // ---------------------------------------------------------------------------
-// The phases where both lengths have a register line (FM == FFT_LINES): rows
+// The phases where both lengths have a register line (FM & FFT_LINES): rows
 // transform in their warps, a column pair on its own few warps under a named
 // barrier, points in registers from the load to the store; the stencil is two
 // passes over the stage state's float pair (moments, then f), each thread
 // walking down a column, instead of five over its differences.  An update of
-// ten RK4 steps at 512^2 897 -> 660 us, at 256^2 600 -> 478.
+// ten RK4 steps at 512^2 897 -> 645 us, at 256^2 604 -> 471, at 128 x 512 647 ->
+// 519, at 512 x 128 857 -> 528.
 // ---------------------------------------------------------------------------
-enum { FFT_ANY = 0, FFT_LINES = 1 };   // FM
 
+// Lengths of the line phases: every even 2^k and 3 2^k that the engine's rows
+// and columns come to (beyond 512 points its stencil phase does not fit a wave
+// of blocks, or a block's shared memory).
+#define FI_ENGINE_LINES(FN) \
+    FN(2) FN(4) FN(6) FN(8) FN(12) FN(16) FN(24) FN(32) FN(48) FN(64) FN(96) FN(128) FN(192) FN(256) FN(384) FN(512)
+inline bool engine_line(int n)
+{
+#define FI_IS(N) || n == N
+    return false FI_ENGINE_LINES(FI_IS);
+#undef FI_IS
+}
+// Row and column lengths of a kernel.  Four-row items: columns from the length
+// on that engine_config takes them for, rows up to 384 points (768 x 512: 1555
+// us a coupling step against 2080 on shared-memory stages; 1024 x 512 took 1833
+// against 1690 of the kernel sequence).
+constexpr int SHORT_LINE = 128;
+constexpr bool engine_row(int n, int ra, int fm)
+{
+    const bool wide = ra == 2 && 2 * n > EngShape<2>::threads;
+    return (n % 3 == 0) == ((fm & FFT_ROW3) != 0) && wide == ((fm & FFT_WIDE) != 0) && (ra == 2 || n <= 384) &&
+           ((fm & (FFT_SHORT | FFT_WIDE)) || n >= SHORT_LINE);
+}
+constexpr bool engine_col(int n, int ra, int fm)
+{
+    return (n % 3 == 0) == ((fm & FFT_COL3) != 0) && (ra == 2 || n > 400) &&
+           ((fm & (FFT_SHORT | FFT_WIDE)) || n >= SHORT_LINE);
+}
+// Lines of n points that are transformed together, `want` at least: whole
+// warps work on them, so short lines share one (some then hold no row or
+// column; they have their room all the same).
+__host__ __device__ constexpr int line_group(int n, int want)
+{
+    const int th = n / line_points(n, true), w = th < 32 ? 32 / th : 1;
+    return w > want ? w : want;
+}
 template <int RA> __host__ __device__ inline size_t lines_a_bytes(int nx)
 {
     return ((size_t)2 * (RA + 4) + 3 * (RA + 2)) * nx * sizeof(float);
 }
 template <int RA> __host__ __device__ inline size_t lines_tab_off(int nx, int h, int ny, int CB)
 {
-    const size_t a = lines_a_bytes<RA>(nx) + (size_t)RA * line_room(h, true) * sizeof(float2);
+    const size_t a = lines_a_bytes<RA>(nx) + (size_t)line_group(h, RA) * line_room(h, true) * sizeof(float2);
     const size_t b = (size_t)CB * line_room(ny, true) * sizeof(float2);
     return ((a > b ? a : b) + 15) & ~(size_t)15;
 }
-// row and column lengths of the line phases (their instances below)
-inline bool engine_line_rows(int h) { return h == 128 || h == 192 || h == 256; }
-inline bool engine_line_cols(int n) { return n == 256 || n == 384 || n == 512; }
+// barrier among `lines` lines of th threads: their warp's, or a named one
+constexpr int line_barrier(int lines, int th) { return th <= 32 ? 1 : lines * th; }
 
 template <int RA, int H>
 __device__ __forceinline__ void engine_rows_fwd(float2* zb, const EngTw<float>& tw)
 {
     constexpr int E = LineShape<float, H>::E, TH = LineShape<float, H>::threads, ROOM = line_smem<float, H>();
+    constexpr int LR = line_group(H, RA), SY = line_barrier(LR, TH);
+    if ((int)threadIdx.x >= LR * TH) return;   // whole warps
     const int line = threadIdx.x / TH, t = threadIdx.x % TH;
-    if (line >= RA) return;   // whole warps
     float2* b = zb + (size_t)line * ROOM;
     float2 v[E];
 #pragma unroll
     for (int m = 0; m < E; ++m) v[m] = b[t + TH * m];
-    line_fft<float, H, -1, 1, true>(v, b, tw.row, t);
-    __syncwarp();
+    line_fft<float, H, -1, SY, true>(v, b, tw.row, t);
+    line_sync<SY>();
 #pragma unroll
     for (int m = 0; m < E; ++m) b[line_pad<E>(t + TH * m)] = v[m];
 }
 
-template <int RA> __device__ void phase_a_lines(const EngineArgs& g, int j0, int stage, float sdf, unsigned char* smem,
-                                                const EngTw<float>& tw)
+template <int RA, int FM>
+__device__ void phase_a_lines(const EngineArgs& g, int j0, int stage, float sdf, unsigned char* smem,
+                              const EngTw<float>& tw)
 {
     const int nx = g.p.nx, ny = g.p.ny, hh = g.p.h;
-    const int tid = threadIdx.x, ngrp = (int)blockDim.x / nx, grp = tid / nx, i = tid - grp * nx;
+    // a thread keeps its column, or every blockDim.x-th one of a grid wider
+    // than the block (only two-row blocks meet one: four-row ones have 1024 threads)
+    constexpr bool WIDE = (FM & FFT_WIDE) != 0;
+    const int tid = threadIdx.x, ngrp = WIDE ? 1 : (int)blockDim.x / nx, grp = WIDE ? 0 : tid / nx;
+    const int i0 = tid - grp * nx, iend = grp < ngrp ? nx : 0;
+#define FI_COLUMNS(i) for (int i = i0; i < iend; i = WIDE ? i + (int)blockDim.x : iend)   // of this thread
     float* yh = reinterpret_cast<float*>(smem);
     float* yl = yh + (RA + 4) * nx;
     float* Mxx = yl + (RA + 4) * nx;
@@ -483,7 +543,7 @@ template <int RA> __device__ void phase_a_lines(const EngineArgs& g, int j0, int
         for (int c = 0; c < 4; ++c) asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(cf[c]) : "l"(q[c]));
     }
     // the stage state x + sdf raw as a float pair, rows j0 - 2 .. j0 + RA + 1
-    if (grp < ngrp) {
+    FI_COLUMNS(i) {
 #pragma unroll
         for (int q = 0; q < RA + 4; ++q) {
             const int r = grp + q * ngrp, gj = j0 - 2 + r;
@@ -505,11 +565,10 @@ template <int RA> __device__ void phase_a_lines(const EngineArgs& g, int j0, int
     if (tid == 0) s_cmf = rprev ? (float)corner_mean((double)cf[0], (double)cf[1], (double)cf[2], (double)cf[3]) : 0.f;
     __syncthreads();
     tmark(g.trace);
-    const bool left = i == 0, right = i == nx - 1;
-    const int ic = left ? 1 : right ? nx - 2 : i;       // centre of the second differences in x
-    const int il = left ? 0 : i - 1, ir = right ? nx - 1 : i + 1;
-    const float cx = left || right ? g.fcf.inv_dx : g.fcf.inv_2dx;
-    if (grp < ngrp) {
+    FI_COLUMNS(i) {
+        const bool left = i == 0, right = i == nx - 1;
+        const int ic = left ? 1 : right ? nx - 2 : i;       // centre of the second differences in x
+        const float cx = left || right ? g.fcf.inv_dx : g.fcf.inv_2dx;
         // moments of grid rows j0 - 1 .. j0 + RA; one-sided second differences
         // are the central ones one cell inside
         const int run = (RA + 2 + ngrp - 1) / ngrp;
@@ -554,7 +613,11 @@ template <int RA> __device__ void phase_a_lines(const EngineArgs& g, int j0, int
     }
     __syncthreads();
     tmark(g.trace);
-    if (grp < ngrp) {
+    FI_COLUMNS(i) {
+        const bool left = i == 0, right = i == nx - 1;
+        const int ic = left ? 1 : right ? nx - 2 : i;
+        const int il = left ? 0 : i - 1, ir = right ? nx - 1 : i + 1;
+        const float cx = left || right ? g.fcf.inv_dx : g.fcf.inv_2dx;
         const float cmd = sdf * s_cmf;
         const int run = (RA + ngrp - 1) / ngrp;
         const int oa = grp * run, ob = oa + run < RA ? oa + run : RA;
@@ -587,9 +650,9 @@ template <int RA> __device__ void phase_a_lines(const EngineArgs& g, int j0, int
     __syncthreads();
     tmark(g.trace);
     switch (hh) {
-    case 128: engine_rows_fwd<RA, 128>(zb, tw); break;
-    case 192: engine_rows_fwd<RA, 192>(zb, tw); break;
-    case 256: engine_rows_fwd<RA, 256>(zb, tw); break;
+#define FI_GO(N) case N: if constexpr (engine_row(N, RA, FM)) engine_rows_fwd<RA, N>(zb, tw); break;
+        FI_ENGINE_LINES(FI_GO)
+#undef FI_GO
     }
     __syncthreads();
     tmark(g.trace);
@@ -619,13 +682,15 @@ template <int RA> __device__ void phase_a_lines(const EngineArgs& g, int j0, int
     tmark(g.trace);
 }
 
-template <int CB, int N>
+#undef FI_COLUMNS
+
+template <int RA, int N>
 __device__ __forceinline__ void engine_cols(const EngineArgs& g, int k0, unsigned char* smem, const EngTw<float>& tw)
 {
     constexpr int E = LineShape<float, N>::E, TH = LineShape<float, N>::threads, ROOM = line_smem<float, N>();
-    constexpr int SY = CB * TH;
+    constexpr int CB = line_group(N, EngShape<RA>::cb), SY = CB * TH;
     static_assert(SY % 32 == 0, "whole warps");
-    if ((int)threadIdx.x >= SY) return;   // whole warps
+    if ((int)threadIdx.x >= SY) return;
     const int c = threadIdx.x % CB, t = threadIdx.x / CB, k = k0 + c;
     const bool live = k <= g.p.h;
     float2* b = reinterpret_cast<float2*>(smem) + (size_t)c * ROOM;
@@ -667,12 +732,13 @@ __device__ __forceinline__ void engine_cols(const EngineArgs& g, int k0, unsigne
     for (int m = 0; m < E; ++m) S[(size_t)(t + TH * m) * g.p.sp + k] = v[m];
 }
 
-template <int CB> __device__ void phase_b_lines(const EngineArgs& g, int k0, unsigned char* smem, const EngTw<float>& tw)
+template <int RA, int FM>
+__device__ void phase_b_lines(const EngineArgs& g, int k0, unsigned char* smem, const EngTw<float>& tw)
 {
     switch (g.p.ny) {
-    case 256: engine_cols<CB, 256>(g, k0, smem, tw); break;
-    case 384: engine_cols<CB, 384>(g, k0, smem, tw); break;
-    case 512: engine_cols<CB, 512>(g, k0, smem, tw); break;
+#define FI_GO(N) case N: if constexpr (engine_col(N, RA, FM)) engine_cols<RA, N>(g, k0, smem, tw); break;
+        FI_ENGINE_LINES(FI_GO)
+#undef FI_GO
     }
     __syncthreads();
     tmark(g.trace);
@@ -683,26 +749,27 @@ __device__ __forceinline__ void engine_rows_inv(const EngineArgs& g, int j0, flo
                                                 const EngTw<float>& tw)
 {
     constexpr int E = LineShape<float, H>::E, TH = LineShape<float, H>::threads, ROOM = line_smem<float, H>();
+    constexpr int LR = line_group(H, RC), SY = line_barrier(LR, TH);
+    if ((int)threadIdx.x >= LR * TH) return;   // whole warps
     const int line = threadIdx.x / TH, t = threadIdx.x % TH, j = j0 + line;
-    if (line >= RC) return;   // whole warps
-    const bool live = j < g.p.ny;
+    const bool live = line < RC && j < g.p.ny;
     const float2* X = (const float2*)g.S + (size_t)(live ? j : 0) * g.p.sp;
     float2 v[E];
-    line_rows_inv<float, H, 1, true>([&](int k) { return X[k]; }, v, reinterpret_cast<float2*>(smem) + (size_t)line * ROOM,
-                                     tw.row, tw.rtw, t, live);
+    line_rows_inv<float, H, SY, true>([&](int k) { return X[k]; }, v, reinterpret_cast<float2*>(smem) + (size_t)line * ROOM,
+                                      tw.row, tw.rtw, t, live);
     if (!live) return;
 #pragma unroll
     for (int m = 0; m < E; ++m)
         *reinterpret_cast<float2*>(out + (size_t)j * g.p.nx + 2 * (t + TH * m)) = cscale(v[m], g.norm_scale_f);
 }
 
-template <int RC> __device__ void phase_c_lines(const EngineArgs& g, int j0, float* out, unsigned char* smem,
-                                                const EngTw<float>& tw)
+template <int RC, int FM>
+__device__ void phase_c_lines(const EngineArgs& g, int j0, float* out, unsigned char* smem, const EngTw<float>& tw)
 {
     switch (g.p.h) {
-    case 128: engine_rows_inv<RC, 128>(g, j0, out, smem, tw); break;
-    case 192: engine_rows_inv<RC, 192>(g, j0, out, smem, tw); break;
-    case 256: engine_rows_inv<RC, 256>(g, j0, out, smem, tw); break;
+#define FI_GO(N) case N: if constexpr (engine_row(N, RC, FM)) engine_rows_inv<RC, N>(g, j0, out, smem, tw); break;
+        FI_ENGINE_LINES(FI_GO)
+#undef FI_GO
     }
     __syncthreads();
     tmark(g.trace);
@@ -745,8 +812,6 @@ __device__ __forceinline__ bool grid_barrier(const EngineArgs& g, unsigned& targ
     return s_bar_ok != 0;
 }
 
-// FM: FFT_LINES where both transform lengths have a line phase, else FFT_ANY
-// (shared-memory stages)
 template <typename T, int RA, int FM>
 __global__ void __launch_bounds__(EngShape<RA>::threads, EngShape<RA>::per_sm) k_engine_rk4(EngineArgs g)
 {
@@ -772,7 +837,7 @@ __global__ void __launch_bounds__(EngShape<RA>::threads, EngShape<RA>::per_sm) k
     typedef typename vec2<T>::type C2;
     EngTw<T> tw;
     {
-        C2* tab = reinterpret_cast<C2*>(smem + (FM == FFT_LINES ? lines_tab_off<RA>(nx, g.p.h, ny, g.CB)
+        C2* tab = reinterpret_cast<C2*>(smem + ((FM & FFT_LINES) ? lines_tab_off<RA>(nx, g.p.h, ny, g.CB)
                                                                  : engine_tab_off<T, RA>(nx, g.p.h, ny, g.CB)));
         const C2* srow = etw<T>(g.p.row);
         const C2* scol = etw<T>(g.p.col);
@@ -825,22 +890,22 @@ __global__ void __launch_bounds__(EngShape<RA>::threads, EngShape<RA>::per_sm) k
         TRACE();
         for (int stage = 0; stage < 4; ++stage) {
             for (int it = blockIdx.x; it < na; it += gridDim.x) {
-                if constexpr (FM == FFT_LINES) phase_a_lines<RA>(g, it * RA, stage, s_sdf[stage], smem, tw);
-                else phase_a<T, RA>(g, it * RA, stage, s_sdf[stage], smem, tw);
+                if constexpr (FM & FFT_LINES) phase_a_lines<RA, FM>(g, it * RA, stage, s_sdf[stage], smem, tw);
+                else phase_a<T, RA, FM>(g, it * RA, stage, s_sdf[stage], smem, tw);
             }
             TRACE();
             if (!grid_barrier(g, bar_target)) return;
             TRACE();
             for (int it = blockIdx.x; it < nb; it += gridDim.x) {
-                if constexpr (FM == FFT_LINES) phase_b_lines<EngShape<RA>::cb>(g, it * g.CB, smem, tw);
-                else phase_b<T>(g, it * g.CB, g.CB, smem, tw);
+                if constexpr (FM & FFT_LINES) phase_b_lines<RA, FM>(g, it * g.CB, smem, tw);
+                else phase_b<T, FM>(g, it * g.CB, g.CB, smem, tw);
             }
             TRACE();
             if (!grid_barrier(g, bar_target)) return;
             TRACE();
             for (int it = blockIdx.x; it < nc; it += gridDim.x) {
-                if constexpr (FM == FFT_LINES) phase_c_lines<RC>(g, it * RC, (float*)g.raw[stage], smem, tw);
-                else phase_c<T, RC>(g, it * RC, (T*)g.raw[stage], smem, tw);
+                if constexpr (FM & FFT_LINES) phase_c_lines<RC, FM>(g, it * RC, (float*)g.raw[stage], smem, tw);
+                else phase_c<T, RC, FM>(g, it * RC, (T*)g.raw[stage], smem, tw);
             }
             TRACE();
             if (!grid_barrier(g, bar_target)) return;
@@ -901,6 +966,42 @@ __global__ void __launch_bounds__(EngShape<RA>::threads, EngShape<RA>::per_sm) k
 #undef TRACE
 }
 
+#define FI_KERNEL(RA, FM) \
+    if (ra == RA && fm == (FM)) return k_engine_rk4<float, RA, (FM)>;
+#if FI_ENGINE_PART == 1
+EngineKernel engine_lines_kernel(int ra, int fm)
+{
+    FI_KERNEL(4, FFT_LINES)
+    FI_KERNEL(4, FFT_LINES | FFT_ROW3)
+    FI_KERNEL(2, FFT_LINES)
+    FI_KERNEL(2, FFT_LINES | FFT_ROW3)
+    FI_KERNEL(2, FFT_LINES | FFT_COL3)
+    FI_KERNEL(2, FFT_LINES | FFT_ROW3 | FFT_COL3)
+    return nullptr;
+}
+#elif FI_ENGINE_PART == 3
+EngineKernel engine_short_kernel(int ra, int fm)
+{
+    FI_KERNEL(4, FFT_LINES | FFT_SHORT)
+    FI_KERNEL(4, FFT_LINES | FFT_SHORT | FFT_ROW3)
+    FI_KERNEL(2, FFT_LINES | FFT_SHORT)
+    FI_KERNEL(2, FFT_LINES | FFT_SHORT | FFT_ROW3)
+    FI_KERNEL(2, FFT_LINES | FFT_SHORT | FFT_COL3)
+    FI_KERNEL(2, FFT_LINES | FFT_SHORT | FFT_ROW3 | FFT_COL3)
+    return nullptr;
+}
+#elif FI_ENGINE_PART == 2
+EngineKernel engine_wide_kernel(int ra, int fm)
+{
+    FI_KERNEL(2, FFT_LINES | FFT_WIDE)
+    FI_KERNEL(2, FFT_LINES | FFT_WIDE | FFT_ROW3)
+    FI_KERNEL(2, FFT_LINES | FFT_WIDE | FFT_COL3)
+    FI_KERNEL(2, FFT_LINES | FFT_WIDE | FFT_ROW3 | FFT_COL3)
+    return nullptr;
+}
+#endif
+
+#if FI_ENGINE_PART == 0
 // hi/lo split of the double state (mixed form), used before the first step
 // and after anything outside the engine changed x or w_ref.
 __global__ void k_split(const double* __restrict__ x, float* __restrict__ hi, float* __restrict__ lo, size_t n)
@@ -945,34 +1046,62 @@ void split_hilo_dxw(const double* x, float* hi, float* lo, const float* wrhi, co
     k_split_dxw<<<b, 256, 0, s>>>(x, hi, lo, wrhi, wrlo, dxw, n);
 }
 
-template <typename T, int RA, int FM> int engine_config_shape(const Plan2D& p, int nsm, int optin, int* grid, int* CB,
-                                                     size_t* smem)
+bool engine_has_lines(const Plan2D& p) { return engine_line(p.h) && engine_line(p.ny); }
+
+namespace {
+
+// The form of the phases for this plan, and its kernel (null where there is none).
+int engine_form(const Plan2D& p, int ra)
 {
-    const int cb = EngShape<RA>::cb;
-    *CB = cb;
-    *smem = engine_smem_bytes<T, RA>(p, cb);
-    if (FM == FFT_LINES) {
-        if (p.nx > EngShape<RA>::threads) return 0;   // a thread owns a column
-        *smem = lines_tab_off<RA>(p.nx, p.h, p.ny, cb) + engine_tab_count<T>(p.h, p.ny) * 2 * sizeof(T) + 64;
+    if (!engine_has_lines(p)) {
+        for (int f = 0; f < p.row.d.nf + p.col.d.nf; ++f) {
+            const int R = f < p.row.d.nf ? p.row.d.fac[f] : p.col.d.fac[f - p.row.d.nf];
+            if (R != 2 && R != 3 && R != 4 && R != 8) return FFT_ANY;
+        }
+        return FFT_23;
     }
+    const int size = ra == 2 && p.nx > EngShape<2>::threads  ? FFT_WIDE
+                     : p.h < SHORT_LINE || p.ny < SHORT_LINE ? FFT_SHORT
+                                                             : 0;
+    return FFT_LINES | (p.h % 3 == 0 ? FFT_ROW3 : 0) | (p.ny % 3 == 0 ? FFT_COL3 : 0) | size;
+}
+EngineKernel engine_kernel(const Plan2D& p, int ra)
+{
+    const int fm = engine_form(p, ra);
+    if (fm == FFT_ANY) return ra == 4 ? k_engine_rk4<float, 4, FFT_ANY> : k_engine_rk4<float, 2, FFT_ANY>;
+    if (fm == FFT_23) return ra == 4 ? k_engine_rk4<float, 4, FFT_23> : k_engine_rk4<float, 2, FFT_23>;
+    if (!engine_row(p.h, ra, fm) || !engine_col(p.ny, ra, fm)) return nullptr;
+    return (fm & FFT_WIDE)    ? engine_wide_kernel(ra, fm)
+           : (fm & FFT_SHORT) ? engine_short_kernel(ra, fm)
+                              : engine_lines_kernel(ra, fm);
+}
+
+template <int RA> int engine_config_shape(const Plan2D& p, int nsm, int optin, int* grid, int* CB, size_t* smem)
+{
+    const EngineKernel kern = engine_kernel(p, RA);
+    if (!kern) return 0;
+    const int fm = engine_form(p, RA);
+    const int cb = (fm & FFT_LINES) ? line_group(p.ny, EngShape<RA>::cb) : EngShape<RA>::cb;
+    *CB = cb;
+    *smem = engine_smem_bytes<float, RA>(p, cb);
+    if (fm & FFT_LINES)
+        *smem = lines_tab_off<RA>(p.nx, p.h, p.ny, cb) + engine_tab_count<float>(p.h, p.ny) * sizeof(float2) + 64;
     if (*smem > (size_t)optin) return 0;
     {
         // the limit is a property of the kernel, shared by every handle:
         // only ever raise it, so a handle of a smaller domain created later
         // does not lower it under a larger one
         static std::mutex mu;
-        static size_t cur = 0;
+        static size_t cur[64] = {};
         std::lock_guard<std::mutex> lk(mu);
-        if (*smem > cur) {
-            if (cudaFuncSetAttribute(k_engine_rk4<T, RA, FM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem) !=
-                cudaSuccess)
+        if (*smem > cur[fm]) {
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem) != cudaSuccess)
                 return 0;
-            cur = *smem;
+            cur[fm] = *smem;
         }
     }
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_engine_rk4<T, RA, FM>, EngShape<RA>::threads, *smem) !=
-            cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, EngShape<RA>::threads, *smem) != cudaSuccess ||
         per_sm < 1)
         return 0;
     if (per_sm > EngShape<RA>::per_sm) per_sm = EngShape<RA>::per_sm;
@@ -991,9 +1120,9 @@ template <typename T, int RA, int FM> int engine_config_shape(const Plan2D& p, i
     return 1;
 }
 
-bool engine_has_lines(const Plan2D& p) { return engine_line_rows(p.h) && engine_line_cols(p.ny); }
+}  // namespace
 
-template <typename T> int engine_config(const Plan2D& p, int* grid, int* CB, size_t* smem, int* RA, int* P2)
+template <typename T> int engine_config(const Plan2D& p, int* grid, int* CB, size_t* smem, int* RA)
 {
     // The plain FP64 form is FP64-throughput bound; it runs faster as the
     // multi-kernel graph (full occupancy) than in the one-grid engine.
@@ -1009,23 +1138,12 @@ template <typename T> int engine_config(const Plan2D& p, int* grid, int* CB, siz
         const int v = atoi(ev);
         if (v == 2 || v == 4) ra = v;
     }
-    const int p2 = engine_has_lines(p) ? 1 : 0;
-    *P2 = p2;
-    if constexpr (sizeof(T) == 4) {
-        auto shape = [&](int r) {
-            if (r == 4) return p2 ? engine_config_shape<T, 4, FFT_LINES>(p, nsm, optin, grid, CB, smem)
-                                  : engine_config_shape<T, 4, FFT_ANY>(p, nsm, optin, grid, CB, smem);
-            return p2 ? engine_config_shape<T, 2, FFT_LINES>(p, nsm, optin, grid, CB, smem)
-                      : engine_config_shape<T, 2, FFT_ANY>(p, nsm, optin, grid, CB, smem);
-        };
-        if (ra == 4 && shape(4)) {
-            *RA = 4;
-            return 1;
-        }
-        *RA = 2;
-        return shape(2);
+    if (ra == 4 && engine_config_shape<4>(p, nsm, optin, grid, CB, smem)) {
+        *RA = 4;
+        return 1;
     }
-    return 0;
+    *RA = 2;
+    return engine_config_shape<2>(p, nsm, optin, grid, CB, smem);
 }
 
 template <typename T> cudaError_t engine_launch(const EngineArgs& g, int grid, size_t smem, cudaStream_t s)
@@ -1043,16 +1161,15 @@ template <typename T> cudaError_t engine_launch(const EngineArgs& g, int grid, s
         attr[0].val.cooperative = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        if (g.ra == 4) return g.p2 ? cudaLaunchKernelEx(&cfg, k_engine_rk4<T, 4, FFT_LINES>, g)
-                                   : cudaLaunchKernelEx(&cfg, k_engine_rk4<T, 4, FFT_ANY>, g);
-        return g.p2 ? cudaLaunchKernelEx(&cfg, k_engine_rk4<T, 2, FFT_LINES>, g)
-                    : cudaLaunchKernelEx(&cfg, k_engine_rk4<T, 2, FFT_ANY>, g);
+        const EngineKernel kern = engine_kernel(g.p, g.ra);
+        return kern ? cudaLaunchKernelEx(&cfg, kern, g) : cudaErrorNotSupported;
     }
 }
 
-template int engine_config<float>(const Plan2D&, int*, int*, size_t*, int*, int*);
-template int engine_config<double>(const Plan2D&, int*, int*, size_t*, int*, int*);
+template int engine_config<float>(const Plan2D&, int*, int*, size_t*, int*);
+template int engine_config<double>(const Plan2D&, int*, int*, size_t*, int*);
 template cudaError_t engine_launch<float>(const EngineArgs&, int, size_t, cudaStream_t);
 template cudaError_t engine_launch<double>(const EngineArgs&, int, size_t, cudaStream_t);
+#endif   // FI_ENGINE_PART == 0
 
 }  // namespace fi

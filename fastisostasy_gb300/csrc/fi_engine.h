@@ -34,7 +34,6 @@ struct EngineArgs {
     int nsteps;
     int CB;                          // spectrum columns per phase-B item
     int ra;                          // rows per stencil item (kernel shape: 2 or 4)
-    int p2;                          // both transform lengths have a line phase
     double spy;
     double norm_scale;               // 1 / (nx*ny*1.) as the reference normalises
     float norm_scale_f;              // the same in float
@@ -49,10 +48,16 @@ struct EngineArgs {
     template <typename T> __device__ __forceinline__ const T* mB_T() const { return (const T*)mB; }
 };
 
+// Kernels on register lines of a form (FM in fi_engine.cu); null where there is none.
+typedef void (*EngineKernel)(EngineArgs);
+EngineKernel engine_lines_kernel(int ra, int fm);
+EngineKernel engine_wide_kernel(int ra, int fm);
+EngineKernel engine_short_kernel(int ra, int fm);
+
 // Grid size (co-resident blocks), phase-B column count, dynamic shared
-// memory, rows per stencil item and transform index mode of the engine for
-// this transform plan; 0 if it cannot run.
-template <typename T> int engine_config(const Plan2D& p, int* grid, int* CB, size_t* smem, int* RA, int* P2);
+// memory and rows per stencil item of the engine for this transform plan; 0 if
+// it cannot run.
+template <typename T> int engine_config(const Plan2D& p, int* grid, int* CB, size_t* smem, int* RA);
 // whether both transform lengths have the engine's line phases
 bool engine_has_lines(const Plan2D& p);
 template <typename T> cudaError_t engine_launch(const EngineArgs& g, int grid, size_t smem, cudaStream_t s);

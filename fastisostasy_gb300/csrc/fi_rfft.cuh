@@ -37,7 +37,8 @@ namespace fi {
 // where a float line is long.
 __host__ __device__ constexpr int line_points(int n, bool f32)
 {
-    return n % 3 == 0 ? (f32 && n >= 768 ? 24 : 12) : f32 ? (n >= 1024 ? 16 : 8) : n <= 256 ? 4 : 8;
+    const int e = n % 3 == 0 ? (f32 && n >= 768 ? 24 : 12) : f32 ? (n >= 1024 ? 16 : 8) : n <= 256 ? 4 : 8;
+    return n < e ? n : e;   // (the step engine's shortest lines: one thread)
 }
 template <typename T, int N> struct LineShape {
     static constexpr int E = line_points(N, sizeof(T) == 4);

@@ -50,8 +50,21 @@ def test_engine_on_lines(nx, ny, even):
     check_engine(nx, ny, even)
 
 
-@pytest.mark.parametrize("nx,ny", [(50, 50), (66, 46), (100, 100), (122, 98), (76, 140), (200, 200), (464, 466)])
+@pytest.mark.parametrize("nx,ny", [(50, 50), (66, 46), (100, 100), (122, 98), (76, 140), (200, 200), (464, 466),
+                                   (72, 54), (144, 288), (216, 486)])
 def test_engine_without_lines(monkeypatch, nx, ny):
-    """Shared-memory stages, radices 5, 7 and larger primes among them, two and four rows a block."""
+    """Shared-memory stages, with radices 5, 7 and larger primes and of 2 and 3 only, two and four rows a block."""
     monkeypatch.setenv("FI_NO_CLUSTER", "1")
     check_engine(nx, ny, nx != 100)
+
+
+@pytest.mark.parametrize("even", [True, False])
+@pytest.mark.parametrize("nx,ny", [(4, 4), (8, 6), (12, 8), (16, 12), (24, 16), (32, 24), (48, 32), (64, 48), (96, 64),
+                                   (128, 96), (192, 128), (384, 192), (512, 24), (768, 96), (1024, 48), (1024, 256),
+                                   (4, 512), (16, 512), (32, 384), (512, 128), (768, 512), (24, 500)])
+def test_engine_on_every_line(monkeypatch, nx, ny, even):
+    """Every length of the line phases in both directions: several lines or
+    columns in a warp, a line of two warps, grids wider than a block (and a last
+    one with a column length that has no line)."""
+    monkeypatch.setenv("FI_NO_CLUSTER", "1")
+    check_engine(nx, ny, even)
