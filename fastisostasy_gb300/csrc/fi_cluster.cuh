@@ -17,14 +17,15 @@
 //      owners); inverse rows, the corner values pushed to every block
 //
 // Stage states are float pairs; an RK4 increment enters them without its
-// corner mean, a constant that every difference drops and that the mantle
-// term takes off once the corners have arrived.  The arithmetic per cell is
-// that of the step engine (RK4), of ts_fused / ts_commit_pair (reference
-// stages) and of dp_stage_pair / dp_err / ts_commit_tpair (true stages).
+// corner mean, a constant that every difference drops and that the mantle term
+// and the sum of the stages take off once the corners have arrived.  The
+// arithmetic per cell is that of the step engine (RK4), of ts_fused /
+// ts_commit_pair (reference stages) and of dp_stage_pair / dp_err /
+// ts_commit_tpair (true stages).
 //
 // Measured (one RK4 update of ten steps, CUDA events, the engine's time
-// first): 32^2 471 -> 188 us, 64^2 485 -> 227, 96^2 575 -> 305, 128^2 523 ->
-// 280, 192^2 621 -> 451, 256^2 602 -> 540.  A 64^2 right-hand side takes 8600
+// first): 32^2 389 -> 186 us, 64^2 399 -> 225, 96^2 457 -> 309, 128^2 436 ->
+// 281, 192^2 508 -> 452, 256^2 475 -> 540.  A 64^2 right-hand side takes 8600
 // clocks, of which the three barriers 1750, the column pass 2000, the row
 // passes 2500 (32 threads a block have a line to work on) and the stencil
 // 2000; at 256^2 the stencil's 7300 and the column pass's 5800 of 20700 lead.
@@ -802,7 +803,9 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) k_cluster(ClusterArgs o
     const size_t n = (size_t)nx * ny;
     (void)n;
     if constexpr (MODE == CLU_RK4) {
-        float acc[CH];   // raw_1 + 2 raw_2 + 2 raw_3 of the own cells
+        // k_1 + 2 k_2 + 2 k_3 of the own cells, each raw less its corner mean
+        // before it is added (the mean can be most of it)
+        float acc[CH];
 #pragma unroll
         for (int q = 0; q < CH; ++q) acc[q] = 0.f;
         for (int step = 0; step < g.nsteps; ++step) {
@@ -814,42 +817,38 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) k_cluster(ClusterArgs o
             }
             __syncthreads();
             if (!S.go) break;   // alike in every block
-            double csum = 0.0;  // last thread: c1 + 2 c2 + 2 c3 + c4
             for (int stage = 0; stage < 4; ++stage) {
                 const float sdf = stage > 0 ? S.f[stage] : 0.f;
                 C.cells([&](int r, int e, int q) {
                     float hi = xh[e], lo = xl[e];
-                    if (stage > 0) {
-                        const float raw = fr[e];
-                        pair_add(hi, lo, sdf * raw, hi, lo);
-                        acc[q] = stage == 1 ? raw : acc[q] + 2.f * raw;
-                    }
+                    if (stage > 0) pair_add(hi, lo, sdf * fr[e], hi, lo);
                     C.put_y(r, hi, lo);
                 });
                 C.template rhs<true>(
                     [&]() {
-                        if (stage == 0) return;
-                        const double cm = C.corner();   // of the previous stage
-                        csum += (stage == 1 ? 1.0 : 2.0) * cm;
-                        S.f[6] = (float)cm;
+                        if (stage > 0) S.f[6] = (float)C.corner();   // of the previous stage
                     },
-                    [&](int e, int) {
+                    [&](int e, int q) {
                         float dy = dxw[e];
-                        if (stage > 0) dy += sdf * (fr[e] - S.f[6]);
+                        if (stage > 0) {
+                            const float k = fr[e] - S.f[6];
+                            dy += sdf * k;
+                            acc[q] = stage == 1 ? k : acc[q] + 2.f * k;
+                        }
                         return dy;
                     });
             }
             cluster_barrier();   // the corners of the last stage
-            if (tid == NT - 1) S.f[5] = (float)(csum + C.corner());
+            if (tid == NT - 1) S.f[5] = (float)C.corner();
             if (tid == 0) {
                 S.t = S.t + S.h;
                 S.n_acc++;
             }
             __syncthreads();
-            const float cs = S.f[5], sc = S.f[4];
+            const float cm = S.f[5], sc = S.f[4];
             C.cells([&](int r, int e, int q) {
                 const size_t c = (size_t)(C.r0 + r) * nx + C.i;
-                const float inc = ((acc[q] + fr[e]) - cs) * sc;
+                const float inc = (acc[q] + (fr[e] - cm)) * sc;
                 if constexpr (XREG) xr[q] += (double)inc;   // the FP64 state update
                 else g.x[c] += (double)inc;
                 float hi, lo;
