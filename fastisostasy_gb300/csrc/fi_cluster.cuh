@@ -133,6 +133,10 @@ __device__ __forceinline__ void st_dsm(uint32_t a, float v)
 {
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
 }
+__device__ __forceinline__ void st_dsm(uint32_t a, double v)
+{
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
 __device__ __forceinline__ void cluster_barrier()
 {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
@@ -172,9 +176,12 @@ __device__ __forceinline__ void pair_add(float xh, float xl, float inc, float& h
 
 // Shared state of a block outside the dynamic arrays.
 struct CluShared {
-    float corner[4];        // raw(1,1), raw(nx,ny), raw(1,ny), raw(nx,1) of the last right-hand side
-    float part[2][16][4];   // the blocks' partial reductions, of this attempt and of the one before
-    float red[16][4];       // the warps' (threads / 32 of them)
+    alignas(16) float corner[4];        // raw(1,1), raw(nx,ny), raw(1,ny), raw(nx,1) of the last right-hand side
+    // the blocks' partial reductions, of this attempt and of the one before,
+    // and the warps' (threads / 32 of them): two maxima and a sum, which takes
+    // the place of two floats where it is in FP64 (sum64)
+    float part[2][16][4];
+    float red[16][4];
     double t, dt, tf, h;
     double tol, err;
     long long n_acc, n_rej, n_att;
@@ -183,6 +190,8 @@ struct CluShared {
     float cm[8];            // corner means of the stage outputs
     float f[24];            // float scalars of the current stage or attempt
 };
+
+__device__ __forceinline__ double* sum64(float* slot) { return reinterpret_cast<double*>(slot + 2); }
 
 // What the transform phases need, the same for all threads of a block.
 struct CluCtx {
@@ -642,7 +651,14 @@ template <int NT, int CH> struct Clu {
 
     // max, max, sum of per-thread values over the cluster; every block gets
     // the same totals (one barrier).  A rejected attempt has no other barrier,
-    // so consecutive reductions use the two halves of S.part in turn.
+    // so consecutive reductions use the two halves of S.part in turn.  The sum
+    // is of floats within a block, as ts_fused_body takes it, or with SUM64 of
+    // the threads' values in FP64, as ts_err_body does.  Maxima stay floats to
+    // the end: one FP64 instruction after another on thread 0 (64 clocks each)
+    // they took 3 us of an attempt (an update of 20 attempts: true stages at
+    // 192^2 1763 -> 1710 us with the FP64 sum, 1786 without this; reference
+    // stages at 128^2 309 -> 254).
+    template <bool SUM64>
     __device__ __forceinline__ void reduce(float m1, float m2, float s2, int parity, double* tot) const
     {
         const unsigned FULL = 0xffffffffu;
@@ -650,37 +666,55 @@ template <int NT, int CH> struct Clu {
         for (int o = 16; o > 0; o >>= 1) {
             m1 = fmaxf(m1, __shfl_xor_sync(FULL, m1, o));
             m2 = fmaxf(m2, __shfl_xor_sync(FULL, m2, o));
-            s2 += __shfl_xor_sync(FULL, s2, o);
         }
-        const int wid = threadIdx.x >> 5;
-        if ((threadIdx.x & 31) == 0) {
+        const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        if constexpr (SUM64) {
+            double d2 = (double)s2;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) d2 += __shfl_xor_sync(FULL, d2, o);
+            if (lane == 0) *sum64(S.red[wid]) = d2;
+        } else {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(FULL, s2, o);
+            if (lane == 0) S.red[wid][2] = s2;
+        }
+        if (lane == 0) {
             S.red[wid][0] = m1;
             S.red[wid][1] = m2;
-            S.red[wid][2] = s2;
         }
         __syncthreads();
+        if constexpr (SUM64) {
+            if (wid == 0) {
+                double d2 = lane < NT / 32 ? *sum64(S.red[lane]) : 0.0;
+#pragma unroll
+                for (int o = NT / 64; o > 0; o >>= 1) d2 += __shfl_down_sync(FULL, d2, o);
+                d2 = __shfl_sync(FULL, d2, 0);
+                if (lane < nc) st_dsm(map_rank(smem_u32(sum64(S.part[parity][rank])), lane), d2);
+            }
+        }
         if ((int)threadIdx.x < nc) {
             float a = 0.f, b = 0.f, c = 0.f;
             for (int q = 0; q < NT / 32; ++q) {
                 a = fmaxf(a, S.red[q][0]);
                 b = fmaxf(b, S.red[q][1]);
-                c += S.red[q][2];
+                if (!SUM64) c += S.red[q][2];
             }
             const int to = threadIdx.x;
             st_dsm(map_rank(smem_u32(&S.part[parity][rank][0]), to), a);
             st_dsm(map_rank(smem_u32(&S.part[parity][rank][1]), to), b);
-            st_dsm(map_rank(smem_u32(&S.part[parity][rank][2]), to), c);
+            if (!SUM64) st_dsm(map_rank(smem_u32(&S.part[parity][rank][2]), to), c);
         }
         cluster_barrier();
         if (threadIdx.x == 0) {
-            double a = 0.0, b = 0.0, c = 0.0;
+            float a = 0.f, b = 0.f;
+            double c = 0.0;
             for (int q = 0; q < nc; ++q) {
-                a = fmax(a, (double)S.part[parity][q][0]);
-                b = fmax(b, (double)S.part[parity][q][1]);
-                c += (double)S.part[parity][q][2];
+                a = fmaxf(a, S.part[parity][q][0]);
+                b = fmaxf(b, S.part[parity][q][1]);
+                c += SUM64 ? *sum64(S.part[parity][q]) : (double)S.part[parity][q][2];
             }
-            tot[0] = a;
-            tot[1] = b;
+            tot[0] = (double)a;
+            tot[1] = (double)b;
             tot[2] = c;
         }
     }
@@ -900,7 +934,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) k_cluster(ClusterArgs o
                 s2 += dx * dx;
             });
             double tot[3];
-            C.reduce(m1, m2, s2, par, tot);
+            C.template reduce<false>(m1, m2, s2, par, tot);
             if (tid == 0) {
                 S.tol = g.atol + g.rtol * fmax(tot[0], tot[1]);
                 S.err = sqrt(tot[2] / (double)n) / S.tol;
@@ -970,7 +1004,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) k_cluster(ClusterArgs o
                 s2 += dx * dx;
             });
             double tot[3];
-            C.reduce(m1, m2, s2, par, tot);
+            C.template reduce<true>(m1, m2, s2, par, tot);
             if (tid == 0) {
                 S.tol = g.atol + g.rtol * fmax(tot[0], tot[1]);
                 S.err = sqrt(tot[2] / (double)n) / S.tol;
