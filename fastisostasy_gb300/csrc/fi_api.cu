@@ -900,6 +900,28 @@ int ensure_pin(fi_handle* h)
     return FI_OK;
 }
 
+// The grid-wide step engine of an RK4 domain: its shape and buffers, where it
+// can run (h->engine_ok).
+int ensure_engine(fi_handle* h)
+{
+    if (h->engine_ok) return FI_OK;
+    const bool ok = mixed(h) ? engine_config<float>(h->prhs, &h->eng_grid, &h->eng_CB, &h->eng_smem, &h->eng_RA) != 0
+                             : engine_config<double>(h->prhs, &h->eng_grid, &h->eng_CB, &h->eng_smem, &h->eng_RA) != 0;
+    cudaGetLastError();
+    if (!ok) return FI_OK;
+    const size_t nk = (size_t)(h->prhs.h + 1) * h->ny;
+    int rc;
+    if ((rc = dalloc(h, &h->ST, nk * 2 * tsz(h))) || (rc = dalloc(h, &h->eng_bar, sizeof(unsigned)))) return rc;
+    // (a domain that steps in a cluster has the transposed factors already)
+    if (!h->mAT && ((rc = dalloc(h, &h->mAT, nk * tsz(h))) || (rc = dalloc(h, &h->mBT, nk * tsz(h))))) return rc;
+    h->engine_ok = true;
+    return FI_OK;
+}
+
+// Whether updates launched now step in a cluster: a traced domain steps on the
+// engine, whose phases the trace stamps.
+bool in_cluster(const fi_handle* h) { return h->clu_ok && !(h->trace && h->engine_ok); }
+
 // The elastic and geoid Green's functions on the host.
 int ensure_green(fi_handle* h)
 {
@@ -1446,7 +1468,7 @@ template <typename T> int update_T(fi_handle* h, const double* dH, double time, 
             enqueue_post<T>(h, raw_last, have_rhs);
             return FI_OK;
         }
-        T* raw_last = (h->clu_ok && nsteps > 0)      ? (T*)enqueue_cluster(h, nsteps)
+        T* raw_last = (in_cluster(h) && nsteps > 0)  ? (T*)enqueue_cluster(h, nsteps)
                       : (h->engine_ok && nsteps > 0) ? enqueue_engine<T>(h, nsteps)
                                                      : enqueue_steps<T>(h, nsteps);
         enqueue_post<T>(h, raw_last, nsteps > 0 ? 1 : 0);
@@ -1596,6 +1618,7 @@ int fi_engine_trace(fi_handle* h, unsigned long long* out, int n)
     if (!h) return FI_E_ARG;
     if (!h->trace) {
         int rc;
+        if (h->clu_ok && h->clu_mode == CLU_RK4 && (rc = ensure_engine(h))) return rc;
         if ((rc = dalloc(h, &h->trace, 256 * sizeof(unsigned long long)))) return rc;
         CK(cudaMemsetAsync(h->trace, 0, 256 * sizeof(unsigned long long), h->s));
         CK(cudaStreamSynchronize(h->s));
@@ -1880,16 +1903,7 @@ int fi_create_handle(const fi_params* pin, int nx_ice, int ny_ice, double dx, do
             cudaGetLastError();
             if (h->clu_ok) { AL2(h->mAT, nk * tsz(h)); AL2(h->mBT, nk * tsz(h)); }
         }
-        if (want && !h->clu_ok) {
-            int ok = mixed(h) ? engine_config<float>(h->prhs, &h->eng_grid, &h->eng_CB, &h->eng_smem, &h->eng_RA)
-                              : engine_config<double>(h->prhs, &h->eng_grid, &h->eng_CB, &h->eng_smem, &h->eng_RA);
-            h->engine_ok = ok != 0;
-            cudaGetLastError();
-            if (h->engine_ok) {
-                AL2(h->ST, nk * c2); AL2(h->mAT, nk * tsz(h)); AL2(h->mBT, nk * tsz(h));
-                AL2(h->eng_bar, sizeof(unsigned));
-            }
-        }
+        if (want && !h->clu_ok && (rc = ensure_engine(h))) return rc;
         if ((rk4_true || tsit_true) && mixed(h)) {
             // the float pairs of x and w_ref (the stage states of every path)
             AL2(h->xhi, n * 4); AL2(h->xlo, n * 4); AL2(h->wrefhi, n * 4); AL2(h->wreflo, n * 4);
@@ -2196,7 +2210,7 @@ int fi_metrics_json(fi_handle* h, char* buf, size_t len)
                            "\"host_update_ms\": %.6f, \"status\": %d}",
                            h->nx, h->ny, h->nx_ice, h->ny_ice, mixed(h) ? "mixed" : "fp64", p.method, p.dt_method,
                            p.stage_mode, h->engine_ok || h->clu_ok ? "true" : "false",
-                           h->clu_ok ? "cluster" : h->engine_ok ? "engine" : "kernels", h->updates, hc.t, hc.dt, hc.n_accept,
+                           in_cluster(h) ? "cluster" : h->engine_ok ? "engine" : "kernels", h->updates, hc.t, hc.dt, hc.n_accept,
                            hc.n_reject, hc.n_attempt, h->launches, (int)h->graphs.size(), 1e3 * h->host_update_s,
                            hc.status);
     return (n < 0 || (size_t)n >= len) ? FI_E_SIZE : FI_OK;

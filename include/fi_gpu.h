@@ -379,7 +379,9 @@ int fi_profile(fi_handle* h, int enable);
  * the last update, taken by block 0 at every phase and sub-phase boundary
  * (up to 256): the first call enables tracing (for updates launched after
  * it: a CUDA graph captured earlier keeps running untraced), later calls
- * copy up to n timestamps into `out`. */
+ * copy up to n timestamps into `out`.  An RK4 domain that otherwise steps in a
+ * thread-block cluster makes its traced updates on the engine; one without the
+ * engine (one kernel a pass, adaptive steps, FP64) leaves no stamps. */
 int fi_engine_trace(fi_handle* h, unsigned long long* out, int n);
 int fi_profile_read(fi_handle* h, double* ms, long long* counts, int n);
 

@@ -5,6 +5,8 @@ stages for lengths without one.
 
 The bound is the mixed form's, 1e-5 of the largest displacement.
 """
+import ctypes as C
+
 import pytest
 
 from fastisostasy_gb300.isostasy import Domain
@@ -68,3 +70,28 @@ def test_engine_on_every_line(monkeypatch, nx, ny, even):
     one with a column length that has no line)."""
     monkeypatch.setenv("FI_NO_CLUSTER", "1")
     check_engine(nx, ny, even)
+
+
+@pytest.mark.parametrize("n", [32, 64, 192, 256])
+def test_engine_trace(monkeypatch, n):
+    """Traced updates stamp the engine's phases also where the domain otherwise
+    steps in a cluster, and give its result within the mixed form's bound."""
+    monkeypatch.setenv("FI_NO_GRAPHS", "1")
+    pair = Pair(workload(n, n, n, True), precision=1)
+    L = pair.dom.L
+    pair.init()
+    pair.step(1)
+    assert pair.dom.metrics()["stepper"] == ("engine" if n == 256 else "cluster")
+    buf = (C.c_ulonglong * 256)()
+    assert L.fi_engine_trace(pair.dom.h, buf, 256) == 0
+    pair.step(2)
+    assert pair.dom.metrics()["stepper"] == "engine"
+    assert L.fi_engine_trace(pair.dom.h, buf, 256) == 0
+    stamps = [v for v in buf if v]
+    # step begin and end, and for each of the four stages six phase boundaries
+    assert len(stamps) >= 4 * 6 + 2 and stamps == sorted(stamps)
+    assert stamps[-1] - stamps[0] < 1e9
+    for f in ("w", "z_bed"):
+        assert rel(pair.dom.field(f), pair.orc.field(f)) <= 1e-5
+    assert pair.dom.scalars()["n_accept"] == 30
+    pair.close()
