@@ -2644,12 +2644,8 @@ int batch_shape(fi_batch* b, int RB, int CB, int waves)
         BMember& m = b->hM[i];
         if (m.lines & 1) m.RB = b->rows_threads / rhs_line_threads(m.p.h, m.p, b->mixed);
         if (m.lines & 2) m.CB = b->cols_threads / rhs_line_threads(m.p.ny, m.p, b->mixed);
-        // stencil tiles: the FP64 state of true stages without the pairs has its own
-        const bool pair = b->mixed && (!b->true_stages || m.yhi);
-        m.fgx = pair ? (m.p.nx + 63) / 64 : (m.p.nx + 31) / 32;
-        const int fblk = pair ? batch_flexure_tiles32(m.p.nx, m.p.ny)
-                       : b->mixed ? m.fgx * ((m.p.ny + 7) / 8)
-                                  : batch_flexure_tiles64(m.p.nx, m.p.ny);
+        m.fgx = b->mixed ? (m.p.nx + 63) / 64 : (m.p.nx + 31) / 32;
+        const int fblk = b->mixed ? batch_flexure_tiles32(m.p.nx, m.p.ny) : batch_flexure_tiles64(m.p.nx, m.p.ny);
         const int rblk = (m.p.ny + m.RB - 1) / m.RB;
         const int cblk = (m.p.h + 1 + m.CB - 1) / m.CB;
         off[i + 1] = off[i] + fblk;
@@ -2965,7 +2961,7 @@ int fi_batch_create(fi_handle* const* hs, int n, fi_batch** out)
     }
     b->hM.swap(M);
     // default shapes: 8 rows / 8 spectrum columns per transform block for
-    // mixed batches (64-byte column segments), 16-row strip tasks, 8 waves;
+    // mixed batches (64-byte column segments), 16-row stencil tiles, 8 waves;
     // FI_BATCH_RB / FI_BATCH_CB / FI_BATCH_WAVES override (tuning)
     int RB = b->mixed ? 8 : 0, CB = b->mixed ? 8 : 0, waves = 8;
     if (const char* e = getenv("FI_BATCH_RB")) { const int v = atoi(e); if (v >= 1 && v <= 16) RB = v; }

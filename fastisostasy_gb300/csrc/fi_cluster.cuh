@@ -45,6 +45,7 @@
 
 #include "fi_cluster.h"
 #include "fi_lines.cuh"
+#include "fi_tableau.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -720,21 +721,6 @@ template <int NT, int CH> struct Clu {
     }
 };
 
-// stage coefficients of RK4 and the reference's weights (fi_state.cu holds the same)
-__constant__ double k_rk4_a[4] = {0.0, 0.5, 0.5, 1.0};
-__constant__ double k_ts_b[6] = {0.0845, 0.0, 0.0, 0.5179, 0.1276, 0.2700};
-__constant__ double k_ts_bh5 = 0.2700 - 1 / 5.0;
-__constant__ double k_dp_a[7][6] = {
-    {0, 0, 0, 0, 0, 0},
-    {1.0 / 5, 0, 0, 0, 0, 0},
-    {3.0 / 40, 9.0 / 40, 0, 0, 0, 0},
-    {44.0 / 45, -56.0 / 15, 32.0 / 9, 0, 0, 0},
-    {19372.0 / 6561, -25360.0 / 2187, 64448.0 / 6561, -212.0 / 729, 0, 0},
-    {9017.0 / 3168, -355.0 / 33, 46732.0 / 5247, 49.0 / 176, -5103.0 / 18656, 0},
-    {35.0 / 384, 0, 500.0 / 1113, 125.0 / 192, -2187.0 / 6784, 11.0 / 84}};
-__constant__ double k_dp_bs[7] = {5179.0 / 57600, 0, 7571.0 / 16695, 393.0 / 640, -92097.0 / 339200, 187.0 / 2100,
-                                  1.0 / 40};
-
 // The next attempt of an adaptive update (attempt_begin_one): thread 0.
 __device__ __forceinline__ void clu_attempt_begin(CluShared& S, int max_iter)
 {
@@ -846,7 +832,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) k_cluster(ClusterArgs o
             if (tid == 0) {
                 S.go = S.status == ST_OK && S.t < S.tf;
                 S.h = fmin(S.dt, S.tf - S.t);   // src/integrators.f90:62-63
-                for (int st = 1; st < 4; ++st) S.f[st] = (float)(k_rk4_a[st] * S.h * g.spy);
+                for (int st = 1; st < 4; ++st) S.f[st] = (float)(c_rk4_a[st] * S.h * g.spy);
                 S.f[4] = (float)((S.h / 6) * g.spy);
             }
             __syncthreads();
@@ -906,9 +892,9 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) k_cluster(ClusterArgs o
             if (tid == 0) {
                 clu_attempt_begin(S, g.max_iter);
                 const double dt = S.h;
-                S.cx = ((dt * k_ts_b[0] + dt * k_ts_b[3]) + dt * k_ts_b[4]) + dt * k_ts_b[5];
+                S.cx = ((dt * c_ts_b[0] + dt * c_ts_b[3]) + dt * c_ts_b[4]) + dt * c_ts_b[5];
                 S.f[0] = (float)S.cx;
-                S.f[1] = (float)(dt * k_ts_b[5] - dt * k_ts_bh5);
+                S.f[1] = (float)(dt * c_ts_b[5] - dt * c_ts_bh[5]);
                 S.f[2] = (float)g.spy;
                 if (S.go) S.have = 1;
             }
@@ -974,7 +960,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) k_cluster(ClusterArgs o
             for (int q = 0; q < CH; ++q) a[q] = 0.f;
             // stage 0 only where no accepted attempt left its right-hand side
             for (int i = valid ? 1 : 0; i <= 6; ++i) {
-                if (tid < i) S.f[tid] = (float)(k_dp_a[i][tid] * S.h * g.spy);
+                if (tid < i) S.f[tid] = (float)(c_dp_a[i][tid] * S.h * g.spy);
                 __syncthreads();
                 C.cells([&](int r, int e, int q) {
                     float v = 0.f;
@@ -992,7 +978,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) k_cluster(ClusterArgs o
                 __syncthreads();
             }
             valid = true;
-            if (tid < 7) S.f[tid] = (float)(((tid < 6 ? k_dp_a[6][tid] : 0.0) - k_dp_bs[tid]) * S.h * g.spy);
+            if (tid < 7) S.f[tid] = (float)(((tid < 6 ? c_dp_a[6][tid] : 0.0) - c_dp_bs[tid]) * S.h * g.spy);
             __syncthreads();
             float m1 = 0.f, m2 = 0.f, s2 = 0.f;
             C.cells([&](int, int e, int q) {

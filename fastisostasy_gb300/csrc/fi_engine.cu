@@ -26,6 +26,7 @@
 
 #include "fi_engine.h"
 #include "fi_lines.cuh"
+#include "fi_tableau.cuh"
 
 // Translation units: the host code and the kernels on shared-memory stages
 // (0, this file), those on register lines (1, fi_engine_lines.cu), of grids
@@ -68,9 +69,6 @@ template <int RA> struct EngShape {
 // kernel / the 2^k ones / those from 128 points: 512^2 668 / 653 / 645 us,
 // 256^2 505 / 494 / 471; 324^2 with / without the odd radices 973 / 942).
 enum { FFT_ANY = 0, FFT_LINES = 1, FFT_ROW3 = 2, FFT_COL3 = 4, FFT_WIDE = 8, FFT_SHORT = 16, FFT_23 = 32 };
-
-// stage coefficients of RK4: y_s = x + a_s h k_{s-1}
-static __constant__ double c_rk4_a[4] = {0.0, 0.5, 0.5, 1.0};
 
 template <typename T, int RA> struct PhaseAMem {
     // level-0 differences on RA+4 rows, moments on RA+2 rows, all full width

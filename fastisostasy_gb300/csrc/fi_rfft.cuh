@@ -68,9 +68,8 @@ template <typename C2> __device__ __forceinline__ C2 cscale(C2 a, decltype(C2::x
     return a;
 }
 
-template <typename T, typename C2, int SIGN> __device__ __forceinline__ C2 rot_w8(C2 o, T h)   // o * exp(SIGN i pi/4) / h
+template <typename C2, int SIGN> __device__ __forceinline__ C2 rot_w8(C2 o)   // o exp(SIGN i pi/4) sqrt(2)
 {
-    (void)h;
     C2 r;
     if (SIGN < 0) { r.x = o.x + o.y; r.y = o.y - o.x; }
     else { r.x = o.x - o.y; r.y = o.y + o.x; }
@@ -106,8 +105,8 @@ template <typename T, typename C2, int SIGN> __device__ __forceinline__ void rdf
     rdft4<T, C2, SIGN>(e0, e1, e2, e3);
     rdft4<T, C2, SIGN>(o0, o1, o2, o3);
     const T h = (T)0.70710678118654752440084436210484903928;
-    const C2 t1 = rot_w8<T, C2, SIGN>(o1, h);                // w8 o1 / h
-    const C2 u3 = rot_w8<T, C2, SIGN>(o3, h);
+    const C2 t1 = rot_w8<C2, SIGN>(o1);                // w8 o1 / h
+    const C2 u3 = rot_w8<C2, SIGN>(o3);
     C2 t3;                                                   // w8^3 o3 / h = (SIGN i) w8 o3 / h
     if (SIGN < 0) { t3.x = u3.y; t3.y = -u3.x; }
     else { t3.x = -u3.y; t3.y = u3.x; }
@@ -133,13 +132,13 @@ template <typename T, typename C2, int SIGN> __device__ __forceinline__ void rdf
     const T sg = (T)(SIGN < 0 ? -1 : 1);
     const C2 w1 = mk2<T>(c1, sg * s1), w3 = mk2<T>(s1, sg * c1), w9 = mk2<T>(-c1, -sg * s1);
     v[5] = cmul(v[5], w1);
-    v[9] = cscale(rot_w8<T, C2, SIGN>(v[9], h), h);
+    v[9] = cscale(rot_w8<C2, SIGN>(v[9]), h);
     v[13] = cmul(v[13], w3);
-    v[6] = cscale(rot_w8<T, C2, SIGN>(v[6], h), h);
+    v[6] = cscale(rot_w8<C2, SIGN>(v[6]), h);
     v[10] = mul_mi(v[10], SIGN);
-    v[14] = cscale(mul_mi(rot_w8<T, C2, SIGN>(v[14], h), SIGN), h);
+    v[14] = cscale(mul_mi(rot_w8<C2, SIGN>(v[14]), SIGN), h);
     v[7] = cmul(v[7], w3);
-    v[11] = cscale(mul_mi(rot_w8<T, C2, SIGN>(v[11], h), SIGN), h);
+    v[11] = cscale(mul_mi(rot_w8<C2, SIGN>(v[11]), SIGN), h);
     v[15] = cmul(v[15], w9);
 #pragma unroll
     for (int q = 0; q < 4; ++q) rdft4<T, C2, SIGN>(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);

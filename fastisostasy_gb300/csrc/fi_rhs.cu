@@ -62,16 +62,19 @@ template <typename K> static void set_smem(K kern, size_t bytes)
 }
 
 // ---------------------------------------------------------------------------
-// Flexure stencil.  Tile TX x TY outputs with a halo of 2; the first-level
-// differences are taken on the double state, then rounded to T.
+// Flexure stencil of the mixed form on a distorted grid (1/(dx K), 1/(dy K) per
+// cell).  Tile TX x TY outputs with a halo of 2; the first-level differences
+// are taken on the double state, then rounded to float.
 // ---------------------------------------------------------------------------
 constexpr int TX = 32, TY = 8, RX = TX + 4, RY = TY + 4;
 
-template <typename T>
-__device__ __forceinline__ void flexure_body(const double* __restrict__ y, const double* __restrict__ wref, const T* __restrict__ q0,
-          const uint8_t* __restrict__ mask, const T* __restrict__ D, const T* __restrict__ inv2eta,
-          T* __restrict__ f, int nx, int ny, FlexCoef c, int bx, int by)
+__global__ void __launch_bounds__(TX* TY)
+k_flexure(const double* __restrict__ y, const double* __restrict__ wref, const float* __restrict__ q0,
+          const uint8_t* __restrict__ mask, const float* __restrict__ D, const float* __restrict__ inv2eta,
+          float* __restrict__ f, int nx, int ny, FlexCoef c, const int* __restrict__ gate)
 {
+    if (gate && *gate == 0) return;
+    typedef float T;
     __shared__ double ys[RY][RX];
     __shared__ T wx[RY][RX];
     __shared__ T Mxx[RY][RX];
@@ -79,23 +82,19 @@ __device__ __forceinline__ void flexure_body(const double* __restrict__ y, const
     __shared__ T Mxy[RY][RX];
     __shared__ T Mxyx[RY][RX];
     const int tid = threadIdx.x + TX * threadIdx.y;
-    const int i0 = bx * TX, j0 = by * TY;
-    const bool uni = (c.ixm == nullptr);
+    const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
 
-    // per-cell spacing accessors (uniform fast path)
-    // (1/(2 d) and 1/d^2 from the stored 1/d: an FP64 division is a chain of a
-    // dozen FP64 instructions, and a cell took eight)
-    auto idx1 = [&](int i, int j) -> double { return uni ? c.inv_dx : c.ixm[(size_t)j * nx + i]; };
-    auto idx2h = [&](int i, int j) -> double { return uni ? c.inv_2dx : 0.5 * c.ixm[(size_t)j * nx + i]; };
+    // per-cell spacings: 1/(2 d) and 1/d^2 from the stored 1/d (an FP64
+    // division is a chain of a dozen FP64 instructions, and a cell took eight)
+    auto idx1 = [&](int i, int j) -> double { return c.ixm[(size_t)j * nx + i]; };
+    auto idx2h = [&](int i, int j) -> double { return 0.5 * c.ixm[(size_t)j * nx + i]; };
     auto idxx = [&](int i, int j) -> double {
-        if (uni) return c.inv_dx2;
         const double d = c.ixm[(size_t)j * nx + i];
         return d * d;
     };
-    auto idy1 = [&](int i, int j) -> double { return uni ? c.inv_dy : c.iym[(size_t)j * nx + i]; };
-    auto idy2h = [&](int i, int j) -> double { return uni ? c.inv_2dy : 0.5 * c.iym[(size_t)j * nx + i]; };
+    auto idy1 = [&](int i, int j) -> double { return c.iym[(size_t)j * nx + i]; };
+    auto idy2h = [&](int i, int j) -> double { return 0.5 * c.iym[(size_t)j * nx + i]; };
     auto idyy = [&](int i, int j) -> double {
-        if (uni) return c.inv_dy2;
         const double d = c.iym[(size_t)j * nx + i];
         return d * d;
     };
@@ -178,16 +177,6 @@ __device__ __forceinline__ void flexure_body(const double* __restrict__ y, const
             f[e] = (((p + mx_xx) + (T)2 * mxy_xy) + my_yy) * inv2eta[e];
         }
     }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(TX* TY)
-k_flexure(const double* __restrict__ y, const double* __restrict__ wref, const T* __restrict__ q0,
-          const uint8_t* __restrict__ mask, const T* __restrict__ D, const T* __restrict__ inv2eta,
-          T* __restrict__ f, int nx, int ny, FlexCoef c, const int* __restrict__ gate)
-{
-    if (gate && *gate == 0) return;
-    flexure_body<T>(y, wref, q0, mask, D, inv2eta, f, nx, ny, c, blockIdx.x, blockIdx.y);
 }
 
 // Mixed form, uniform spacing.  The only double work per cell is the pair of
@@ -473,13 +462,14 @@ static int strip_seg_single(int nx, int ny)
 // ---------------------------------------------------------------------------
 constexpr int TY64 = 16;                              // 32 x R outputs, 32 x 8 threads
 constexpr int YC = TX + 4, MC = TX + 2;
+constexpr int SMS = 152;   // multiprocessors of a GB300
 static int tile64_rows(int nx, int ny)
 {
     int best = 16;
     long long least = -1;
     for (int r : {16, 8, 4}) {
         const long long tiles = (long long)((nx + TX - 1) / TX) * ((ny + r - 1) / r);
-        const long long cost = (tiles + 151) / 152 * (2 * r + 2) + r / 2;
+        const long long cost = (tiles + SMS - 1) / SMS * (2 * r + 2) + r / 2;
         if (least < 0 || cost < least) { least = cost; best = r; }
     }
     return best;
@@ -959,7 +949,7 @@ void launch_flexure(const double* y, const double* wref, const T* q0, const uint
                 k_flexure64k<R><<<g64, b64, 0, s>>>(y, wref, q0, mask, D, inv2eta, f, nx, ny, c, gate);
         });
     } else {
-        k_flexure<T><<<g, b, 0, s>>>(y, wref, q0, mask, D, inv2eta, f, nx, ny, c, gate);
+        k_flexure<<<g, b, 0, s>>>(y, wref, q0, mask, D, inv2eta, f, nx, ny, c, gate);
     }
 }
 
@@ -1506,9 +1496,9 @@ void batch_rows_inv(const BMember* M, BList L, int nblk, int threads, size_t sme
 }
 
 // True stages: the RHS at stage state y (stage 0: x, 1-5: the stage buffer,
-// 6: x2) with the mantle term at that state: mixed members over
-// the float pair of the stage state (stage 0: of x) and its dxw, mixed ones
-// without the pairs and FP64 members over the FP64 state.
+// 6: x2) with the mantle term at that state: mixed members over the float pair
+// of the stage state (stage 0: of x) and its dxw, FP64 members over the FP64
+// state.
 template <typename T>
 __global__ void __launch_bounds__(256) k_b_flexure_y(const BMember* __restrict__ M, BList L, int stage)
 {
@@ -1517,15 +1507,9 @@ __global__ void __launch_bounds__(256) k_b_flexure_y(const BMember* __restrict__
         const int bx = local % b.fgx, by = local / b.fgx;
         const double* y = stage == 0 ? b.d.x : (stage == 6 ? b.d.ts_x2 : b.yst);
         if constexpr (sizeof(T) == 4) {
-            if (b.yhi) {
-                const bool s0 = stage == 0;
-                flexure_tile(s0 ? b.xhi : b.yhi, s0 ? b.xlo : b.ylo, nullptr, s0 ? b.xdw : b.ydw, (const float*)b.q0,
-                             b.mask, (const float*)b.D, (const float*)b.inv2eta, (float*)b.f, b.p.nx, b.p.ny, b.fcf,
-                             bx, by);
-            } else {
-                flexure_f32_body(y, b.wref, (const float*)b.q0, b.mask, (const float*)b.D,
-                                        (const float*)b.inv2eta, (float*)b.f, b.p.nx, b.p.ny, b.fcf, bx, by);
-            }
+            const bool s0 = stage == 0;
+            flexure_tile(s0 ? b.xhi : b.yhi, s0 ? b.xlo : b.ylo, nullptr, s0 ? b.xdw : b.ydw, (const float*)b.q0, b.mask,
+                         (const float*)b.D, (const float*)b.inv2eta, (float*)b.f, b.p.nx, b.p.ny, b.fcf, bx, by);
         } else if (b.fc.ixm == nullptr) {
             flexure_tile64<false, TY64>(y, nullptr, b.wref, (const double*)b.q0, b.mask, (const double*)b.D,
                                   (const double*)b.inv2eta, (double*)b.f, b.p.nx, b.p.ny, b.fc64, bx, by);

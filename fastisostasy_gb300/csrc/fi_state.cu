@@ -14,6 +14,7 @@
 
 #include "fi_batch.h"
 #include "fi_state.h"
+#include "fi_tableau.cuh"
 
 namespace fi {
 
@@ -584,8 +585,6 @@ k_euler_final(const Ctl* __restrict__ c, double* __restrict__ x, double* __restr
 }
 
 // --- Tsitouras 5(4), reference-compatible (single distinct RHS value) --------
-__constant__ double c_ts_b[6] = {0.0845, 0.0, 0.0, 0.5179, 0.1276, 0.2700};
-__constant__ double c_ts_bh[6] = {0.0845, 0.0, 0.0, 0.5179, 0.1276, 0.2700 - 1 / 5.0};
 
 __device__ __forceinline__ void ts_x12(double x, double k, double dt, double& x1, double& x2)
 {
@@ -854,16 +853,6 @@ __global__ void k_ts_attempt_end(Ctl* c, cudaGraphConditionalHandle loop, int fs
 
 // --- Tsitouras 5(4) with true stages: the Dormand-Prince 5(4) pair whose
 // truncated coefficients the reference prints, with FSAL ----------------------
-__constant__ double c_dp_a[7][6] = {
-    {0, 0, 0, 0, 0, 0},
-    {1.0 / 5, 0, 0, 0, 0, 0},
-    {3.0 / 40, 9.0 / 40, 0, 0, 0, 0},
-    {44.0 / 45, -56.0 / 15, 32.0 / 9, 0, 0, 0},
-    {19372.0 / 6561, -25360.0 / 2187, 64448.0 / 6561, -212.0 / 729, 0, 0},
-    {9017.0 / 3168, -355.0 / 33, 46732.0 / 5247, 49.0 / 176, -5103.0 / 18656, 0},
-    {35.0 / 384, 0, 500.0 / 1113, 125.0 / 192, -2187.0 / 6784, 11.0 / 84}};
-__constant__ double c_dp_bs[7] = {5179.0 / 57600, 0, 7571.0 / 16695, 393.0 / 640, -92097.0 / 339200, 187.0 / 2100,
-                                  1.0 / 40};
 
 // block corner means of the stage outputs 0..ns-1 (shared, one thread each)
 template <typename T>

@@ -188,7 +188,7 @@ class Ensemble:
         self.wls = list(workloads)
         self.hss = [(C.c_void_p * len(m))(*[self.doms[i].h.value for i in m]) for m in self.groups]
         self.batches = []
-        self.shapes = []   # autotuned (rows, columns, strip rows, waves) per batch
+        self.shapes = []   # autotuned (rows, columns, tile rows, waves) per batch
         if mode == "graph":
             for g, (hs, m) in enumerate(zip(self.hss, self.groups)):
                 bh = C.c_void_p()
