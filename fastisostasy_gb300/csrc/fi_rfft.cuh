@@ -21,7 +21,8 @@
 // and SM), gains the smaller operation count: 1024^2 52 -> 43, 94 -> 80,
 // 50 -> 43 us, 512^2 20.9 -> 16.1, 30.9 -> 24.2, 19.1 -> 15.3 us.
 // Lengths 2^k from 16 and 3 2^k from 24 on take this form (faster at each one
-// measured); the others keep the shared-memory stages.
+// measured; in the step engine shorter ones too); the others keep the
+// shared-memory stages.
 #pragma once
 
 #include "fi_fft.cuh"
