@@ -28,10 +28,13 @@ int cluster_config(const Plan2D& p, int mode, int* nc, int* threads, int* stages
 {
     if (p.nx < 16 || p.ny < 16) return 0;
     // A length without a register line takes the shared-memory stages, on 8 or
-    // 16 multiprocessors: faster than the grid-wide paths on the smallest
-    // domains (50^2: 520 against 663 us an RK4 update of ten steps), no longer
-    // at 80^2 (567 against 608 alone, 3 % slower in a served mix) and slower
-    // from 100^2 on (721 against 711; 122 = 2 61: 1368 against 892)
+    // 16 multiprocessors: faster than the grid-wide engine on the smallest
+    // domains (an RK4 update of ten steps: 34^2 371 against 584 us, 50^2 379
+    // against 549).  The line was drawn with direct sums for the odd radices
+    // (80^2 567 against 608 alone, 3 % slower in a served mix; 100^2 721
+    // against 711, 122 = 2 61 1368 against 892); with the present stages the
+    // cluster leads above it as well (80^2 436 against 563, 100^2 469 against
+    // 598, 122^2 651 against 713), which a served mix has not been timed for.
     if ((!CluLay::line_ok(p.h) || !CluLay::line_ok(p.ny)) && p.nx * p.ny > 4096) return 0;
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
